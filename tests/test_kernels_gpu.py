@@ -89,6 +89,23 @@ def test_gemm_f32(M, N, K):
     assert torch.equal(o3[0], o4[M // 2])
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 8, 64), (2, 9, 1024), (3, 1000, 1028), (4, 16, 3200), (8, 40, 4608), (9, 33, 1026),
+                                   (32, 65, 63), (33, 32, 65), (63, 2500, 128), (64, 9472, 96), (192, 5000, 1000)])
+def test_gemm_f32_one_order(M, N, K):
+    """Both kernels and every tile (few rows up to 32; 32x32, 32x64 and 64x64 tiles; operands that 16-byte copies do not
+    take) add in one order: rows taken alone are the same bits.  The bound: K products and sums of 2^-24 each."""
+    a, w, b = rnd(M, K, seed=1), rnd(N, K, seed=2), rnd(N, seed=3)
+    out = torch.empty(M, N, device=DEV)
+    ops().gemm_f32(a, w, b, out)
+    want = a.double() @ w.double().T + b.double()
+    size = a.double().abs() @ w.double().abs().T + b.double().abs()
+    assert bool(((out.double() - want).abs() <= (min(K, 64) + K // 64 + 3) * 2.0 ** -24 * size).all())
+    for n in sorted({1, 2, 5, min(M, 40)}):
+        part = torch.empty(min(n, M), N, device=DEV)
+        ops().gemm_f32(a[M - min(n, M):].contiguous(), w, b, part)
+        assert torch.equal(part, out[M - min(n, M):]), n
+
+
 def _ragged(q_lens, ctx):
     cu = [0]
     for q in q_lens:
