@@ -246,6 +246,20 @@ def test_attention_generic(dtype, nH, nKV, hd, ps, window):
     close(o1, o2, dtype)
 
 
+@pytest.mark.parametrize("hd", [64, 66, 128, 200, 520])
+def test_attention_generic_row_alone(hd):
+    """A row's result depends on its position alone: positions around the tiles of 8 keys, in one step and one by one."""
+    nH, nKV, ps, n = 4, 2, 16, 41
+    k, v, table, pos, re = _paged_setup(torch.float32, nKV, hd, ps, [n], [0], num_pages=64)
+    q = rnd(n, nH * hd, seed=14)
+    for window in (None, 11):
+        whole, one = torch.empty_like(q), torch.empty(1, nH * hd, device=DEV)
+        ops().attention_generic(q, k, v, table, pos, re, whole, nH, window, 1 / math.sqrt(hd))
+        for r in (0, 1, 7, 8, 9, 31, 32, 40):
+            ops().attention_generic(q[r:r + 1].contiguous(), k, v, table, pos[r:r + 1].contiguous(), re[:1], one, nH, window, 1 / math.sqrt(hd))
+            assert torch.equal(one[0], whole[r]), (window, r)
+
+
 def test_attention_finds_a_far_key():
     """One key among hundreds, on another page, carries a score that stands out: the output
     must be its value row.  Random pages elsewhere would hide a wrong page or a wrong slot."""
