@@ -1,5 +1,6 @@
 """Each CUDA kernel alone against its plain statement (tests/kernel_refs.py), at sizes other
 than the engine's: widths that are no power of two, odd head counts, ragged batches."""
+import functools
 import math
 
 import pytest
@@ -154,6 +155,39 @@ def test_shortconv_long_portions(L, H, bias):
     close(o1, o2, dtype)
     close(st1, st2, torch.float32)
     assert torch.equal(st1[4], st2[4]) and torch.equal(st1[8], st2[8])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H", [4, 132, 1024, 2044, 2048, 4100, 8192, 333, 4102])
+@pytest.mark.parametrize("kind", ["plain", "delta", "stack", "post", "rows"])
+def test_add_layernorm_sizes(dtype, H, kind):
+    """One, two and four columns-of-four a thread, sizes behind them and sizes not divisible by four."""
+    n = 5
+    h1 = rnd(n, H, seed=1) + 0.5
+    h2 = h1.clone()
+    w, post = rnd(H, seed=2), rnd(H, seed=3) if kind == "post" else None
+    rows = torch.tensor([3, 0, 3], dtype=torch.int32, device=DEV) if kind == "rows" else None
+    delta = rnd(n, H, dtype=dtype, seed=4) if kind == "delta" else rnd(3, n, H, seed=4) if kind == "stack" else None
+    m = 3 if kind == "rows" else n
+    o1, o2 = torch.zeros(m, H, dtype=dtype, device=DEV), torch.zeros(m, H, dtype=dtype, device=DEV)
+    ops().add_layernorm(h1, delta, w, o1, 1e-5, rows, post)
+    ref.add_layernorm(h2, delta, w, o2, 1e-5, rows, post)
+    close(o1, o2, dtype)
+    close(h1, h2, torch.float32)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,H", [(1, 3), (3, 4), (7, 129), (64, 1024)])
+def test_residual_add_sizes(dtype, n, H):
+    h = rnd(n, H, seed=1)
+    d = rnd(n, H, dtype=dtype, seed=2)
+    want = h + d.float()
+    ops().residual_add(h, d)
+    assert torch.equal(h, want)
+    s = rnd(3, n, H, seed=3)
+    want = h + s[0] + s[1] + s[2]
+    ops().residual_add(h, s)
+    assert torch.equal(h, want)
 
 
 def _paged_setup(dtype, n_kv, hd, ps, q_lens, ctx, seed=0, num_pages=64):
