@@ -25,7 +25,14 @@ template <typename TO, typename TI>
 __device__ __forceinline__ float ng_ld_sum(const TI* p, size_t idx, int n_part, size_t stride) {
     if (n_part <= 1) return ng_ld(p + idx);
     float v = 0.f;
-    for (int s = 0; s < n_part; ++s) v += ng_ld(p + s * stride + idx);
+    for (int s0 = 0; s0 < n_part; s0 += 4) {            // four loads in flight; one at a time, each waits for memory
+        float f[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) f[k] = s0 + k < n_part ? ng_ld(p + (s0 + k) * stride + idx) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (s0 + k < n_part) v += f[k];
+    }
     TO r;
     ng_st(&r, v);
     return ng_ld(&r);

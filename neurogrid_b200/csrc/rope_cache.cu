@@ -102,6 +102,16 @@ rope_cache_kernel(const TI* __restrict__ qkv, T* __restrict__ q_out, const float
         cs[u] = 1.f;
         if (inv_freq && i < half) sincosf(pf * inv_freq[i], &sn[u], &cs[u]);
     }
+    // and the norms' weights, as far as registers allow
+    constexpr bool HELD = PAIRS <= 2;
+    float nw[2][HELD ? PAIRS : 1][2];
+    if constexpr (HELD)
+#pragma unroll
+        for (int u = 0; u < PAIRS; ++u) {
+            const int i = min(lane + 32 * u, half - 1), a = half_pairing ? i : 2 * i, b = half_pairing ? i + half : 2 * i + 1;
+            nw[0][u][0] = qw ? qw[a] : 1.f; nw[0][u][1] = qw ? qw[b] : 1.f;
+            nw[1][u][0] = kw ? kw[a] : 1.f; nw[1][u][1] = kw ? kw[b] : 1.f;
+        }
     ng_pdl_wait();
     qkv = ng_after_wait(qkv);
     if (!page_ok && threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, NG_STATUS_BAD_PAGE);
@@ -145,7 +155,10 @@ rope_cache_kernel(const TI* __restrict__ qkv, T* __restrict__ q_out, const float
                 if (i < half) {
                     const int a = half_pairing ? i : 2 * i, b = half_pairing ? i + half : 2 * i + 1;
                     float y1 = x1[hb][u], y2 = x2[hb][u];
-                    if (w) { y1 = y1 * r * w[a]; y2 = y2 * r * w[b]; }
+                    if (w) {
+                        if constexpr (HELD) { y1 = y1 * r * (is_q ? nw[0][u][0] : nw[1][u][0]); y2 = y2 * r * (is_q ? nw[0][u][1] : nw[1][u][1]); }
+                        else { y1 = y1 * r * w[a]; y2 = y2 * r * w[b]; }
+                    }
                     if (inv_freq && !is_v) {
                         const float z1 = y1 * cs[u] - y2 * sn[u], z2 = y1 * sn[u] + y2 * cs[u];
                         y1 = z1; y2 = z2;

@@ -103,6 +103,65 @@ shortconv_kernel(const TI* __restrict__ p, const float* __restrict__ w, const fl
     }
 }
 
+// A step of single tokens (no entry has more than one): a thread per channel and entry.  Bound by the latency of its
+// loads, so the three inputs' partial sums are all requested at once (the kernel above walks a tile: B and x, then C,
+// then B and x again for the slot, each a round trip to the L2), and the slot takes u from the register: 2.7 us a launch of
+// 8 rows of 2,048 channels inside a step's graph against 7.8 us.
+template <typename TI, typename T, int L>
+__global__ void __launch_bounds__(CONV_THREADS)
+shortconv_token_kernel(const TI* __restrict__ p, const float* __restrict__ w, const float* __restrict__ bias,
+                       float* __restrict__ state, T* __restrict__ out, const int* __restrict__ cu_q,
+                       const int* __restrict__ ctx_before, const int* __restrict__ slots, int H, int n_part, size_t pstride) {
+    ng_pdl_trigger();
+    const int e = blockIdx.y;
+    const int row = cu_q[e];
+    const int d = blockIdx.x * CONV_THREADS + threadIdx.x;
+    if (cu_q[e + 1] <= row || d >= H) {
+        ng_pdl_wait();
+        return;
+    }
+    const int ctx = ctx_before[e];
+    float* st = state + (size_t)slots[e] * (L - 1) * H + d;      // st[j*H]: u at position ctx-(L-1)+j
+    float wk[L], old[L - 1];
+#pragma unroll
+    for (int k = 0; k < L; ++k) wk[k] = w[(size_t)d * L + k];
+#pragma unroll
+    for (int j = 0; j < L - 1; ++j) old[j] = ctx - (L - 1) + j >= 0 ? st[(size_t)j * H] : 0.f;
+    const float b = bias ? bias[d] : 0.f;
+    ng_pdl_wait();
+    p = ng_after_wait(p);
+    const size_t at = (size_t)row * 3 * H + d;
+    float in[3] = {0.f, 0.f, 0.f};                               // B, C, x
+    for (int s0 = 0; s0 < n_part; s0 += 4) {
+        float f[4][3];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) f[k][i] = s0 + k < n_part ? ng_ld(p + (s0 + k) * pstride + at + (size_t)i * H) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                if (s0 + k < n_part) in[i] += f[k][i];           // ascending, as ng_ld_sum adds
+    }
+    if (n_part > 1)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            T r;
+            ng_st(&r, in[i]);
+            in[i] = ng_ld(&r);
+        }
+    const float u = in[0] * in[2];
+    float acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < L - 1; ++k) acc = fmaf(wk[k], old[k], acc);
+    acc = fmaf(wk[L - 1], u, acc) + b;
+    ng_st(out + (size_t)row * H + d, in[1] * acc);
+#pragma unroll
+    for (int j = 0; j < L - 2; ++j) st[(size_t)j * H] = old[j + 1];
+    st[(size_t)(L - 2) * H] = u;
+}
+
 // The bulk case (bfloat16 in and out, no partial sums, even width): two channels per thread, so
 // that every access is 4 bytes wide.  Same arithmetic and the same ownership of the slot.
 template <int L>
@@ -326,6 +385,16 @@ NG_EXPORT int ng_shortconv(const void* p, const float* w, const float* bias, flo
     dim3 grid((H + CONV_THREADS - 1) / CONV_THREADS, (max_q + CONV_TILE - 1) / CONV_TILE, n_entries);
     if (grid.y > 65535 || grid.z > 65535) return NG_BAD_SIZE;
     const size_t ps = (size_t)partial_stride;
+    if (max_q == 1 && n_entries <= 65535) {
+        dim3 g1((H + CONV_THREADS - 1) / CONV_THREADS, n_entries);
+#define CONV_TOKEN(TI, T, NP, PS)                                                                                      \
+    NG_LAUNCH((shortconv_token_kernel<TI, T, NG_CONV_L>), g1, CONV_THREADS, 0, stream, (const TI*)p, w, bias, state, (T*)out, \
+              cu_q, ctx_before, slots, H, NP, PS)
+        if (act_bf16 && n_partials > 1) CONV_TOKEN(float, __nv_bfloat16, n_partials, ps);
+        else if (act_bf16) CONV_TOKEN(__nv_bfloat16, __nv_bfloat16, 1, 0);
+        else CONV_TOKEN(float, float, n_partials < 1 ? 1 : n_partials, ps);
+        return ng_launch_status();
+    }
     if (act_bf16 && n_partials <= 1 && H % 8 == 0 && max_q >= 64 && ((uintptr_t)p & 15) == 0 && ((uintptr_t)out & 15) == 0 &&
         ((uintptr_t)state & 15) == 0 && (((uintptr_t)w | (uintptr_t)bias) & 3) == 0) {
         dim3 g8((H / 8 + CONV_THREADS - 1) / CONV_THREADS, (max_q + CONV_TILE8 - 1) / CONV_TILE8, grid.z);

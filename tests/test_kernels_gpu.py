@@ -158,6 +158,28 @@ def test_shortconv_long_portions(L, H, bias):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("L,H,parts", [(3, 2048, 1), (3, 200, 3), (2, 96, 5), (4, 130, 9)])
+def test_shortconv_single_tokens(dtype, L, H, parts):
+    """A step of single tokens: one tensor or a stack of partial sums (fewer than, exactly and more than four at a time), a
+    request at its first tokens, one without a token in the step."""
+    ctx = [5, 0, 1, 40, 7, 2]
+    cu = torch.tensor([0, 1, 2, 3, 4, 4, 5], dtype=torch.int32, device=DEV)
+    cb, slots = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in (ctx, [3, 0, 5, 1, 6, 2]))
+    stack = rnd(parts, 5, 3 * H, seed=4, std=0.5)
+    p = stack[0].to(dtype) if parts == 1 else stack
+    whole = p if parts == 1 else functools.reduce(torch.add, stack).to(dtype)
+    w, b = rnd(H, L, seed=5, std=0.3), rnd(H, seed=6, std=0.1)
+    st1 = rnd(8, L - 1, H, seed=7)
+    st2 = st1.clone()
+    o1, o2 = torch.zeros(5, H, dtype=dtype, device=DEV), torch.zeros(5, H, dtype=dtype, device=DEV)
+    ops().shortconv(p, w, b, st1, o1, cu, cb, slots, 6, 1)
+    ref.shortconv(whole, w, b, st2, o2, cu, cb, slots, 6, 1)
+    close(o1, o2, dtype)
+    close(st1, st2, torch.float32)
+    assert all(torch.equal(st1[i], st2[i]) for i in (4, 6, 7))             # slots without a token stay
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H", [4, 132, 1024, 2044, 2048, 4100, 8192, 333, 4102])
 @pytest.mark.parametrize("kind", ["plain", "delta", "stack", "post", "rows"])
 def test_add_layernorm_sizes(dtype, H, kind):
