@@ -757,8 +757,7 @@ def metanex_kernel_times(eng, l2, pk):
         tok = torch.randint(0, model.spec.vocab_size, (rows,), generator=g, device=dev).to(torch.int32)
         status = torch.zeros(1, dtype=torch.int32, device=dev)
         sd = blk.side
-        ssc = torch.empty(max(1, ops.token_side_scratch(rows, D, sd.spec.dim)), device=dev) if rows < 128 else None
-        us = timed(lambda: ops.token_side(h, tok, sd.table, sd.w_gate, sd.w_proj, sd.w_norm, re, sd.spec.eps, status, ssc))
+        us = timed(lambda: ops.token_side(h, tok, sd.table, sd.w_gate, sd.w_proj, sd.w_norm, re, sd.spec.eps, status))
         mem(f"{tag}_token_side", us, 2 * rows * D * 4 + (sd.w_gate.numel() + sd.w_proj.numel()) * 4)
         # router and weighting of the experts' activations
         f = blk.ffn

@@ -15,6 +15,7 @@ import scenarios
 from helpers import make_ctx, make_runner, rel_err
 from neurogrid_b200.config import (InputConvSpec, LatentAttentionSpec, MoESpec, NoPositionSpec, RetentionSpec, RopeSpec,
                                    ScalarRMSNormSpec, TokenSideSpec)
+from neurogrid_b200.csrc import ops
 from neurogrid_b200.engine import StepEntry
 from neurogrid_b200.parts import PagedView, SlotView, build
 from neurogrid_b200.parts.input_conv import InputConv, TokenSide
@@ -332,6 +333,37 @@ def test_token_side(dtype, rows, H):
     want = h.double().cpu() + plain.token_side(h.double().cpu(), toks, pw, layer, dim, 1e-5)
     part.forward(h, ctx)
     assert rel_err(h, want) < 1e-5
+
+
+@pytest.mark.parametrize("rows,H,dim", [(1, 2048, 64), (16, 1024, 64), (17, 1028, 13), (255, 2048, 64), (256, 1024, 64),
+                                        (271, 2048, 60), (300, 1036, 64), (300, 2052, 8), (20, 40, 70), (3, 2055, 9), (300, 40, 70)])
+def test_token_side_sizes(rows, H, dim):
+    """A cluster of blocks for one and for four rows, blocks of 16 rows, and sizes that their registers do not hold; rows
+    without a request stay as they are, a row's bits do not depend on the others.  The bound: float32 sums of H and dim terms."""
+    V = 50
+    g = torch.Generator().manual_seed(rows + H)
+    rnd = lambda *s, std=1.0: (torch.randn(*s, generator=g) * std).to(DEV)  # noqa: E731
+    h, table, wg, wp, wn = rnd(rows, H, std=2.0), rnd(V, dim), rnd(dim, H, std=H ** -0.5), rnd(dim, H, std=dim ** -0.5), rnd(H)
+    toks = torch.randint(0, V, (rows,), generator=g).to(torch.int32).to(DEV)
+    entry = torch.zeros(rows, dtype=torch.int32, device=DEV)
+    if rows > 2:
+        entry[rows // 2] = -1
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got = h.clone()
+    ops.token_side(got, toks, table, wg, wp, wn, entry, 1e-5, status)
+    x = h.double()
+    y = (torch.nn.functional.gelu(x @ wg.double().T, approximate="tanh") * table.double()[toks.long()]) @ wp.double()
+    want = x + y * torch.rsqrt((y * y).mean(-1, keepdim=True) + 1e-5) * wn.double()
+    want[entry < 0] = x[entry < 0]
+    assert int(status) == 0 and rel_err(got, want) < 1e-5
+    assert torch.equal(got[entry < 0], h[entry < 0])
+    swap = torch.arange(rows - 1, -1, -1, device=DEV)
+    back = h[swap].contiguous()
+    ops.token_side(back, toks[swap].contiguous(), table, wg, wp, wn, entry[swap].contiguous(), 1e-5, status)
+    assert torch.equal(back[swap], got)
+    toks[0] = V
+    ops.token_side(got, toks, table, wg, wp, wn, entry, 1e-5, status)
+    assert int(status) != 0
 
 
 # ------------------------------------------------------------------------------------------ whole models
