@@ -189,16 +189,33 @@ token_side_cluster_kernel(float* __restrict__ h_, const int* __restrict__ tokens
 }
 
 // ---- many rows -------------------------------------------------------------------------------------------------
-// Bound by the FMA pipe (2 * 2 * dim * H operations a row).  A block takes 16 rows, staged in shared memory.  Gate: eight
-// consecutive k at a time go to one of the eight warps, which forms all 16 x 64 values over its k, 4 x 8 a lane (even
-// and odd k in the halves of a packed FMA), with the next eight k of W_gate on their way to its registers; the warps' sums are added
-// in order.  Projection: a thread owns four neighbouring columns (NC times) for all 16 rows and keeps y in registers
-// until the row's mean square is known.
+// Bound by the FMA pipe (2 * 2 * dim * H operations a row) once the matrices come through shared memory: read from the L2
+// straight into registers, rows H apart, they cost 20 wavefronts a load and the kernel 60 us (2,048 rows of 1,024), now 36 us;
+// 93 us for one that read shared memory for every FMA.  A block takes 16 rows, staged in shared memory; both matrices pass through one
+// ring of 17 KB stages, TL_STAGES - 1 ahead.  Gate: a stage is 64 k of W_gate; each of the eight warps takes eight of them and
+// forms all 16 x 64 values over its k, 4 x 8 a lane (even and odd k in the halves of a packed FMA); the warps' sums are
+// added in order.  Projection: a stage is four rows of 1,024 columns of W_proj^T; a thread owns four neighbouring columns (NC
+// times) for all 16 rows and keeps y in registers until the row's mean square is known.
 #define TL_ROWS 16
 #define TL_THREADS 256
 #define TL_WARPS (TL_THREADS / 32)
 #define TL_DIM 64
 #define TL_COLS (4 * TL_THREADS)
+#define TL_STAGES 4
+#define TL_KS 64                         // k of a gate stage
+#define TL_PITCH (TL_KS + 4)             // eight rows' 16 bytes in different banks
+#define TL_STAGE (TL_DIM * TL_PITCH)
+#define TL_PI 4                          // rows of W_proj^T of a stage
+static_assert(TL_PI * TL_COLS <= TL_STAGE, "a stage holds either");
+
+__host__ __device__ constexpr int tl_rows_floats(int H) {          // the rows; the warps' sums take their place
+    return TL_ROWS * (H + 4) > TL_WARPS * TL_ROWS * TL_DIM ? TL_ROWS * (H + 4) : TL_WARPS * TL_ROWS * TL_DIM;
+}
+// 16 bytes to shared memory, asynchronously; zeros where `real` is false
+__device__ __forceinline__ void tl_copy(float* dst, const float* src, bool real) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(real ? 16 : 0) : "memory");
+}
 
 template <int NC>
 __global__ void __launch_bounds__(TL_THREADS, 1)
@@ -209,24 +226,42 @@ token_side_tile_kernel(float* __restrict__ h_, const int* __restrict__ tokens, c
     extern __shared__ __align__(16) float ts_sm[];
     const int ldx = H + 4;                                         // rows 4 words apart modulo the banks
     float* xs = ts_sm;                                             // [16][H + 4]
-    float* part = xs + TL_ROWS * ldx;                              // [8 warps][16][64]
-    float2* g2 = reinterpret_cast<float2*>(part + TL_WARPS * TL_ROWS * TL_DIM);      // [64][16]: (g, g)
+    float* part = ts_sm;                                           // then [8 warps][16][64]
+    float* ring = ts_sm + tl_rows_floats(H);                       // [TL_STAGES][TL_STAGE]
+    float2* g2 = reinterpret_cast<float2*>(ring + TL_STAGES * TL_STAGE);            // [64][16]: (g, g)
     __shared__ int s_tok[TL_ROWS], s_live[TL_ROWS];
     __shared__ float red[TL_WARPS][TL_ROWS], scale[TL_ROWS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r0 = blockIdx.x * TL_ROWS, rg = lane >> 3, cg = lane & 7;
+    const int gate_stages = (H + TL_KS - 1) / TL_KS, pieces = (dim + TL_PI - 1) / TL_PI, stages = gate_stages + NC * pieces;
     ng_pdl_trigger();
-    const ulonglong2 none = make_ulonglong2(0ull, 0ull);
-    ulonglong2 nxt[8][2];
-    auto load_w = [&](int k) {                                     // eight k of the lane's eight rows of W_gate
+    auto request = [&](int t) {                                    // one group of copies a stage, empty ones at the end
+        float* s = ring + (t % TL_STAGES) * TL_STAGE;
+        if (t < gate_stages) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
+            for (int q = 0; q < TL_DIM * TL_KS / 4 / TL_THREADS; ++q) {
+                const int i = tid + q * TL_THREADS, r = i / (TL_KS / 4), k = (i % (TL_KS / 4)) * 4;
+                const bool real = r < dim && t * TL_KS + k < H;
+                tl_copy(s + r * TL_PITCH + k, real ? w_gate + (size_t)r * H + t * TL_KS + k : w_gate, real);
+            }
+        } else if (t < stages) {
+            const int c = (t - gate_stages) / pieces, i0 = ((t - gate_stages) % pieces) * TL_PI, col = c * TL_COLS + tid * 4;
 #pragma unroll
-            for (int q = 0; q < 2; ++q)
-                nxt[j][q] = cg + 8 * j < dim && k + 4 * q < H
-                                ? *reinterpret_cast<const ulonglong2*>(w_gate + (size_t)(cg + 8 * j) * H + k + 4 * q) : none;
+            for (int q = 0; q < TL_PI; ++q) {
+                const bool real = i0 + q < dim && col < H;
+                tl_copy(s + q * TL_COLS + tid * 4, real ? w_proj_t + (size_t)(i0 + q) * H + col : w_proj_t, real);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    load_w(warp * 8);
+    // stage t has landed and the one read before it may be written again
+    auto next = [&](int t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(TL_STAGES - 2) : "memory");
+        __syncthreads();
+        request(t + TL_STAGES - 1);
+        return ring + (t % TL_STAGES) * TL_STAGE;
+    };
+    for (int t = 0; t < TL_STAGES - 1; ++t) request(t);
     ng_pdl_wait();
     float* h = ng_after_wait(h_);
     if (tid < TL_ROWS) {
@@ -235,34 +270,36 @@ token_side_tile_kernel(float* __restrict__ h_, const int* __restrict__ tokens, c
         s_tok[tid] = tok;
     }
     __syncthreads();
+#pragma unroll 8
     for (int i = tid; i < TL_ROWS * (H / 4); i += TL_THREADS) {
         const int r = i / (H / 4), j = (i % (H / 4)) * 4;
         *reinterpret_cast<float4*>(xs + r * ldx + j) =
             s_live[r] ? *reinterpret_cast<const float4*>(h + (size_t)(r0 + r) * H + j) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    __syncthreads();
     {
         uint64_t acc[4][8];
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[r][j] = 0ull;
-        for (int k = warp * 8; k < H; k += 8 * TL_WARPS) {
-            ulonglong2 cur[8][2];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) cur[j][0] = nxt[j][0], cur[j][1] = nxt[j][1];
-            load_w(k + 8 * TL_WARPS);
+        for (int t = 0; t < gate_stages; ++t) {
+            const float* w = next(t) + cg * TL_PITCH + warp * 8;
+            const int k = t * TL_KS + warp * 8;
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
-                if (k + 4 * q >= H) break;
+                if (k + 4 * q >= H) break;                         // (the rows end there)
+                ulonglong2 xv[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const ulonglong2 xv = *reinterpret_cast<const ulonglong2*>(xs + (4 * r + rg) * ldx + k + 4 * q);
+                for (int r = 0; r < 4; ++r) xv[r] = *reinterpret_cast<const ulonglong2*>(xs + (4 * r + rg) * ldx + k + 4 * q);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[r][j] = ts_fma2(xv.y, cur[j][q].y, ts_fma2(xv.x, cur[j][q].x, acc[r][j]));
+                for (int j = 0; j < 8; ++j) {
+                    const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(w + 8 * j * TL_PITCH + 4 * q);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) acc[r][j] = ts_fma2(xv[r].y, wv.y, ts_fma2(xv[r].x, wv.x, acc[r][j]));
                 }
             }
         }
+        __syncthreads();                                           // the rows are done with
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -270,8 +307,9 @@ token_side_tile_kernel(float* __restrict__ h_, const int* __restrict__ tokens, c
                 part[(warp * TL_ROWS + 4 * r + rg) * TL_DIM + cg + 8 * j] = ts_lo(acc[r][j]) + ts_hi(acc[r][j]);
     }
     __syncthreads();
-    for (int i = tid; i < TL_ROWS * TL_DIM; i += TL_THREADS) {
-        const int r = i / TL_DIM, d = i % TL_DIM;
+#pragma unroll
+    for (int q = 0; q < TL_ROWS * TL_DIM / TL_THREADS; ++q) {
+        const int i = tid + q * TL_THREADS, r = i / TL_DIM, d = i % TL_DIM;
         float a = 0.f;
 #pragma unroll
         for (int k = 0; k < TL_WARPS; ++k) a += part[(k * TL_ROWS + r) * TL_DIM + d];
@@ -282,14 +320,14 @@ token_side_tile_kernel(float* __restrict__ h_, const int* __restrict__ tokens, c
     uint64_t y[NC][TL_ROWS][2];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-        const int col = c * TL_COLS + tid * 4;
 #pragma unroll
         for (int r = 0; r < TL_ROWS; ++r) y[c][r][0] = y[c][r][1] = 0ull;
-        if (col < H) {
-#pragma unroll 4
-            for (int i = 0; i < dim; ++i) {
-                const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(w_proj_t + (size_t)i * H + col);
-                const ulonglong2* gp = reinterpret_cast<const ulonglong2*>(g2 + i * TL_ROWS);
+        for (int t = 0; t < pieces; ++t) {
+            const float* w = next(gate_stages + c * pieces + t) + tid * 4;
+#pragma unroll
+            for (int q = 0; q < TL_PI; ++q) {                      // (rows beyond dim are zeros, and so are their g)
+                const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(w + q * TL_COLS);
+                const ulonglong2* gp = reinterpret_cast<const ulonglong2*>(g2 + (t * TL_PI + q) * TL_ROWS);
 #pragma unroll
                 for (int r = 0; r < TL_ROWS; r += 2) {
                     const ulonglong2 gv = gp[r / 2];
@@ -327,11 +365,11 @@ token_side_tile_kernel(float* __restrict__ h_, const int* __restrict__ tokens, c
 #pragma unroll
         for (int r = 0; r < TL_ROWS; ++r) {
             if (!s_live[r]) continue;
-            const float4 x = *reinterpret_cast<const float4*>(xs + r * ldx + col);
+            float4* hp = reinterpret_cast<float4*>(h + (size_t)(r0 + r) * H + col);
+            const float4 x = *hp;
             const float f = scale[r];
-            *reinterpret_cast<float4*>(h + (size_t)(r0 + r) * H + col) =
-                make_float4(x.x + ts_lo(y[c][r][0]) * f * w.x, x.y + ts_hi(y[c][r][0]) * f * w.y,
-                            x.z + ts_lo(y[c][r][1]) * f * w.z, x.w + ts_hi(y[c][r][1]) * f * w.w);
+            *hp = make_float4(x.x + ts_lo(y[c][r][0]) * f * w.x, x.y + ts_hi(y[c][r][0]) * f * w.y,
+                              x.z + ts_lo(y[c][r][1]) * f * w.z, x.w + ts_hi(y[c][r][1]) * f * w.w);
         }
     }
 }
@@ -347,13 +385,13 @@ NG_EXPORT int ng_token_side(float* h, const int* tokens, const float* table, con
     const bool wide = H % 4 == 0 && (((uintptr_t)h | (uintptr_t)w_gate | (uintptr_t)w_proj_t | (uintptr_t)w_norm) & 15) == 0;
     const bool fit = wide && dim <= TL_DIM && H <= 2 * TL_COLS;
     if (n_rows >= TS_LONG && fit) {
-        const size_t smem = (size_t)(TL_ROWS * (H + 4) + TL_WARPS * TL_ROWS * TL_DIM + 2 * TL_DIM * TL_ROWS) * sizeof(float);
+        const size_t smem = (size_t)(tl_rows_floats(H) + TL_STAGES * TL_STAGE + 2 * TL_DIM * TL_ROWS) * sizeof(float);
         const int blocks = (n_rows + TL_ROWS - 1) / TL_ROWS;
 #define TL_GO(NC)                                                                                                      \
     do {                                                                                                               \
         static bool configured = false;                                                                                \
         if (!configured) {                                                                                             \
-            if (cudaFuncSetAttribute(token_side_tile_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) \
+            if (cudaFuncSetAttribute(token_side_tile_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) \
                 return NG_LAUNCH_FAILED;                                                                               \
             configured = true;                                                                                         \
         }                                                                                                              \
