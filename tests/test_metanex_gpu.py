@@ -366,6 +366,35 @@ def test_token_side_sizes(rows, H, dim):
     assert int(status) != 0
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n,H,E,top", [(1, 2048, 16, 4), (8, 512, 3, 3), (5, 516, 40, 32), (255, 2052, 17, 2), (256, 1024, 16, 4),
+                                       (515, 1540, 33, 7), (3000, 128, 17, 1), (600, 75, 5, 1), (2, 64, 100, 5)])
+def test_moe_router_choice(dtype, n, H, E, top):
+    """A block per row and a warp per row (from 256 rows on), widths of one and of several pieces and not divisible by four;
+    more experts than a warp has lanes, and than shared memory holds; of equal logits the
+    lower index; logits that are not numbers take the first experts left, as a walk from index 0 does."""
+    g = torch.Generator().manual_seed(n)
+    x = torch.randn(n, H, generator=g).to(dtype).to(DEV)
+    w = (torch.randn(E, H, generator=g) * H ** -0.5).to(DEV)
+    b = torch.randn(E, generator=g).to(DEV)
+    w[E - 1], b[E - 1] = w[0], b[0]                                      # a tie
+    got = torch.empty(n, E, device=DEV)
+    ops.moe_router(x, w, b, got, top)
+    z = x.double() @ w.double().T + b.double()
+    kept = got > 0
+    assert bool((kept.sum(-1) == top).all())
+    order = torch.sort(z, dim=-1, descending=True, stable=True)
+    low = order.values[:, top - 1:top]
+    assert bool((z[kept].view(n, top) >= low - 1e-5).all())
+    want = torch.zeros_like(z).masked_scatter_(kept, torch.softmax(z[kept].view(n, top), -1))
+    assert rel_err(got, want) < 1e-5
+    if top < E:
+        assert not bool((kept[:, E - 1] & ~kept[:, 0]).any())
+    x[0] = float("nan")
+    ops.moe_router(x, w, b, got, top)
+    assert bool(torch.isnan(got[0, :top]).all()) and bool((got[0, top:] == 0).all())
+
+
 # ------------------------------------------------------------------------------------------ whole models
 LENS = {"P": [1, 9, 40, 131, 64, 23, 77], "Q": [3, 50, 97, 30, 64], "R": [2, 17, 90, 33]}
 
