@@ -26,11 +26,15 @@ retention_kernel(const T* __restrict__ x, const float* __restrict__ inv_freq, in
     float* part = ks + dk;          // [G * dv]
     float* red = part + G * dv;     // [32]
     ng_pdl_trigger();
-    ng_pdl_wait();
+    // the batch description and the state (written by an earlier step, which the step's first copy is behind) do not
+    // depend on the product in front of this kernel: a step of single tokens has its state in registers when that ends
     const int e = blockIdx.x, head = blockIdx.y;
     const int q0 = cu_q[e];
     const int qlen = cu_q[e + 1] - q0;
-    if (qlen <= 0) return;
+    if (qlen <= 0) {
+        ng_pdl_wait();
+        return;
+    }
     const int ctx = ctx_before[e];
     const int tid = threadIdx.x;
     const int j = tid % dv, g = tid / dv;          // blockDim.x is a multiple of 32 >= G * dv
@@ -49,9 +53,13 @@ retention_kernel(const T* __restrict__ x, const float* __restrict__ inv_freq, in
         const int i = i0 + r;
         s[r] = (live && ctx > 0 && i < dk) ? S[(size_t)i * dv + j] : 0.f;
     }
+    ng_pdl_wait();
+    x = ng_after_wait(x);
     for (int t = 0; t < qlen; ++t) {
         const T* row = x + (size_t)(q0 + t) * ld;
         const float pos = (float)(ctx + t);
+        const float vj = live ? ng_ld(row + off_v + j) : 0.f;
+        const float gate = tid < dv ? ng_ld(row + off_g + tid) : 0.f;
         for (int i = tid; i < dk; i += blockDim.x) {
             float qv = ng_ld(row + off_q + i), kv = ng_ld(row + off_k + i);
             if (i < rot_dims) {
@@ -69,7 +77,6 @@ retention_kernel(const T* __restrict__ x, const float* __restrict__ inv_freq, in
         }
         __syncthreads();
         if (live) {
-            const float vj = ng_ld(row + off_v + j);
             float acc = 0.f;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -87,7 +94,6 @@ retention_kernel(const T* __restrict__ x, const float* __restrict__ inv_freq, in
             for (int gg = 0; gg < G; ++gg) o += part[gg * dv + tid];
         const float ss = ng_block_sum(tid < dv ? o * o : 0.f, red);
         if (tid < dv) {
-            const float gate = ng_ld(row + off_g + tid);
             const float y = o * rsqrtf(ss / (float)dv + eps) * (gate / (1.f + expf(-gate)));
             ng_st(out + (size_t)(q0 + t) * nH * dv + (size_t)head * dv + tid, y);
         }
@@ -235,13 +241,14 @@ __global__ void retention_scan_kernel(float* __restrict__ u_scratch, float* __re
     const int nc = (qlen + RC - 1) / RC;
     float* U0 = u_scratch + (((size_t)(q0 / RC + e)) * nH + head) * dk * dv + i;
     const size_t stride = (size_t)nH * dk * dv;
-    // eight chunks' additions are fetched at once: the walk itself is a chain, the loads need not be
-    for (int c0 = 0; c0 < nc; c0 += 8) {
-        float u[8];
+    // sixteen chunks' additions are fetched at once: the walk itself is a chain, the loads need not be
+    constexpr int AHEAD = 16;
+    for (int c0 = 0; c0 < nc; c0 += AHEAD) {
+        float u[AHEAD];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) u[k] = c0 + k < nc ? U0[(size_t)(c0 + k) * stride] : 0.f;
+        for (int k = 0; k < AHEAD; ++k) u[k] = c0 + k < nc ? U0[(size_t)(c0 + k) * stride] : 0.f;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < AHEAD; ++k) {
             const int c = c0 + k;
             if (c >= nc) break;
             U0[(size_t)c * stride] = s;
@@ -382,6 +389,241 @@ __global__ void retention_norm_gate_kernel(const float* __restrict__ o, const T*
     }
 }
 
+// ---------------------------------------------------------------------------------- heads of 128 x 128
+// `local` and `out` for the common head size, with register tiles that make them bound by the FMA pipe instead of by shared
+// memory (8 x 8 and 4 x 4 elements a thread, four 16-byte reads for 64 and eight for 64 FMAs, where the kernels above
+// read one and more words an FMA).  A block takes a whole head's chunk: `out` has the head's 128 columns together, so the
+// head's norm and gate are its epilogue (one kernel and one float32 pass over the rows less).  The state of the chunk
+// passes through two buffers of 32 rows while the scores are formed.  2,048 tokens, 8 heads: local 26 us (65 us with the
+// kernel above), out 48 us (114 us and 8 us for the norm).
+#define R1_D 128
+#define R1_P (R1_D + 4)                  // eight rows' 16 bytes in different banks
+#define R1_THREADS 256
+
+__device__ __forceinline__ float4 r1_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 r1_ld4(const __nv_bfloat16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void r1_st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void r1_st4(__nv_bfloat16* p, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    uint2 u;
+    u.x = *reinterpret_cast<const uint32_t*>(&a);
+    u.y = *reinterpret_cast<const uint32_t*>(&b);
+    *reinterpret_cast<uint2*>(p) = u;
+}
+
+// q and k of a chunk, rotated, k scaled (and each row of k times `weight[t]`, if given); rows past n are zero.  A thread
+// takes coordinate pairs: (p, p + half) inside the rotated ones, neighbours behind them.
+template <typename T, bool WANT_Q>
+__device__ __forceinline__ void r1_load_qk(const T* __restrict__ q, const T* __restrict__ k, size_t ld, int n, int pos0,
+                                           const float* __restrict__ inv_freq, int rot_dims, float kscale,
+                                           const float* weight, float* Qs, float* Ks) {
+    const int half = rot_dims / 2;
+#pragma unroll 4
+    for (int u = 0; u < RC * R1_D / 2 / R1_THREADS; ++u) {
+        const int idx = threadIdx.x + u * R1_THREADS, t = idx / (R1_D / 2), p = idx % (R1_D / 2);
+        const int a = p < half ? p : rot_dims + 2 * (p - half), b = p < half ? p + half : a + 1;
+        float qa = 0.f, qb = 0.f, ka = 0.f, kb = 0.f;
+        if (t < n) {
+            if (WANT_Q) qa = ng_ld(q + t * ld + a), qb = ng_ld(q + t * ld + b);
+            ka = ng_ld(k + t * ld + a), kb = ng_ld(k + t * ld + b);
+            if (p < half) {
+                float sn, cs;
+                sincosf((float)(pos0 + t) * inv_freq[p], &sn, &cs);
+                const float z = ka * cs - kb * sn;
+                kb = kb * cs + ka * sn;
+                ka = z;
+                if (WANT_Q) {
+                    const float y = qa * cs - qb * sn;
+                    qb = qb * cs + qa * sn;
+                    qa = y;
+                }
+            }
+        }
+        const float f = weight ? weight[t] : 1.f;
+        if (WANT_Q) Qs[t * R1_P + a] = qa, Qs[t * R1_P + b] = qb;
+        Ks[t * R1_P + a] = ka * kscale * f;
+        Ks[t * R1_P + b] = kb * kscale * f;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void r1_load_v(const T* __restrict__ v, size_t ld, int n, float* Vs) {
+#pragma unroll
+    for (int u = 0; u < RC * R1_D / 4 / R1_THREADS; ++u) {
+        const int idx = threadIdx.x + u * R1_THREADS, t = idx / (R1_D / 4), c = (idx % (R1_D / 4)) * 4;
+        *reinterpret_cast<float4*>(Vs + t * R1_D + c) = t < n ? r1_ld4(v + t * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(R1_THREADS)
+retention_local128_kernel(const T* __restrict__ x, const float* __restrict__ inv_freq, const float* __restrict__ decay,
+                          float* __restrict__ u_scratch, const int* __restrict__ cu_q, const int* __restrict__ ctx_before,
+                          int nH, int rot_dims) {
+    __shared__ __align__(16) float Ks[RC * R1_P], Vs[RC * R1_D];
+    __shared__ float pw[RC + 1], wt[RC];
+    ng_pdl_trigger();
+    const int e = blockIdx.x, c = blockIdx.y, head = blockIdx.z, tid = threadIdx.x;
+    const int q0 = cu_q[e], qlen = cu_q[e + 1] - q0;
+    const int n = min(RC, qlen - c * RC);
+    ret_powers(pw, decay[head]);
+    __syncthreads();
+    if (tid < RC) wt[tid] = tid < n ? pw[n - 1 - tid] : 0.f;
+    ng_pdl_wait();
+    x = ng_after_wait(x);
+    if (n <= 0) return;
+    __syncthreads();
+    const size_t ld = 4 * (size_t)nH * R1_D;
+    const T* row = x + (size_t)(q0 + c * RC) * ld + (size_t)head * R1_D;
+    r1_load_qk<T, false>(row, row + (size_t)nH * R1_D, ld, n, ctx_before[e] + c * RC, inv_freq, rot_dims, rsqrtf((float)R1_D), wt, nullptr, Ks);
+    r1_load_v(row + 2 * (size_t)nH * R1_D, ld, n, Vs);
+    __syncthreads();
+    // rows d0 .. and d0 + 64 .., columns c0 .. and c0 + 64 .., four each
+    const int d0 = (tid / 16) * 4, c0 = (tid % 16) * 4;
+    float acc[8][8] = {};
+    for (int j = 0; j < n; ++j) {
+        const float4 k0 = r1_ld4(Ks + j * R1_P + d0), k1 = r1_ld4(Ks + j * R1_P + d0 + 64);
+        const float4 v0 = r1_ld4(Vs + j * R1_D + c0), v1 = r1_ld4(Vs + j * R1_D + c0 + 64);
+        const float kk[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w}, vv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+            for (int cc = 0; cc < 8; ++cc) acc[r][cc] = fmaf(kk[r], vv[cc], acc[r][cc]);
+    }
+    float* U = u_scratch + (((size_t)(q0 / RC + e + c)) * nH + head) * R1_D * R1_D;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        float* d = U + (size_t)(d0 + (r & 3) + (r >> 2) * 64) * R1_D + c0;
+        *reinterpret_cast<float4*>(d) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        *reinterpret_cast<float4*>(d + 64) = make_float4(acc[r][4], acc[r][5], acc[r][6], acc[r][7]);
+    }
+}
+
+#define R1_PIECE 32                      // rows of the state of a buffer
+#define R1_OUT_SMEM ((2 * RC * R1_P + RC * R1_D + RC * (RC + 4) + 2 * R1_PIECE * R1_D) * 4)
+
+template <typename T>
+__global__ void __launch_bounds__(R1_THREADS, 2)
+retention_out128_kernel(const T* __restrict__ x, const float* __restrict__ inv_freq, const float* __restrict__ decay,
+                        const float* __restrict__ u_scratch, T* __restrict__ out, const int* __restrict__ cu_q,
+                        const int* __restrict__ ctx_before, int nH, int rot_dims, float eps) {
+    extern __shared__ __align__(16) float r1_sm[];
+    float* Qs = r1_sm;                       // [RC][R1_P]
+    float* Ks = Qs + RC * R1_P;              // [RC][R1_P]
+    float* Vs = Ks + RC * R1_P;              // [RC][128]
+    float* As = Vs + RC * R1_D;              // [RC][RC + 4]
+    float* Ss = As + RC * (RC + 4);          // [2][32][128]
+    __shared__ float pw[RC + 1], red[4][RC];
+    constexpr int LDA = RC + 4;
+    ng_pdl_trigger();
+    const int e = blockIdx.x, c = blockIdx.y, head = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int q0 = cu_q[e], qlen = cu_q[e + 1] - q0;
+    const int n = min(RC, qlen - c * RC);
+    ret_powers(pw, decay[head]);
+    ng_pdl_wait();
+    if (n <= 0) return;
+    const float* Sb = ng_after_wait(u_scratch) + (((size_t)(q0 / RC + e + c)) * nH + head) * R1_D * R1_D;
+    auto request = [&](int piece) {
+        float* d = Ss + (piece & 1) * R1_PIECE * R1_D;
+#pragma unroll
+        for (int u = 0; u < R1_PIECE * R1_D / 4 / R1_THREADS; ++u) {
+            const int i = (tid + u * R1_THREADS) * 4;
+            const uint32_t a = (uint32_t)__cvta_generic_to_shared(d + i);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(Sb + piece * R1_PIECE * R1_D + i) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    request(0);
+    request(1);
+    const size_t ld = 4 * (size_t)nH * R1_D;
+    const T* row = ng_after_wait(x) + (size_t)(q0 + c * RC) * ld + (size_t)head * R1_D;
+    r1_load_qk<T, true>(row, row + (size_t)nH * R1_D, ld, n, ctx_before[e] + c * RC, inv_freq, rot_dims, rsqrtf((float)R1_D), nullptr, Qs, Ks);
+    r1_load_v(row + 2 * (size_t)nH * R1_D, ld, n, Vs);
+    __syncthreads();
+    {   // A: rows i, i + 16, columns j, j + 16; the lanes of a warp read 4 + 8 rows
+        const int i = (warp & 3) * 4 + (lane >> 3), j = (warp >> 2) * 8 + (lane & 7);
+        float a[2][2] = {};
+#pragma unroll 8
+        for (int d = 0; d < R1_D; d += 4) {
+            const float4 qv[2] = {r1_ld4(Qs + i * R1_P + d), r1_ld4(Qs + (i + 16) * R1_P + d)};
+            const float4 kv[2] = {r1_ld4(Ks + j * R1_P + d), r1_ld4(Ks + (j + 16) * R1_P + d)};
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int cc = 0; cc < 2; ++cc)
+                    a[r][cc] = fmaf(qv[r].w, kv[cc].w, fmaf(qv[r].z, kv[cc].z, fmaf(qv[r].y, kv[cc].y, fmaf(qv[r].x, kv[cc].x, a[r][cc]))));
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc) {
+                const int ii = i + 16 * r, jj = j + 16 * cc;
+                As[ii * LDA + jj] = jj <= ii ? a[r][cc] * pw[ii - jj] : 0.f;
+            }
+    }
+    // o: four rows and four columns a thread; from the state (Q S) and inside the chunk (A V), kept apart until the end.  A
+    // warp covers 16 rows and 32 columns.
+    const int i0 = (warp & 1) * 16 + (lane >> 3) * 4, c0 = (warp >> 1) * 32 + (lane & 7) * 4;
+    float st[4][4] = {}, in[4][4] = {};
+    auto add = [&](float (&o)[4][4], const float* left, int ldl, const float* right) {       // four columns of left, four rows of right
+        float4 l[4], rr[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) l[r] = r1_ld4(left + (i0 + r) * ldl);
+#pragma unroll
+        for (int d = 0; d < 4; ++d) rr[d] = r1_ld4(right + d * R1_D + c0);
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float q = d == 0 ? l[r].x : d == 1 ? l[r].y : d == 2 ? l[r].z : l[r].w;
+                o[r][0] = fmaf(q, rr[d].x, o[r][0]);
+                o[r][1] = fmaf(q, rr[d].y, o[r][1]);
+                o[r][2] = fmaf(q, rr[d].z, o[r][2]);
+                o[r][3] = fmaf(q, rr[d].w, o[r][3]);
+            }
+    };
+#pragma unroll 1
+    for (int piece = 0; piece < R1_D / R1_PIECE; ++piece) {
+        if (piece + 1 < R1_D / R1_PIECE) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const float* S = Ss + (piece & 1) * R1_PIECE * R1_D;
+#pragma unroll 4
+        for (int d = 0; d < R1_PIECE; d += 4) add(st, Qs + piece * R1_PIECE + d, R1_P, S + d * R1_D);
+        __syncthreads();
+        if (piece + 2 < R1_D / R1_PIECE) request(piece + 2);
+    }
+#pragma unroll 4
+    for (int j = 0; j < RC; j += 4) add(in, As + j, LDA, Vs + j * R1_D);
+    float ss[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        ss[r] = 0.f;
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+            in[r][cc] += pw[i0 + r + 1] * st[r][cc];
+            ss[r] += in[r][cc] * in[r][cc];
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], o);
+        if ((lane & 7) == 0) red[warp >> 1][i0 + r] = ss[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int t = i0 + r;
+        if (t >= n) continue;
+        const float f = rsqrtf(((red[0][t] + red[1][t]) + (red[2][t] + red[3][t])) / (float)R1_D + eps);
+        const float4 g = r1_ld4(row + (size_t)t * ld + 3 * (size_t)nH * R1_D + c0);
+        r1_st4(out + ((size_t)(q0 + c * RC + t) * nH + head) * R1_D + c0,
+               make_float4(in[r][0] * f * (g.x / (1.f + expf(-g.x))), in[r][1] * f * (g.y / (1.f + expf(-g.y))),
+                           in[r][2] * f * (g.z / (1.f + expf(-g.z))), in[r][3] * f * (g.w / (1.f + expf(-g.w)))));
+    }
+}
+
 static int retention_chunk_slice(int dv) { return dv % 32 == 0 ? 32 : dv; }
 static size_t retention_out_smem(int dk, int dv) {
     const int dvs = retention_chunk_slice(dv);
@@ -432,6 +674,27 @@ NG_EXPORT int ng_retention_chunked(const void* x, const float* inv_freq, int rot
     dim3 grid(n_entries, (max_q + RC - 1) / RC, nH * (dv / dvs));
     dim3 sgrid((dk * dv + 255) / 256, n_entries, nH);
     if (grid.y > 65535 || grid.z > 65535 || sgrid.y > 65535 || sgrid.z > 65535) return NG_BAD_SIZE;
+    // 16-byte accesses to rows of the activation type and to the chunks' states
+    if (dk == R1_D && dv == R1_D && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)u_scratch) & 15) == 0) {
+        static bool set[2] = {false, false};
+        dim3 hgrid(n_entries, grid.y, nH);
+#define R1_GO(T)                                                                                                       \
+    do {                                                                                                               \
+        if (!set[which]) {                                                                                             \
+            if (cudaFuncSetAttribute(retention_out128_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, R1_OUT_SMEM) != cudaSuccess) \
+                return NG_LAUNCH_FAILED;                                                                               \
+            set[which] = true;                                                                                         \
+        }                                                                                                              \
+        NG_LAUNCH((retention_local128_kernel<T>), hgrid, R1_THREADS, 0, stream, (const T*)x, inv_freq, decay, u_scratch, cu_q, \
+                  ctx_before, nH, rot_dims);                                                                           \
+        NG_LAUNCH((retention_scan_kernel), sgrid, 256, 0, stream, u_scratch, state, decay, cu_q, ctx_before, slots, nH, dk, dv); \
+        NG_LAUNCH((retention_out128_kernel<T>), hgrid, R1_THREADS, R1_OUT_SMEM, stream, (const T*)x, inv_freq, decay,  \
+                  (const float*)u_scratch, (T*)out, cu_q, ctx_before, nH, rot_dims, eps);                              \
+        return ng_launch_status();                                                                                     \
+    } while (0)
+        if (act_bf16) R1_GO(__nv_bfloat16);
+        R1_GO(float);
+    }
     const unsigned nblocks = (unsigned)(((size_t)n_rows * nH + 7) / 8);
     const size_t sl = retention_local_smem(dk, dv), so = retention_out_smem(dk, dv);
     if (act_bf16) {

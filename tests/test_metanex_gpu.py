@@ -182,6 +182,30 @@ def test_retention_chunk_kernel(dtype, heads, dk, dv, rot):
     assert torch.allclose(state[0], state[1], rtol=1e-3, atol=1e-4) and torch.allclose(state[0], state[2], rtol=1e-3, atol=1e-4)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("lens,rot", [([1, 32, 33, 64, 95], 64), ([545, 3], 128), ([31, 600], 0)])
+def test_retention_chunks_of_128(dtype, lens, rot):
+    """Heads of 128 x 128, chunk by chunk, several requests side by side, with and without a state behind them: against the
+    token-by-token kernel (float32 sums in another order; the bound is the activation type's rounding)."""
+    heads, d = 3, 128
+    n = sum(lens)
+    g = torch.Generator().manual_seed(n)
+    x = (torch.randn(n, 4 * heads * d, generator=g)).to(dtype).to(DEV)
+    inv = (300.0 ** (-2.0 * torch.arange(rot // 2, dtype=torch.float64) / max(rot, 1))).float().to(DEV) if rot else None
+    decay = torch.tensor([0.999, 0.9, 1.0], device=DEV)
+    ctx = make_ctx(lens, [5 * (i % 2) for i in range(len(lens))], list(range(len(lens))), dtype=dtype)
+    state = torch.randn(len(lens) + 1, heads, d, d, generator=g).to(DEV)
+    res = []
+    for chunked in (False, True):
+        st, o = state.clone(), torch.empty(n, heads * d, dtype=dtype, device=DEV)
+        kw = dict(scratch=torch.empty(n, heads * d, device=DEV), max_q=max(lens), state_scratch=torch.empty(
+            ops.retention_chunked_scratch(n, len(lens), heads, d, d), device=DEV)) if chunked else {}
+        ops.retention(x, inv, rot, decay, st, o, ctx.cu_q, ctx.ctx_before, ctx.slots, len(lens), heads, d, d, 1e-5, **kw)
+        res.append((o, st))
+    assert rel_err(res[1][0], res[0][0]) < (1e-5 if dtype == torch.float32 else 2.0 ** -7)
+    assert rel_err(res[1][1], res[0][1]) < 1e-5 and torch.equal(res[1][1][-1], state[-1])
+
+
 def test_retention_reads_a_far_key():
     """One key, 700 tokens back, is made to stand out for the last query (same direction, large): a head that decays
     slowly must still answer with its value, a head that decays fast must not."""
