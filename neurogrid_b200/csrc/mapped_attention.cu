@@ -33,8 +33,17 @@
 #define MA_MAX_PAIRS 8    // pairs of a head per lane in the prep kernel: d <= 512
 
 // ------------------------------------------------------------------------------------------ prep
-// OWN_V: value heads are normed or mixed (a form of its own: the others' values are copied as they are)
-template <typename T, bool OWN_V>
+// OWN_V: value heads are normed or mixed (a form of its own: the others' values are copied as they are).  PAIRS: pairs of
+// a head a lane holds (d <= 64 * PAIRS).  HB: heads a warp takes at a time, their loads in flight together (steps of
+// many rows, where one block walks all heads of its row).  `wide`: neighbouring pairs, and values in pieces of 16 bytes,
+// lie where one access reaches them.  2,048 rows of 32 + 8 heads of 64: 21.3 us (38.9 us with loads of one element, one
+// head at a time and eight pairs' worth of predicated code); 8 rows inside a step's graph: 2.7 us (5.2 us).
+__device__ __forceinline__ float2 prep_ld2(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
+__device__ __forceinline__ float2 prep_ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ void prep_st2(__nv_bfloat16* p, float a, float b) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b); }
+__device__ __forceinline__ void prep_st2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+
+template <typename T, bool OWN_V, int PAIRS, int HB>
 __global__ void __launch_bounds__(MA_THREADS)
 qkv_prep_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, const float* __restrict__ qw,
                 const float* __restrict__ kw, const float* __restrict__ inv_freq, int rot_dims,
@@ -42,7 +51,7 @@ qkv_prep_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, const float* _
                 const int* __restrict__ positions, const int* __restrict__ row_entry, int nQ, int nK, int nV, int d,
                 int dv, int page_size, int num_pages, float eps, int* __restrict__ status, int whole, float temp_coef,
                 int temp_every, int ld, int half_pairing, int unit_norm, int v_is_k, float rot_mag, int v_norm, int v_mode,
-                float v_lambda, float* __restrict__ v_first) {
+                float v_lambda, float* __restrict__ v_first, int wide) {
     extern __shared__ float rot[];                      // cos[rot_dims/2], sin[rot_dims/2]
     __shared__ float red[32];
     ng_pdl_trigger();
@@ -57,24 +66,24 @@ qkv_prep_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, const float* _
         rot[i] = c * rot_mag;
         rot[half_rot + i] = s * rot_mag;
     }
+    size_t k_base = 0, v_base = 0;
+    bool page_ok = true;
+    if (entry >= 0 && nK + nV > 0) {
+        const int page = table[(size_t)entry * table_stride + pos / page_size];
+        page_ok = page >= 0 && page < num_pages;
+        const size_t p = page_ok ? page : 0, slot = pos % page_size;
+        k_base = (p * nK * page_size + slot) * d;
+        v_base = (p * nV * page_size + slot) * dv;
+    }
     __syncthreads();
     ng_pdl_wait();
     qkv = ng_after_wait(qkv);
     const T* in = qkv + (size_t)row * ld;             // ld: a row's pitch (columns behind v belong to the caller)
     T* qo = q_out + (size_t)row * nQ * d;
+    if (!page_ok && threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, NG_STATUS_BAD_PAGE);
     if (entry < 0) {                                   // padding row: defined output, no cache write
         for (int j = blockIdx.y * MA_THREADS + threadIdx.x; j < nQ * d; j += MA_THREADS * gridDim.y) ng_st(qo + j, 0.f);
         return;
-    }
-    size_t k_base = 0, v_base = 0;
-    bool page_ok = true;
-    if (nK + nV > 0) {
-        const int page = table[(size_t)entry * table_stride + pos / page_size];
-        page_ok = page >= 0 && page < num_pages;
-        if (!page_ok && threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, NG_STATUS_BAD_PAGE);
-        const size_t p = page_ok ? page : 0, slot = pos % page_size;
-        k_base = (p * nK * page_size + slot) * d;
-        v_base = (p * nV * page_size + slot) * dv;
     }
     const int half = d / 2;
     // one norm over all of the row's q and one over all of its k: every block of the row forms both sums itself
@@ -90,61 +99,78 @@ qkv_prep_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, const float* _
     }
     const float temp = temp_coef != 0.f ? 1.f + temp_coef * logf((float)((pos + 1) / temp_every + 1)) : 1.f;
     // few rows: the heads are dealt over gridDim.y blocks of a row; many rows: one block walks all heads of its row
-    for (int hh = blockIdx.y * MA_WARPS + warp; hh < nQ + nK; hh += MA_WARPS * gridDim.y) {
-        const bool is_q = hh < nQ;
-        if (!is_q && !page_ok) continue;
-        const T* src = in + (size_t)hh * d;
-        const float* w = is_q ? qw : kw;
-        if (w && whole) w += (size_t)(is_q ? hh : hh - nQ) * d;        // a weight per coordinate of the projection
-        const float post = is_q ? temp : 1.f;
-        float x1[MA_MAX_PAIRS], x2[MA_MAX_PAIRS];
-        float ss = 0.f;
+    for (int h0 = (blockIdx.y * MA_WARPS + warp) * HB; h0 < nQ + nK; h0 += MA_WARPS * gridDim.y * HB) {
+        float x1[HB][PAIRS], x2[HB][PAIRS], odd[HB];
 #pragma unroll
-        for (int u = 0; u < MA_MAX_PAIRS; ++u) {
-            const int i = lane + 32 * u;
-            x1[u] = x2[u] = 0.f;
-            if (i < half) {
-                // pair i: (2i, 2i+1), or with half pairing (i, i + rot_dims/2) inside the rotated coordinates
-                const bool hp = half_pairing && i < half_rot;
-                x1[u] = ng_ld(src + (hp ? i : 2 * i));
-                x2[u] = ng_ld(src + (hp ? i + half_rot : 2 * i + 1));
-            }
-            ss += x1[u] * x1[u] + x2[u] * x2[u];
-        }
-        if ((d & 1) && lane == 0) {                     // an odd last coordinate has no partner
-            const float t = ng_ld(src + d - 1);
-            ss += t * t;
-        }
-        float r = 1.f;
-        if (w) r = whole ? (is_q ? r_q : r_k) : rsqrtf(ng_warp_sum(ss) / (float)d + eps);
-        // a norm without weights: a rotation does not change a head's sum of squares, so the factor of the
-        // unrotated head is the factor of the rotated one
-        else if (unit_norm) r = rsqrtf(ng_warp_sum(ss) / (float)d + eps);
-        T* dst = is_q ? qo + (size_t)hh * d : k_pages + k_base + (size_t)(hh - nQ) * page_size * d;
+        for (int hb = 0; hb < HB; ++hb) {
+            const T* src = in + (size_t)min(h0 + hb, nQ + nK - 1) * d;
 #pragma unroll
-        for (int u = 0; u < MA_MAX_PAIRS; ++u) {
-            const int i = lane + 32 * u;
-            if (i < half) {
-                const bool hp = half_pairing && i < half_rot;
-                const int c1 = hp ? i : 2 * i, c2 = hp ? i + half_rot : 2 * i + 1;
-                float y1 = x1[u], y2 = x2[u];
-                if (w) { y1 = y1 * r * w[c1]; y2 = y2 * r * w[c2]; }
-                else if (unit_norm) { y1 *= r; y2 *= r; }
-                y1 *= post; y2 *= post;
-                if (i < half_rot) {
-                    const float c = rot[i], s = rot[half_rot + i];
-                    const float z1 = y1 * c - y2 * s, z2 = y2 * c + y1 * s;
-                    y1 = z1; y2 = z2;
+            for (int u = 0; u < PAIRS; ++u) {
+                const int i = lane + 32 * u;
+                x1[hb][u] = x2[hb][u] = 0.f;
+                if (i < half) {
+                    // pair i: (2i, 2i+1), or with half pairing (i, i + rot_dims/2) inside the rotated coordinates
+                    const bool hp = half_pairing && i < half_rot;
+                    if (wide && !hp) {
+                        const float2 f = prep_ld2(src + 2 * i);
+                        x1[hb][u] = f.x;
+                        x2[hb][u] = f.y;
+                    } else {
+                        x1[hb][u] = ng_ld(src + (hp ? i : 2 * i));
+                        x2[hb][u] = ng_ld(src + (hp ? i + half_rot : 2 * i + 1));
+                    }
                 }
-                ng_st(dst + c1, y1);
-                ng_st(dst + c2, y2);
             }
+            odd[hb] = (d & 1) && lane == 0 ? ng_ld(src + d - 1) : 0.f;      // an odd last coordinate has no partner
         }
-        if ((d & 1) && lane == 0) {
-            float t = ng_ld(src + d - 1);
-            if (w) t = t * r * w[d - 1];
-            else if (unit_norm) t *= r;
-            ng_st(dst + d - 1, t * post);
+#pragma unroll
+        for (int hb = 0; hb < HB; ++hb) {
+            const int hh = h0 + hb;
+            const bool is_q = hh < nQ;
+            if (hh >= nQ + nK) break;
+            if (!is_q && !page_ok) continue;
+            const float* w = is_q ? qw : kw;
+            if (w && whole) w += (size_t)(is_q ? hh : hh - nQ) * d;        // a weight per coordinate of the projection
+            const float post = is_q ? temp : 1.f;
+            float ss = 0.f;
+#pragma unroll
+            for (int u = 0; u < PAIRS; ++u) ss += x1[hb][u] * x1[hb][u] + x2[hb][u] * x2[hb][u];
+            ss += odd[hb] * odd[hb];
+            float r = 1.f;
+            if (w) r = whole ? (is_q ? r_q : r_k) : rsqrtf(ng_warp_sum(ss) / (float)d + eps);
+            // a norm without weights: a rotation does not change a head's sum of squares, so the factor of the
+            // unrotated head is the factor of the rotated one
+            else if (unit_norm) r = rsqrtf(ng_warp_sum(ss) / (float)d + eps);
+            T* dst = is_q ? qo + (size_t)hh * d : k_pages + k_base + (size_t)(hh - nQ) * page_size * d;
+#pragma unroll
+            for (int u = 0; u < PAIRS; ++u) {
+                const int i = lane + 32 * u;
+                if (i < half) {
+                    const bool hp = half_pairing && i < half_rot;
+                    const int c1 = hp ? i : 2 * i, c2 = hp ? i + half_rot : 2 * i + 1;
+                    float y1 = x1[hb][u], y2 = x2[hb][u];
+                    if (w) { y1 = y1 * r * w[c1]; y2 = y2 * r * w[c2]; }
+                    else if (unit_norm) { y1 *= r; y2 *= r; }
+                    y1 *= post; y2 *= post;
+                    if (i < half_rot) {
+                        const float c = rot[i], s = rot[half_rot + i];
+                        const float z1 = y1 * c - y2 * s, z2 = y2 * c + y1 * s;
+                        y1 = z1; y2 = z2;
+                    }
+                    if (wide && !hp) {
+                        prep_st2(dst + c1, y1, y2);
+                    } else {
+                        ng_st(dst + c1, y1);
+                        ng_st(dst + c2, y2);
+                    }
+                }
+            }
+            if ((d & 1) && lane == 0) {
+                float t = odd[hb];
+                if (w) t = t * r * w[d - 1];
+                else if (unit_norm) t *= r;
+                ng_st(dst + d - 1, t * post);
+            }
         }
     }
     if (page_ok) {
@@ -174,6 +200,14 @@ qkv_prep_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, const float* _
             }
             return;
         }
+        constexpr int V16 = 16 / sizeof(T);
+        if (wide && dv % V16 == 0) {
+            for (int j = (blockIdx.y * MA_THREADS + threadIdx.x) * V16; j < nV * dv; j += MA_THREADS * gridDim.y * V16) {
+                const int hv = j / dv, c = j - hv * dv;
+                *reinterpret_cast<uint4*>(v_pages + v_base + (size_t)hv * page_size * dv + c) = *reinterpret_cast<const uint4*>(vs + j);
+            }
+            return;
+        }
         for (int j = blockIdx.y * MA_THREADS + threadIdx.x; j < nV * dv; j += MA_THREADS * gridDim.y) {
             const int hv = j / dv, c = j - hv * dv;
             v_pages[v_base + (size_t)hv * page_size * dv + c] = vs[j];
@@ -199,18 +233,28 @@ NG_EXPORT int ng_qkv_prep(const void* qkv, void* q_out, const float* qw, const f
     const size_t smem = (size_t)rot_dims * sizeof(float);
     const int head_blocks = n_rows >= 256 ? 1 : min(64, (nQ + nK + MA_WARPS - 1) / MA_WARPS);
     const dim3 grid(n_rows, head_blocks);
-#define PREP_LAUNCH(TT, OWN)                                                                                           \
-    NG_LAUNCH((qkv_prep_kernel<TT, OWN>), grid, MA_THREADS, smem, stream, (const TT*)qkv, (TT*)q_out, qw, kw, inv_freq, \
-              rot_dims, (TT*)k_pages, (TT*)v_pages, table, table_stride, positions, row_entry, nQ, nK, nV, d, dv,      \
+    // every row, head and page slot on a 16-byte boundary: the projection's columns in front of v are whole pieces too
+    const int el = act_bf16 ? 8 : 4;
+    const bool wide = d % el == 0 && dv % el == 0 && ld % el == 0 &&
+                      (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0;
+#define PREP_LAUNCH(TT, OWN, PAIRS, HB)                                                                                \
+    NG_LAUNCH((qkv_prep_kernel<TT, OWN, PAIRS, HB>), grid, MA_THREADS, smem, stream, (const TT*)qkv, (TT*)q_out, qw, kw, \
+              inv_freq, rot_dims, (TT*)k_pages, (TT*)v_pages, table, table_stride, positions, row_entry, nQ, nK, nV, d, dv, \
               page_size, num_pages, eps, status, whole, temp_coef, temp_every, ld, half_pairing, unit_norm, v_is_k,    \
-              rot_mag, v_norm, v_mode, v_lambda, v_first)
+              rot_mag, v_norm, v_mode, v_lambda, v_first, (int)wide)
+#define PREP_SIZES(TT, OWN)                                                                                            \
+    do {                                                                                                               \
+        if (d <= 64) { if (head_blocks == 1) PREP_LAUNCH(TT, OWN, 1, 4); else PREP_LAUNCH(TT, OWN, 1, 1); }            \
+        else if (d <= 128) { if (head_blocks == 1) PREP_LAUNCH(TT, OWN, 2, 4); else PREP_LAUNCH(TT, OWN, 2, 1); }      \
+        else PREP_LAUNCH(TT, OWN, MA_MAX_PAIRS, 1);                                                                    \
+    } while (0)
     const bool own_v = (v_norm || v_mode) && nV > 0;
     if (act_bf16) {
-        if (own_v) PREP_LAUNCH(__nv_bfloat16, true);
-        else PREP_LAUNCH(__nv_bfloat16, false);
+        if (own_v) PREP_SIZES(__nv_bfloat16, true);
+        else PREP_SIZES(__nv_bfloat16, false);
     } else {
-        if (own_v) PREP_LAUNCH(float, true);
-        else PREP_LAUNCH(float, false);
+        if (own_v) PREP_SIZES(float, true);
+        else PREP_SIZES(float, false);
     }
     return ng_launch_status();
 }
@@ -558,31 +602,4 @@ NG_EXPORT int ng_mapped_attention(const void* q, const void* k_pages, const void
                head_norm, slopes, sinks, sigmoid, score_bias, gate, gate_ld};
     if (act_bf16) return n_maps == 2 ? ma_launch<__nv_bfloat16, 2>(p, n_rows, stream) : ma_launch<__nv_bfloat16, 1>(p, n_rows, stream);
     return n_maps == 2 ? ma_launch<float, 2>(p, n_rows, stream) : ma_launch<float, 1>(p, n_rows, stream);
-}
-
-// The runs' states of every (row, head) merged and the heads finished (maps combined, head norm), for states that another
-// kernel left in `partial` (float32 [n_rows, nH, n_splits, n_maps, dv + 2]: maximum, sum, weighted values).  Rows of no
-// entry get zeros.  `sinks` (per head, or null) adds exp(sink) to every head's sum.  `sigmoid`: the weights are not
-// normalised (the states' maxima are 0 and their sums not read); `gate` as above.
-NG_EXPORT int ng_mapped_attention_merge(float* partial, const int* row_entry, void* out, int out_ld, int n_rows, int nH,
-                                        int n_maps, int dv, int n_splits, float lambda, float post_scale, float eps,
-                                        int head_norm, const float* sinks, int sigmoid, const void* gate, int gate_ld, int act_bf16,
-                                        cudaStream_t stream) {
-    if (n_rows <= 0) return NG_OK;
-    if (!partial || dv <= 0 || dv > 64 * MA_DVU || nH <= 0 || nH > 65535 || n_maps < 1 || n_maps > 2 || n_splits < 1 || out_ld < nH * dv ||
-        (sigmoid && (n_maps != 1 || sinks)) || (gate && gate_ld < nH))
-        return NG_BAD_SIZE;
-    MaParams p{nullptr, nullptr, nullptr, nullptr, 0, nullptr, row_entry, out, out_ld, partial, nH, 1, 0, dv, 1, 0, 0, 0, n_splits, 0,
-               0.f, 0.f, lambda, post_scale, eps, head_norm, nullptr, sinks, sigmoid, nullptr, gate, gate_ld};
-    dim3 grid(n_rows, nH);
-    const size_t smem = ((size_t)n_maps * dv + n_splits) * sizeof(float);
-    if (smem > 48 * 1024) return NG_BAD_SIZE;
-    if (act_bf16) {
-        if (n_maps == 2) NG_LAUNCH((mapped_attention_merge_kernel<__nv_bfloat16, 2>), grid, MA_THREADS, smem, stream, p);
-        else NG_LAUNCH((mapped_attention_merge_kernel<__nv_bfloat16, 1>), grid, MA_THREADS, smem, stream, p);
-    } else {
-        if (n_maps == 2) NG_LAUNCH((mapped_attention_merge_kernel<float, 2>), grid, MA_THREADS, smem, stream, p);
-        else NG_LAUNCH((mapped_attention_merge_kernel<float, 1>), grid, MA_THREADS, smem, stream, p);
-    }
-    return ng_launch_status();
 }

@@ -40,7 +40,7 @@ struct MmaParams {
     int nH, nG, page_size, num_pages, window, keep_first;
     int chunk;                         // > 0: a row sees only the keys of its own chunk of that many positions (counted from 0)
     float scale, softcap, lambda, post_scale, eps; int head_norm;
-    float* partial; int n_splits;      // GROUP: runs of keys, their states [row, head, run, map, DV + 2]
+    int n_splits, n_rows; const int* row_entry;       // GROUP: runs of keys (a cluster's blocks); rows of no entry get zeros
     const float* slopes; const float* sinks;    // per head or null: slope * (pos - key position) off every score; exp(sink) in the sum
     const float* score_bias;           // SIGMOID: added to head h's scores, or null
     const bf16* gate; int gate_ld;     // a logit per row and head, rows gate_ld apart, or null
@@ -106,7 +106,7 @@ template <int M>
 constexpr size_t smem_bytes() {
     constexpr size_t ROWS = (WARPS / M) * 16;
     constexpr size_t tiles = (M * ROWS * QP + 2 * ((size_t)M * KT * KP + (size_t)KT * VP)) * sizeof(bf16);
-    constexpr size_t epi = M * ROWS * QP * sizeof(bf16) + (M * ROWS > 64 ? M * ROWS : 64) * DV * sizeof(float);
+    constexpr size_t epi = M * ROWS * QP * sizeof(bf16) + ((M * ROWS > 64 ? M * ROWS : 64) * DV + 16 * M * (DV + 2)) * sizeof(float);
     return tiles > epi ? tiles : epi;
 }
 // blocks of an SM that its shared memory holds (227 KB, 1 KB of each block's own): the registers are shared out to as many
@@ -133,8 +133,18 @@ mapped_attention_mma_kernel(const MmaParams p) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int q0 = p.cu_q[entry], q_len = p.cu_q[entry + 1] - q0;
     const int r0 = GROUP ? 0 : blockIdx.x * ROWS;        // first row of the block within the entry
-    ng_pdl_wait();
-    if (GROUP ? q_len != 1 : r0 >= q_len) return;
+    if (GROUP && blockIdx.x == 0) {                      // rows of no entry: defined output (row r is looked at by entry r mod entries)
+        const int cols = (p.nH / p.nG) * DV;
+        for (int r = entry; r < p.n_rows; r += gridDim.y)
+            if (p.row_entry[r] < 0) {
+                ng_pdl_wait();
+                for (int c = tid; c < cols; c += THREADS) p.out[(size_t)r * p.out_ld + (size_t)blockIdx.z * cols + c] = __float2bfloat16_rn(0.f);
+            }
+    }
+    if (GROUP ? q_len != 1 : r0 >= q_len) {              // (all blocks of a cluster leave here, or none)
+        ng_pdl_wait();
+        return;
+    }
     const int before = p.ctx_before[entry];
     const int group_heads = p.nH / p.nG;
     const int n_rows = GROUP ? group_heads : min(ROWS, q_len - r0);
@@ -143,21 +153,6 @@ mapped_attention_mma_kernel(const MmaParams p) {
     const int map = M == 2 ? (warp & 1) : 0;
     const int wt = GROUP ? 0 : M == 2 ? (warp >> 1) : warp;              // the warp's tile of 16 rows
     const int k_off = GROUP ? (M == 2 ? (warp >> 1) : warp) * KW : 0;    // ... and its first key of every tile
-    const bf16* qg = ng_after_wait(p.q);
-    // ---- Q: rows r0.., both maps, into shared memory (rows beyond the entry: zeros)
-    for (int i = tid; i < M * ROWS * (D / 8); i += THREADS) {
-        const int ch = i % (D / 8), row = (i / (D / 8)) % ROWS, m = i / ((D / 8) * ROWS);
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (row < n_rows)
-            v = *reinterpret_cast<const uint4*>(qg + ((size_t)(q0 + (GROUP ? 0 : r0 + row)) * p.nH + head + (GROUP ? row : 0)) * M * D +
-                                                (size_t)m * D + ch * 8);
-        *reinterpret_cast<uint4*>(Qs + ((size_t)m * ROWS + row) * QP + ch * 8) = v;
-    }
-    __syncthreads();
-    uint32_t qf[D / 16][4];
-#pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks)
-        ldsm_x4(qf[ks], Qs + ((size_t)map * ROWS + wt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * QP + ks * 16 + (lane >> 4) * 8);
     // ---- the keys the block's rows see: kept first tokens [0, n_sink), then [lo, last position]
     const int pos_first = before + r0, pos_last = GROUP ? pos_first : before + r0 + n_rows - 1;
     int lo = p.window > 0 ? max(0, pos_first - p.window + 1) : 0;
@@ -238,7 +233,27 @@ mapped_attention_mma_kernel(const MmaParams p) {
     };
     lookup(t_begin, 0);
     __syncthreads();
-    copy_tile(0, 0);
+    // the first tile, if all its keys are older than the step (an earlier step wrote them), before the wait
+    const int t_old = min(n_keys, t_begin + KT) - 1;
+    const bool old_tile = t_old < t_begin || (t_old < n_sink ? t_old : lo + (t_old - n_sink)) < before;
+    if (old_tile) copy_tile(0, 0);
+    ng_pdl_wait();
+    const bf16* qg = ng_after_wait(p.q);
+    // ---- Q: rows r0.., both maps, into shared memory (rows beyond the entry: zeros)
+    for (int i = tid; i < M * ROWS * (D / 8); i += THREADS) {
+        const int ch = i % (D / 8), row = (i / (D / 8)) % ROWS, m = i / ((D / 8) * ROWS);
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (row < n_rows)
+            v = *reinterpret_cast<const uint4*>(qg + ((size_t)(q0 + (GROUP ? 0 : r0 + row)) * p.nH + head + (GROUP ? row : 0)) * M * D +
+                                                (size_t)m * D + ch * 8);
+        *reinterpret_cast<uint4*>(Qs + ((size_t)m * ROWS + row) * QP + ch * 8) = v;
+    }
+    __syncthreads();
+    uint32_t qf[D / 16][4];
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks)
+        ldsm_x4(qf[ks], Qs + ((size_t)map * ROWS + wt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * QP + ks * 16 + (lane >> 4) * 8);
+    if (!old_tile) copy_tile(0, 0);
     int buf = 0, it = 0;
     for (int t0 = t_begin; t0 < n_keys; t0 += KT, buf ^= 1, ++it) {
         const bool more = t0 + KT < n_keys;
@@ -375,8 +390,9 @@ mapped_attention_mma_kernel(const MmaParams p) {
     l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
     l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
     if (GROUP) {
-        // the warps' states through shared memory, over the tiles; then, per head and map, their sum in warp order as the
-        // kernel that merges runs reads it: maximum (natural logarithm), sum, weighted values relative to that maximum
+        // the warps' states through shared memory, over the tiles; then, per head and map, their sum in warp order: maximum,
+        // sum and weighted values of the block's run, in the tiles' place as well
+        float* Rs = Os + (size_t)WARPS * 16 * DV;        // [16][M][DV + 2]
         if (tq == 0) {
             part_m[warp][gq] = m_a; part_m[warp][gq + 8] = m_b;
             part_l[warp][gq] = l_a; part_l[warp][gq + 8] = l_b;
@@ -387,7 +403,6 @@ mapped_attention_mma_kernel(const MmaParams p) {
             *reinterpret_cast<float2*>(Os + ((size_t)warp * 16 + gq + 8) * DV + j * 8 + 2 * tq) = make_float2(o[j][2], o[j][3]);
         }
         __syncthreads();
-        constexpr float LN2 = 0.6931471805599453f;
         for (int rm = warp; rm < n_rows * M; rm += WARPS) {
             const int r = rm / M, m = rm % M;            // (the warps of map m are m, m + M, ...)
             float mt = -INFINITY, f[PARTS], lt = 0.f;
@@ -399,8 +414,8 @@ mapped_attention_mma_kernel(const MmaParams p) {
                 f[x] = mx == -INFINITY ? 0.f : ex2f(mx - mt);
                 lt += part_l[m + x * M][r] * f[x];
             }
-            float* ps = p.partial + ((((size_t)q0 * p.nH + head + r) * p.n_splits + blockIdx.x) * M + m) * (DV + 2);
-            if (lane == 0) { ps[0] = mt * LN2; ps[1] = lt; }
+            float* ps = Rs + (size_t)rm * (DV + 2);
+            if (lane == 0) { ps[0] = mt; ps[1] = lt; }
             for (int c = lane; c < DV; c += 32) {
                 float a = 0.f;
 #pragma unroll
@@ -408,6 +423,56 @@ mapped_attention_mma_kernel(const MmaParams p) {
                 ps[2 + c] = a;
             }
         }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        // a warp finishes a head: the runs' states in run order, the maps combined, the head's norm and gate
+        const uint32_t rs = (uint32_t)__cvta_generic_to_shared(Rs);
+        auto state = [&](int run, int idx) {
+            uint32_t a;
+            float v;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(rs + 4 * idx), "r"(run));
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+            return v;
+        };
+        const bf16* gate = ng_after_wait(p.gate);
+        for (int r = blockIdx.x * WARPS + warp; r < n_rows; r += p.n_splits * WARPS) {
+            float v[DV / 32 + 1], ss = 0.f;
+#pragma unroll
+            for (int u = 0; u < DV / 32 + 1; ++u) v[u] = 0.f;
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int at = (r * M + m) * (DV + 2);
+                // a lane per run for the maximum, the factors and the sum
+                const float mr = lane < p.n_splits ? state(lane, at) : -INFINITY, lr = lane < p.n_splits ? state(lane, at + 1) : 0.f;
+                const float mt = ng_warp_max(mr);
+                const float f = mr == -INFINITY ? 0.f : exp2f(mr - mt);
+                float l = ng_warp_sum(lr * f);
+                if (p.sinks) l += exp2f(p.sinks[head + r] * 1.4426950408889634f - mt);      // the term without key or value
+                const float scale = (SIGMOID ? 1.f : l > 0.f ? 1.f / l : 0.f) * (m == 1 ? -p.lambda : 1.f);
+                float acc[DV / 32 + 1];
+#pragma unroll
+                for (int u = 0; u < DV / 32 + 1; ++u) acc[u] = 0.f;
+#pragma unroll 4
+                for (int x = 0; x < p.n_splits; ++x) {
+                    const float fx = __shfl_sync(0xffffffffu, f, x);
+#pragma unroll
+                    for (int u = 0; u < DV / 32 + 1; ++u)
+                        if (lane + 32 * u < DV) acc[u] = fmaf(state(x, at + 2 + lane + 32 * u), fx, acc[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < DV / 32 + 1; ++u) v[u] = fmaf(acc[u], scale, v[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < DV / 32 + 1; ++u) ss += v[u] * v[u];
+            float k = p.post_scale;
+            if (p.gate) k *= rcpf(1.f + ex2f(-1.4426950408889634f * __bfloat162float(gate[(size_t)q0 * p.gate_ld + head + r])));
+            if (p.head_norm) k *= rsqrtf(ng_warp_sum(ss) / (float)DV + p.eps);
+            bf16* dst = p.out + (size_t)q0 * p.out_ld + (size_t)(head + r) * DV;
+#pragma unroll
+            for (int u = 0; u < DV / 32 + 1; ++u)
+                if (lane + 32 * u < DV) dst[lane + 32 * u] = __float2bfloat16_rn(v[u] * k);
+        }
+        // a block's states stay until every block has read them
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
         return;
     }
     if (p.sinks) {                                       // the term without key or value, once per row
@@ -462,6 +527,25 @@ static int mma_launch(const MmaParams& p, int n_entries, int max_q, cudaStream_t
     }
     dim3 grid(GROUP ? p.n_splits : (max_q + ROWS - 1) / ROWS, n_entries, GROUP ? p.nG : p.nH);
     if (grid.y > 65535 || grid.z > 65535) return NG_BAD_SIZE;
+    if (GROUP) {                                         // as ng_launch, the runs as a cluster
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr2[2];
+        memset(attr2, 0, sizeof(attr2));
+        attr2[0].id = cudaLaunchAttributeClusterDimension;
+        attr2[0].val.clusterDim.x = p.n_splits;
+        attr2[0].val.clusterDim.y = attr2[0].val.clusterDim.z = 1;
+        attr2[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr2[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr2;
+        cfg.numAttrs = ng_pdl_enabled() ? 2 : 1;
+        cudaLaunchKernelEx(&cfg, mapped_attention_mma_kernel<M, GROUP>, MmaParams(p));
+        return ng_launch_status();
+    }
     NG_LAUNCH((mapped_attention_mma_kernel<M, GROUP>), grid, THREADS, smem, stream, p);
     return ng_launch_status();
 }
@@ -483,7 +567,7 @@ NG_EXPORT int ng_mapped_attention_mma(const void* q, const void* k_pages, const 
         return NG_BAD_SIZE;
     MmaParams p{(const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, table, table_stride, cu_q, ctx_before, (bf16*)out,
                 out_ld, nH, nG, page_size, num_pages, window, keep_first, chunk, scale, softcap, lambda, post_scale, eps, head_norm,
-                nullptr, 1, slopes, sinks, score_bias, (const bf16*)gate, gate_ld};
+                1, 0, nullptr, slopes, sinks, score_bias, (const bf16*)gate, gate_ld};
 #if !NG_MA_SIGMOID
     if (n_maps == 2) return mma_launch<2, false>(p, n_entries, max_q, stream);
 #endif
@@ -491,24 +575,25 @@ NG_EXPORT int ng_mapped_attention_mma(const void* q, const void* k_pages, const 
 }
 
 // The same for entries of one token: the heads of a KV group are the rows of a tile (nH / nG <= 16), every row's keys are
-// cut into n_splits runs, and each run's state goes to partial (float32 [N, nH, n_splits, n_maps, DV + 2]: maximum, sum,
-// weighted values), from where the kernel that merges runs (mapped_attention.cu) finishes the heads.  Entries of another
-// length are left alone.
+// cut into n_splits runs (at most eight: the blocks of a cluster).  Entries of another length are left alone; the n_rows
+// rows of no entry (row_entry < 0) get zeros.
 NG_EXPORT int ng_mapped_attention_group(const void* q, const void* k_pages, const void* v_pages, const int* table,
-                                        int table_stride, const int* cu_q, const int* ctx_before, float* partial,
-                                        int n_entries, int n_splits, int nH, int nG, int n_maps, int d, int dv, int page_size,
-                                        int num_pages, int window, int keep_first, float scale, float softcap,
-                                        const float* slopes, int chunk, int sigmoid, const float* score_bias,
-                                        cudaStream_t stream) {
+                                        int table_stride, const int* cu_q, const int* ctx_before, const int* row_entry, void* out,
+                                        int out_ld, int n_rows, int n_entries, int n_splits, int nH, int nG, int n_maps, int d,
+                                        int dv, int page_size, int num_pages, int window, int keep_first, float scale,
+                                        float softcap, float lambda, float post_scale, float eps, int head_norm,
+                                        const float* slopes, const float* sinks, int chunk, int sigmoid,
+                                        const float* score_bias, const void* gate, int gate_ld, cudaStream_t stream) {
     if (n_entries <= 0) return NG_OK;
     if (d != D || dv != DV || nH <= 0 || nG <= 0 || nH % nG || nH / nG > 16 || page_size <= 0 || n_maps < 1 || n_maps > 2 ||
-        window < 0 || keep_first < 0 || chunk < 0 || (chunk > 0 && keep_first > 0) || n_splits < 1 || n_splits > 65535 || !partial ||
-        ((uintptr_t)q & 15) ||
-        ((uintptr_t)k_pages & 15) || ((uintptr_t)v_pages & 15) || (sigmoid != 0) != SIGMOID || (SIGMOID && n_maps != 1))
+        window < 0 || keep_first < 0 || chunk < 0 || (chunk > 0 && keep_first > 0) || n_splits < 1 || n_splits > 65535 ||
+        out_ld < nH * dv || ((uintptr_t)q & 15) ||
+        ((uintptr_t)k_pages & 15) || ((uintptr_t)v_pages & 15) || (sigmoid != 0) != SIGMOID || (SIGMOID && (n_maps != 1 || sinks)) ||
+        (gate && gate_ld < nH))
         return NG_BAD_SIZE;
-    MmaParams p{(const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, table, table_stride, cu_q, ctx_before, nullptr, 0,
-                nH, nG, page_size, num_pages, window, keep_first, chunk, scale, softcap, 0.f, 1.f, 0.f, 0, partial, n_splits, slopes,
-                nullptr, score_bias, nullptr, 0};
+    MmaParams p{(const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, table, table_stride, cu_q, ctx_before, (bf16*)out,
+                out_ld, nH, nG, page_size, num_pages, window, keep_first, chunk, scale, softcap, lambda, post_scale, eps, head_norm,
+                n_splits > 8 ? 8 : n_splits, n_rows, row_entry, slopes, sinks, score_bias, (const bf16*)gate, gate_ld};
 #if !NG_MA_SIGMOID
     if (n_maps == 2) return mma_launch<2, true>(p, n_entries, 1, stream);
 #endif

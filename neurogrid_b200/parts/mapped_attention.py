@@ -35,7 +35,7 @@ class MappedAttention:
 
     graph_safe = True      # launches depend on device data and on launch-time constants only
     GROUP_MAX_ROWS = 256   # decode-only steps of up to this many rows run the heads of a KV group as a tensor-core tile
-    GROUP_MAX_RUNS = 512   # ... with rows * runs a row bounded by this
+    GROUP_MAX_RUNS = 8     # ... a row's keys in up to this many runs (the blocks of a cluster)
     SPLIT_MAX_ROWS = 32    # steps of up to this many rows may cut each row's keys into runs
     SPLIT_MIN_KEYS = 128   # ... of at least this many keys (one tile of the kernel)
     MAX_SPLITS = 16
@@ -149,7 +149,7 @@ class MappedAttention:
         """Runs a row's keys are cut into when single tokens run as tiles of a KV group's heads (tiles of 64 keys)."""
         s = self.spec
         want = -(-3 * ops.sm_count(self.device) // max(1, n_rows * s.n_kv_heads))
-        return max(1, min(self.MAX_SPLITS, want, self._longest(cache) // 64, self.GROUP_MAX_RUNS // n_rows))
+        return max(1, min(self.GROUP_MAX_RUNS, want, self._longest(cache) // 64))
 
     # a block arrangement that ends mixer and feed-forward with ONE product calls ``core`` and multiplies itself
     def inner_width(self):
@@ -221,13 +221,8 @@ class MappedAttention:
         if ctx.max_q == 1 and n <= self.GROUP_MAX_ROWS and not ctx.fixed_launches and \
                 ops.mapped_attention_group_takes(s.key_dim, s.value_dim, s.n_heads, s.n_kv_heads, self.dtype):
             n_splits = self._group_splits(n, cache)
-            per_run = ops.mapped_attention_partial_floats(1, s.n_heads, s.n_maps, s.value_dim, 2) // 2
-            # (scratch whose bound follows from the layer's sizes is named after them: a layer of other sizes has its own)
-            partial = ctx.ws.flat(f"mattn_group_partial_{s.n_heads}x{s.n_maps}x{s.value_dim}", n * n_splits * per_run,
-                                  torch.float32,
-                                  reserve=max(self.GROUP_MAX_RUNS, min(ctx.ws.max_rows, self.GROUP_MAX_ROWS)) * per_run)
             ops.mapped_attention_group(q, cache.k_pages, cache.v_pages, cache.table, ctx.cu_q, ctx.ctx_before, ctx.row_entry,
-                                       out, partial, ctx.n_entries, s.n_heads, s.n_maps, s.window, s.keep_first,
+                                       out, None, ctx.n_entries, s.n_heads, s.n_maps, s.window, s.keep_first,
                                        s.softmax_scale, s.softcap or 0.0, self.lam, s.n_maps == 2, 1.0 - s.diff, s.eps, n_splits,
                                        **extra)
             return
