@@ -560,6 +560,36 @@ def mapped_attention_mma(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.
              _stream()), "mapped_attention_mma")
 
 
+def mapped_attention_sm100_takes(dim: int, vdim: int, n_maps: int, page_size: int, dtype) -> bool:
+    """Whether the tcgen05 kernel takes these sizes (keys of 64, values of 64 or 128, pages of 8 to 64 tokens)."""
+    return MAPPED_BACKEND == "mma" and dtype == torch.bfloat16 and dim == 64 and vdim in (64, 128) and n_maps in (1, 2) \
+        and page_size in (8, 16, 32, 64)
+
+
+def mapped_attention_sm100(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, table: torch.Tensor,
+                           cu_q: torch.Tensor, ctx_before: torch.Tensor, out: torch.Tensor, n_entries: int, max_q: int,
+                           n_heads: int, n_maps: int, window: Optional[int], keep_first: int, scale: float, softcap: float,
+                           lam: float, head_norm: bool, post_scale: float, eps: float, status: torch.Tensor,
+                           out_scale: float = 1.0) -> None:
+    """``mapped_attention_mma`` by the tcgen05 kernel (``mapped_attention_sm100_takes``): no score bias per head, sinks, gates
+    or chunks.  ``status``: a wait that runs out is reported there."""
+    n = q.shape[0]
+    num_pages, n_k, page_size, dim = k_pages.shape
+    n_g, vdim = v_pages.shape[1], v_pages.shape[3]
+    if n_k != n_g * n_maps or q.shape != (n, n_heads * n_maps * dim) or out.shape != (n, n_heads * vdim) \
+            or q.dtype != torch.bfloat16 or k_pages.dtype != torch.bfloat16 or v_pages.dtype != torch.bfloat16 \
+            or out.dtype != torch.bfloat16 or v_pages.shape[0] != num_pages or v_pages.shape[2] != page_size:
+        raise KernelError("mapped_attention_sm100: shapes or dtypes do not fit")
+    _i32(table, "table"), _i32(cu_q, "cu_q"), _i32(ctx_before, "ctx_before"), _i32(status, "status")
+    f = _fn("mapped_attention_sm100", "ng_mapped_attention_sm100", [_c_void_p] * 4 + [_c_int] + [_c_void_p] * 3 + [_c_int] * 13
+            + [_c_float] * 5 + [_c_int, _c_void_p, _c_void_p])
+    _check(f(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(table), table.shape[1], _ptr(cu_q), _ptr(ctx_before),
+             out.data_ptr(), _column_block(out, "attention out"), n, n_entries, max_q, n_heads, n_g, n_maps, dim, vdim,
+             page_size, num_pages, int(window or 0), int(keep_first), float(scale), float(softcap or 0.0), float(lam),
+             _post(head_norm, post_scale, out_scale), float(eps), int(bool(head_norm)), _ptr(status), _stream()),
+           "mapped_attention_sm100")
+
+
 def mapped_attention_group_takes(dim: int, vdim: int, n_heads: int, n_kv_heads: int, dtype) -> bool:
     """Whether single-token entries can run with the heads of a KV group as the rows of a tensor-core tile."""
     return mapped_attention_mma_takes(dim, vdim, dtype) and n_heads // n_kv_heads <= 16

@@ -36,6 +36,7 @@ class MappedAttention:
     graph_safe = True      # launches depend on device data and on launch-time constants only
     GROUP_MAX_ROWS = 256   # decode-only steps of up to this many rows run the heads of a KV group as a tensor-core tile
     GROUP_MAX_RUNS = 8     # ... a row's keys in up to this many runs (the blocks of a cluster)
+    TILE_MIN_ROWS = 64     # steps with a portion of at least this many rows (half a tile of the tcgen05 kernel) run on it
     SPLIT_MAX_ROWS = 32    # steps of up to this many rows may cut each row's keys into runs
     SPLIT_MIN_KEYS = 128   # ... of at least this many keys (one tile of the kernel)
     MAX_SPLITS = 16
@@ -132,7 +133,14 @@ class MappedAttention:
         jobs = [("gemm_sm100" if self.dtype == torch.bfloat16 else "gemm_f32", None), ("mapped_attention", None)]
         if ops.mapped_attention_mma_takes(s.key_dim, s.value_dim, self.dtype):
             jobs.append(("mapped_attention_mma", ops.mapped_attention_mma_defines(s.key_dim, s.value_dim, self.sigmoid)))
+        if self._plain_scores() and ops.mapped_attention_sm100_takes(s.key_dim, s.value_dim, s.n_maps, 16, self.dtype):
+            jobs.append(("mapped_attention_sm100", None))
         return jobs
+
+    def _plain_scores(self):
+        """Softmax over scores without a bias per head, sinks, chunks or a gate per head: what the tcgen05 kernel forms."""
+        s = self.spec
+        return not self.sigmoid and not getattr(s, "sinks", False) and not getattr(s, "chunk", None) and not getattr(s, "head_gate", False)
 
     def scratch_bytes_per_row(self):
         s = self.spec
@@ -225,6 +233,14 @@ class MappedAttention:
                                        out, None, ctx.n_entries, s.n_heads, s.n_maps, s.window, s.keep_first,
                                        s.softmax_scale, s.softcap or 0.0, self.lam, s.n_maps == 2, 1.0 - s.diff, s.eps, n_splits,
                                        **extra)
+            return
+        if ctx.max_q >= self.TILE_MIN_ROWS and self._plain_scores() and slopes is None and self.sinks is None and head_gate is None \
+                and ops.mapped_attention_sm100_takes(s.key_dim, s.value_dim, s.n_maps, cache.k_pages.shape[2], self.dtype) \
+                and out.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0:
+            ops.mapped_attention_sm100(q, cache.k_pages, cache.v_pages, cache.table, ctx.cu_q, ctx.ctx_before, out,
+                                       ctx.n_entries, ctx.max_q, s.n_heads, s.n_maps, s.window, s.keep_first,
+                                       s.softmax_scale, s.softcap or 0.0, self.lam, s.n_maps == 2, 1.0 - s.diff, s.eps,
+                                       ctx.status, out_scale=out_scale)
             return
         if n > self.SPLIT_MAX_ROWS and ops.mapped_attention_mma_takes(s.key_dim, s.value_dim, self.dtype):
             ops.mapped_attention_mma(q, cache.k_pages, cache.v_pages, cache.table, ctx.cu_q, ctx.ctx_before, out,

@@ -226,6 +226,43 @@ def test_attention_core_at_every_edge(dtype, M, H, G, dim, vdim, window, keep, s
             assert rel_err(got, whole) < 1.5e-2               # both round the output to bfloat16, nothing else differs
 
 
+@pytest.mark.parametrize("M,H,G,vdim,window,keep,softcap,ps", [
+    (1, 4, 2, 64, None, 0, None, 16), (1, 4, 1, 64, 200, 0, None, 8), (1, 2, 2, 128, 100, 4, 9.0, 32), (2, 2, 1, 128, 130, 4, 30.0, 16),
+    (2, 4, 2, 64, None, 0, None, 64), (2, 2, 2, 128, 20, 150, None, 16), (1, 2, 1, 64, 20, 70, 3.0, 8)])
+@pytest.mark.parametrize("lens,befores", [([256], [0]), ([129, 64], [300, 7]), ([1, 385, 40], [130, 0, 641])])
+def test_tcgen05_kernel_over_its_forms(M, H, G, vdim, window, keep, softcap, ps, lens, befores):
+    """One and two maps, values of 64 and 128, every page size, windows shorter than a tile and longer than a row tile, kept first
+    tokens that end inside and behind the first tiles, portions of one row, of a second stream's first row and across tiles,
+    a key without a page; against the row-by-row kernel (both round the output to bfloat16, nothing else differs)."""
+    dtype, o, d = torch.bfloat16, ops(), 64
+    total = [a + b for a, b in zip(lens, befores)]
+    n_pages = sum(-(-t // ps) for t in total)
+    g = torch.Generator().manual_seed(sum(total) + ps)
+    kp = torch.randn(n_pages, G * M, ps, d, generator=g).to(dtype).to(DEV)
+    vp = torch.randn(n_pages, G, ps, vdim, generator=g).to(dtype).to(DEV)
+    table = torch.full((len(lens), 96), -1, dtype=torch.int32)
+    perm = torch.randperm(n_pages, generator=g).to(torch.int32)
+    at = 0
+    for e, t in enumerate(total):
+        k = -(-t // ps)
+        table[e, :k] = perm[at:at + k]
+        at += k
+    n = sum(lens)
+    q = (2 * torch.randn(n, H * M * d, generator=g)).to(dtype).to(DEV)
+    ctx = make_ctx(lens, befores, list(range(len(lens))), dtype=dtype)
+    for holes in (False, True):
+        if holes:
+            table[0, 1] = -1
+        t = table.to(DEV)
+        a, b = torch.empty(n, H * vdim, dtype=dtype, device=DEV), torch.full((n + 1, H * vdim + 8), 7.0, dtype=dtype, device=DEV)
+        args = (window, keep, 0.2, softcap or 0.0, 0.4, M == 2, 0.6, 1e-5)
+        o.mapped_attention(q, kp, vp, t, ctx.positions, ctx.row_entry, a, H, M, *args)
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+        o.mapped_attention_sm100(q, kp, vp, t, ctx.cu_q, ctx.ctx_before, b[:n, :H * vdim], len(lens), max(lens), H, M, *args, status)
+        assert int(status) == 0 and bool((b[n] == 7).all()) and bool((b[:, H * vdim:] == 7).all())
+        assert rel_err(b[:n, :H * vdim], a) < 1.5e-2
+
+
 def test_tensor_core_kernel_with_several_entries_in_a_step():
     """Entries of unequal length (one of a single token, one shorter than a tile, one of several tiles), each after
     a context of its own, in one launch; each compared with the row-by-row kernel."""
