@@ -6,27 +6,36 @@
 // bfloat16 values the tensor cores add in float32.
 //
 // A block runs two streams of 128 query rows of one head: with one map two row tiles that share keys and values, with two maps
-// the two maps of one row tile (their own q and k, shared values), combined in the epilogue.  Ten warps:
-//   warps 0-3, 4-7  softmax of stream 0 and 1: thread r owns row r = TMEM lane r
-//   warp 8          producer: TMA loads of Q and of the tiles' keys and values, gathered page by page (a lane per page)
-//   warp 9          MMA issuer: S = Q K^T, O += P V (one elected lane), accumulators in TMEM
-// TMEM of a stream: 64 columns of S, which the hi and mid terms of P replace, 32 of the lo terms, the values' columns of O.  The tensor
-// pipe runs the MMAs in order: "S of tile j is there" says that P V of the tile before has read its P and that O holds it,
-// so S has one buffer a stream and the streams fill each other's waits (while one stream's scores are on their way the
-// other's softmax has the SM).  Every mbarrier wait is bounded; a waiter that gives up sets a status bit and the block runs to
-// its end (TMEM is always released).  2,048 tokens, window 1,024, inside a step: 32 heads of 64 with one map 103 us (217 us with
-// the mma.sync kernel), 16 heads with two maps and values of 128 120 us (406 us).
+// the two maps of one row tile (their own q and k, shared values), combined in the epilogue.  Warps:
+//   warps 0-7, 8-15 softmax of stream 0 and 1: two threads a row (TMEM lane), 32 of a tile's keys each
+//   warp 16         producer: TMA loads of Q and of the tiles' keys and values, gathered page by page (a lane per page)
+//   warp 17 (, 18)  MMA issuer: S = Q K^T, O += P V (one elected lane), accumulators in TMEM; one a stream where S has two
+//                   buffers (a stream does not wait behind the other's softmax), one for both otherwise (which keeps
+//                   them out of step: two issuers took 125 us where one takes 106)
+// TMEM of a stream: 64 columns of S, which the hi and mid terms of P replace, 32 of the lo terms, the values' columns of O.  The
+// kernel is bound by the chain S - softmax - P V of its few warps, so with values of 64 S and P have two buffers, which fill
+// the 512 columns, and the next tile's scores are there when a softmax warp comes for them.  Values of 128 leave room for one:
+// there "S of tile j is there" also says that P V of the tile before has read its P and that O holds it (the tensor pipe
+// runs the MMAs in order), and the streams fill each other's waits.  Every mbarrier wait is bounded; a waiter that gives up sets a status bit and the block runs to
+// its end (TMEM is always released).  2,048 tokens, window 1,024: 32 heads of 64 with one map 67 us (212 us with
+// the mma.sync kernel; 98 with one thread a row, one buffer and one issuer, 85 with two buffers, 77 with two threads a row), 16
+// heads with two maps and values of 128 106 us (398 us; 114 with one thread a row).
 #include "sm100_common.cuh"
 
 #define HD 64                  // key size
 #define BQ 128                 // query rows of a stream
 #define BK 64                  // keys per tile
 #define NG_STATUS_MAPPED_TIMEOUT 16
-#define THREADS 320
+#define HK (BK / 2)            // keys of a softmax thread
+#define PRODUCER 16            // the warps behind the sixteen of the softmax
+#define ISSUER 17
 static_assert(BQ == BLOCK_W, "a stream's query rows are the 128 rows of the MMA");
 
 template <int M, int DV>
 struct Cfg {
+    static constexpr int NB = DV == 64 ? 2 : 1;                      // buffers of S and P a stream
+    static constexpr int ISSUERS = NB;                               // warps that issue MMAs
+    static constexpr int THREADS = 32 * (17 + ISSUERS);
     static constexpr int STAGES = M == 2 && DV == 128 ? 4 : 5;
     static constexpr int STAGE_EL = M * BK * HD + BK * DV;           // keys of every map, then values in blocks of 64 columns
     static constexpr int TABLE_INTS = 1024;
@@ -46,6 +55,15 @@ struct Params {
     float scale, softcap, lambda, post_scale, eps;
 };
 
+// 32 consecutive float32 columns of this thread's TMEM lane, one load and one wait
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
+    uint32_t r[32];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr) : "memory");
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
 __device__ __forceinline__ void tmem_st16u(uint32_t taddr, const uint32_t (&v)[16]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
                  :: "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
@@ -61,7 +79,7 @@ __device__ __forceinline__ float lo_f(uint32_t w) { return __uint_as_float(w << 
 __device__ __forceinline__ float hi_f(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
 template <int M, int DV>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(Cfg<M, DV>::THREADS, 1)
 mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                               const __grid_constant__ CUtensorMap map_v, const Params p) {
     typedef Cfg<M, DV> C;
@@ -70,8 +88,9 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
     bf16* q_s = reinterpret_cast<bf16*>(base);                        // [2][BQ * HD], K-major swizzled
     bf16* kv_s = q_s + 2 * BQ * HD;                                   // [STAGES][STAGE_EL]
     int* pages = reinterpret_cast<int*>(kv_s + (size_t)C::STAGES * C::STAGE_EL);
-    __shared__ uint64_t q_full, kv_full[C::STAGES], kv_empty[C::STAGES], s_full[2], p_full[2], o_full;
+    __shared__ uint64_t q_full, kv_full[C::STAGES], kv_empty[C::STAGES], s_full[2][C::NB], p_full[2][C::NB], o_ready[2][2], o_full;
     __shared__ uint32_t tmem_base;
+    __shared__ float max_x[2][2][2][BQ], sum_x[2][2][BQ];             // what the two threads of a row tell each other
     __shared__ int hole;                                              // a key that rows of the block see has no page
     ng_pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -107,13 +126,16 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
 
     if (threadIdx.x == 0) {
         mbar_init(&q_full, 1);
-        for (int s = 0; s < C::STAGES; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&p_full[s], 4); }
-        mbar_init(&o_full, 1);
+        for (int s = 0; s < C::STAGES; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], C::ISSUERS == 2 ? streams : 1); }
+        for (int s = 0; s < 2; ++s) {
+            for (int b = 0; b < C::NB; ++b) { mbar_init(&s_full[s][b], 1); mbar_init(&p_full[s][b], 8); }
+            for (int b = 0; b < 2; ++b) mbar_init(&o_ready[s][b], 1);
+        }
+        mbar_init(&o_full, C::ISSUERS == 2 ? streams : 1);
         hole = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 9) {
+    if (warp == ISSUER) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(smem_u32(&tmem_base)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -125,23 +147,23 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
     const bool tab_smem = n_pages <= C::TABLE_INTS;
     auto no_page = [&](int page) { return page < 0 || page >= p.num_pages; };
     __syncthreads();                                                  // `hole` is set
-    for (int i = threadIdx.x; i < n_pages; i += THREADS) {
+    for (int i = threadIdx.x; i < n_pages; i += C::THREADS) {
         const int page = trow[first_page + i], begin = (first_page + i) << p.ps_log2;
         if (tab_smem) pages[i] = page;
         if (no_page(page) && (begin + (1 << p.ps_log2) > lo_key || begin < p.keep_first)) hole = 1;
     }
-    for (int i = threadIdx.x; (i << p.ps_log2) < min(p.keep_first, n_sink * BK); i += THREADS)
+    for (int i = threadIdx.x; (i << p.ps_log2) < min(p.keep_first, n_sink * BK); i += C::THREADS)
         if (no_page(trow[i])) hole = 1;
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem = tmem_base;
-    // columns: S and lo of both streams, then both O
-    auto tm_s = [&](int s) { return tmem + s * (BK + BK / 2); };
-    auto tm_o = [&](int s) { return tmem + 2 * (BK + BK / 2) + s * DV; };
+    // columns: S and lo of every buffer of both streams, then both O
+    auto tm_s = [&](int s, int b) { return tmem + (s * C::NB + b) * (BK + BK / 2); };
+    auto tm_o = [&](int s) { return tmem + 2 * C::NB * (BK + BK / 2) + s * DV; };
     bool ok = true;
 
-    if (warp == 8) {
+    if (warp == PRODUCER) {
         // ------------------------------------------------------------------ producer
         if (lane == 0) {
             mbar_expect_tx(&q_full, streams * BQ * HD * 2);
@@ -172,67 +194,76 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
             }
         }
         if (!ok && lane == 0) atomicOr(p.status, NG_STATUS_MAPPED_TIMEOUT);
-    } else if (warp == 9) {
+    } else if (warp >= ISSUER) {
         // ------------------------------------------------------------------ MMA issuer
         // All lanes run the loop and its waits, one elected lane issues (descriptors stay in uniform registers)
         constexpr uint32_t idesc_s = make_idesc(BK, 0), idesc_o = make_idesc(DV, 1);
         ok = __all_sync(0xffffffffu, mbar_wait(&q_full, 0));
-        int p_phase[2] = {0, 0};
-        bool begun[2] = {false, false};
-        for (int t = 0; t <= n_tiles && ok; ++t) {
+        const int s_lo = C::ISSUERS == 2 ? warp - ISSUER : 0, s_hi = C::ISSUERS == 2 ? s_lo : streams - 1;    // the warp's streams
+        int n_s[2] = {0, 0}, n_p[2] = {0, 0};                         // tiles whose S / whose P V has been issued
+        auto issue_s = [&](int s, int t) {                                   // S of tile t, over a P that an MMA issued before has read
+            if (!__all_sync(0xffffffffu, mbar_wait(&kv_full[t % C::STAGES], (t / C::STAGES) & 1))) { ok = false; return; }
+            tcgen05_fence_after();
+            const uint64_t dq = make_desc_sw128(q_s + s * BQ * HD);
+            const uint64_t dk = make_desc_sw128(kv_s + (size_t)(t % C::STAGES) * C::STAGE_EL + (M == 2 ? s * BK * HD : 0));
+            const int b = n_s[s] % C::NB;
+            const uint32_t ts = tm_s(s, b);
+            if (leader) {
+#pragma unroll
+                for (int k = 0; k < HD / 16; ++k)
+                    tcgen05_mma_f16(ts, dq + (uint64_t)(2 * k), dk + (uint64_t)(2 * k), idesc_s, k > 0);
+                tcgen05_commit(&s_full[s][b]);
+            }
+            ++n_s[s];
+            __syncwarp();
+        };
+        auto issue_pv = [&](int s, int t) {                                  // O += P V of tile t
+            const int b = n_p[s] % C::NB;
+            if (!__all_sync(0xffffffffu, mbar_wait(&p_full[s][b], (n_p[s] / C::NB) & 1))) { ok = false; return; }
+            tcgen05_fence_after();
+            // MN-major values: 64-column blocks BK * 64 elements apart, groups of eight keys 1,024 bytes apart
+            const bf16* v = kv_s + (size_t)(t % C::STAGES) * C::STAGE_EL + M * BK * HD;
+            uint64_t dv = make_desc_sw128_mn(v);
+            dv = (dv & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(BK * 64 * 2 >> 4) << 16);
+            const uint32_t ts = tm_s(s, b), to = tm_o(s);
+            const bool fresh = n_p[s] == 0;
+            if (leader) {
+#pragma unroll
+                for (int term = 2; term >= 0; --term)                 // smallest terms first: lo (behind S), mid, hi
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k)                 // 16 keys per MMA: 8 columns of P, 2,048 bytes of V
+                        tcgen05_mma_f16_ts(to, ts + 32 * term + 8 * k, dv + (uint64_t)(128 * k), idesc_o,
+                                           !(fresh && term == 2 && k == 0));
+                if (C::NB == 2) tcgen05_commit(&o_ready[s][n_p[s] & 1]);
+            }
+            ++n_p[s];
+            __syncwarp();
+        };
+        for (int t = 0; t <= n_tiles && ok && s_hi < streams; ++t) {
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
-                if (s >= streams || !ok) break;
-                if (t > 0 && sees(s, t - 1)) {                        // O += P V of the tile before
-                    ok = __all_sync(0xffffffffu, mbar_wait(&p_full[s], p_phase[s]));
-                    if (!ok) break;
-                    p_phase[s] ^= 1;
-                    tcgen05_fence_after();
-                    // MN-major values: 64-column blocks BK * 64 elements apart, groups of eight keys 1,024 bytes apart
-                    const bf16* v = kv_s + (size_t)((t - 1) % C::STAGES) * C::STAGE_EL + M * BK * HD;
-                    uint64_t dv = make_desc_sw128_mn(v);
-                    dv = (dv & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(BK * 64 * 2 >> 4) << 16);
-                    const uint32_t ts = tm_s(s), to = tm_o(s);
-                    const bool fresh = !begun[s];
-                    if (leader) {
-#pragma unroll
-                        for (int term = 2; term >= 0; --term)             // smallest terms first: lo (behind S), mid, hi
-#pragma unroll
-                            for (int k = 0; k < BK / 16; ++k)             // 16 keys per MMA: 8 columns of P, 2,048 bytes of V
-                                tcgen05_mma_f16_ts(to, ts + 32 * term + 8 * k, dv + (uint64_t)(128 * k), idesc_o,
-                                                   !(fresh && term == 2 && k == 0));
-                    }
-                    begun[s] = true;
-                    __syncwarp();
-                }
-                if (t > 0 && s == streams - 1) {                      // the tile's keys and values may be overwritten
-                    if (leader) {
+                if (s < s_lo || s > s_hi || !ok) continue;
+                const bool pv = t > 0 && sees(s, t - 1), sk = t < n_tiles && sees(s, t);
+                if (C::NB == 2 && sk) issue_s(s, t);                  // into the buffer whose P V was issued a round ago
+                if (ok && pv) issue_pv(s, t - 1);
+                if (ok && t > 0 && s == s_hi) {                       // the warp is done with the tile's keys and values
+                    // (if it saw nothing of the tile: once the tile is there, so that its stage is not filled twice)
+                    if (!pv) ok = __all_sync(0xffffffffu, mbar_wait(&kv_full[(t - 1) % C::STAGES], ((t - 1) / C::STAGES) & 1));
+                    if (leader && ok) {
                         tcgen05_commit(&kv_empty[(t - 1) % C::STAGES]);
-                        if (t == n_tiles) tcgen05_commit(&o_full);    // O of both streams is complete
+                        if (t == n_tiles) tcgen05_commit(&o_full);    // the warp's part of O is complete
                     }
                     __syncwarp();
                 }
-                if (t < n_tiles && sees(s, t)) {                      // S of this tile, over the P that the MMAs above read
-                    ok = __all_sync(0xffffffffu, mbar_wait(&kv_full[t % C::STAGES], (t / C::STAGES) & 1));
-                    if (!ok) break;
-                    tcgen05_fence_after();
-                    const uint64_t dq = make_desc_sw128(q_s + s * BQ * HD);
-                    const uint64_t dk = make_desc_sw128(kv_s + (size_t)(t % C::STAGES) * C::STAGE_EL + (M == 2 ? s * BK * HD : 0));
-                    const uint32_t ts = tm_s(s);
-                    if (leader) {
-#pragma unroll
-                        for (int k = 0; k < HD / 16; ++k)
-                            tcgen05_mma_f16(ts, dq + (uint64_t)(2 * k), dk + (uint64_t)(2 * k), idesc_s, k > 0);
-                        tcgen05_commit(&s_full[s]);
-                    }
-                    __syncwarp();
-                }
+                if (ok && C::NB == 1 && sk) issue_s(s, t);
             }
         }
         if (!ok && leader) atomicOr(p.status, NG_STATUS_MAPPED_TIMEOUT);
     } else {
-        // ------------------------------------------------------------------ softmax: thread = query row of its stream
-        const int s = warp >> 2, r = (warp & 3) * 32 + lane;
+        // ------------------------------------------------------------------ softmax: two threads a query row of their stream
+        // A thread has 32 of a tile's keys and half of the values' columns of O.  A wait that runs out does not leave the
+        // loop: the two warps of a row meet at barriers, as often as the tiles say.
+        const int s = warp >> 3, half = (warp >> 2) & 1, r = (warp & 3) * 32 + lane;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         const int row = (M == 2 ? 0 : s * BQ) + r;                    // within the block
         const bool warp_live = (M == 2 ? 0 : s * BQ) + (warp & 3) * 32 < rows_here;
@@ -241,48 +272,54 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
         const int w_last = min(pos_last, w_first + 31);
         const float scale2 = p.scale * 1.4426950408889634f, inv_cap = p.softcap > 0.f ? p.scale / p.softcap : 0.f;
         const float cap2 = p.softcap * 1.4426950408889634f;
-        const uint32_t ts = tm_s(s) + lane_base, to = tm_o(s) + lane_base;
-        // m is the reference point of the exponentials (base 2).  It follows the running maximum lazily: only when a
-        // tile's maximum exceeds it by more than 2^8 is O rescaled; otherwise weights simply reach 256.
+        const uint32_t to = tm_o(s) + lane_base + half * (DV / 2);
+        auto pair_meets = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + s * 4 + (warp & 3)) : "memory"); };
+        // m is the reference point of the exponentials (base 2), the same in both threads of a row.  It follows the running
+        // maximum lazily: only when a tile's maximum exceeds it by more than 2^8 is O rescaled; otherwise weights simply
+        // reach 256.
         float m = -INFINITY, l = 0.f;
-        int phase = 0;
-        bool begun = false;
+        int n = 0;                                                    // tiles seen so far
         for (int t = 0; t < n_tiles && s < streams; ++t) {
             if (!sees(s, t)) continue;
-            ok = __all_sync(0xffffffffu, mbar_wait(&s_full[s], phase));
-            if (!ok) break;
-            phase ^= 1;
+            const int b = n % C::NB;
+            const uint32_t ts = tm_s(s, b) + lane_base;
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&s_full[s][b], (n / C::NB) & 1));
             tcgen05_fence_after();
             if (warp_live) {
-                const int key0 = tile_of(t) * BK;
-                float sc[BK];
-                tmem_ld64(ts, sc);
+                const int key0 = tile_of(t) * BK, my0 = key0 + half * HK;
+                float sc[HK];
+                tmem_ld32(ts + half * HK, sc);
                 if (p.softcap > 0.f) {
 #pragma unroll
-                    for (int i = 0; i < BK; ++i) sc[i] = cap2 * tanh_ex2(sc[i] * inv_cap);
+                    for (int i = 0; i < HK; ++i) sc[i] = cap2 * tanh_ex2(sc[i] * inv_cap);
                 } else {
 #pragma unroll
-                    for (int i = 0; i < BK; ++i) sc[i] *= scale2;
+                    for (int i = 0; i < HK; ++i) sc[i] *= scale2;
                 }
                 // only tiles that cross a row's diagonal or the window's edge need the mask
                 const bool whole = key0 + BK - 1 <= w_first && (p.window <= 0 || key0 > w_last - p.window || key0 + BK <= p.keep_first);
                 if (!whole || hole) {                                         // (a key without a page is not seen)
 #pragma unroll
-                    for (int i = 0; i < BK; ++i) {
-                        const int key = key0 + i;
+                    for (int i = 0; i < HK; ++i) {
+                        const int key = my0 + i;
                         const bool vis = key <= pos && (p.window <= 0 || key > pos - p.window || key < p.keep_first);
                         sc[i] = vis && !(hole && no_page(trow[key >> p.ps_log2])) ? sc[i] : -INFINITY;
                     }
                 }
                 float m0 = sc[0], m1 = sc[1], m2 = sc[2], m3 = sc[3];
 #pragma unroll
-                for (int i = 4; i < BK; i += 4) {
+                for (int i = 4; i < HK; i += 4) {
                     m0 = fmaxf(m0, sc[i]);
                     m1 = fmaxf(m1, sc[i + 1]);
                     m2 = fmaxf(m2, sc[i + 2]);
                     m3 = fmaxf(m3, sc[i + 3]);
                 }
-                const float mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+                float mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+                max_x[n & 1][s][half][r] = mx;
+                tcgen05_fence_before();
+                pair_meets();                                                 // the row's maximum; and both threads have read its S
+                tcgen05_fence_after();
+                mx = fmaxf(mx, max_x[n & 1][s][half ^ 1][r]);
                 float corr = 1.f;
                 if (mx > m + 8.f || (m == -INFINITY && mx > -INFINITY)) {     // move the reference point
                     corr = ex2(m - mx);                                       // 0 the first time
@@ -290,28 +327,28 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
                 }
                 const float ref = m == -INFINITY ? 0.f : m;
                 float l0 = 0.f, l1 = 0.f;
+                uint32_t hi[HK / 2], mid[HK / 2], lo[HK / 2];
 #pragma unroll
-                for (int h = 0; h < BK; h += 32) {                            // 32 keys at a time: 16 words of each term
-                    uint32_t hi[16], mid[16], lo[16];
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const float a = ex2(sc[h + 2 * i] - ref), b = ex2(sc[h + 2 * i + 1] - ref);
-                        l0 += a;
-                        l1 += b;
-                        hi[i] = pack_bf16(a, b);
-                        const float ar = a - lo_f(hi[i]), br = b - hi_f(hi[i]);
-                        mid[i] = pack_bf16(ar, br);
-                        lo[i] = pack_bf16(ar - lo_f(mid[i]), br - hi_f(mid[i]));
-                    }
-                    // over this row's S (all of it has been read)
-                    tmem_st16u(ts + h / 2, hi);
-                    tmem_st16u(ts + 32 + h / 2, mid);
-                    tmem_st16u(ts + 64 + h / 2, lo);
+                for (int i = 0; i < HK / 2; ++i) {
+                    const float a = ex2(sc[2 * i] - ref), c = ex2(sc[2 * i + 1] - ref);
+                    l0 += a;
+                    l1 += c;
+                    hi[i] = pack_bf16(a, c);
+                    const float ar = a - lo_f(hi[i]), cr = c - hi_f(hi[i]);
+                    mid[i] = pack_bf16(ar, cr);
+                    lo[i] = pack_bf16(ar - lo_f(mid[i]), cr - hi_f(mid[i]));
                 }
+                tmem_st16u(ts + half * (HK / 2), hi);                         // over the row's S
+                tmem_st16u(ts + 32 + half * (HK / 2), mid);
+                tmem_st16u(ts + 64 + half * (HK / 2), lo);
                 l = l * corr + (l0 + l1);
-                if (begun && __any_sync(0xffffffffu, corr != 1.f)) {          // O holds the tiles before (S of this one is behind them)
+                if (n > 0 && __any_sync(0xffffffffu, corr != 1.f)) {          // O has to hold the tiles before
+                    if (C::NB == 2) {
+                        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&o_ready[s][(n - 1) & 1], ((n - 1) >> 1) & 1));
+                        tcgen05_fence_after();
+                    }
 #pragma unroll
-                    for (int c = 0; c < DV; c += 16) {
+                    for (int c = 0; c < DV / 2; c += 16) {
                         float v[16];
                         tmem_ld16(to + c, v);
 #pragma unroll
@@ -319,24 +356,28 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
                         tmem_st16(to + c, v);
                     }
                 }
-                begun = true;
                 tmem_st_wait();
             }
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&p_full[s]);
+            if (lane == 0) mbar_arrive(&p_full[s][b]);
+            ++n;
         }
         // ---- epilogue: O / l, the maps combined, the head's norm
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&o_full, 0));
         if (!ok && lane == 0) atomicOr(p.status, NG_STATUS_MAPPED_TIMEOUT);
         tcgen05_fence_after();
+        sum_x[s][half][r] = l;
+        pair_meets();
+        l += sum_x[s][half ^ 1][r];
         const float inv = l > 0.f ? 1.f / l : 0.f;
-        float* second = reinterpret_cast<float*>(kv_s) + (size_t)r * C::PITCH;       // M == 2: the second map's rows, over the tiles
+        const bool mine = ok && warp_live && s < streams;
+        float* second = reinterpret_cast<float*>(kv_s) + (size_t)r * C::PITCH + half * (DV / 2);   // M == 2: the second map's rows, over the tiles
         if (M == 2) {
-            if (s == 1 && warp_live && ok) {
+            if (s == 1 && mine) {
                 const float f = -p.lambda * inv;
 #pragma unroll
-                for (int c = 0; c < DV; c += 16) {
+                for (int c = 0; c < DV / 2; c += 16) {
                     float v[16];
                     tmem_ld16(to + c, v);
 #pragma unroll
@@ -344,32 +385,36 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
                         *reinterpret_cast<float4*>(second + c + i) = make_float4(v[i] * f, v[i + 1] * f, v[i + 2] * f, v[i + 3] * f);
                 }
             }
-            asm volatile("bar.sync 1, 256;" ::: "memory");            // the eight softmax warps
+            asm volatile("bar.sync 9, 512;" ::: "memory");            // the sixteen softmax warps
         }
-        if (ok && warp_live && (M == 1 || s == 0) && s < streams) {
-            float ss = 0.f;
-            if (M == 2 || p.head_norm) {
+        const bool writes = mine && (M == 1 || s == 0);
+        float ss = 0.f;
+        if (writes && (M == 2 || p.head_norm)) {
 #pragma unroll
-                for (int c = 0; c < DV; c += 16) {
-                    float v[16];
-                    tmem_ld16(to + c, v);
+            for (int c = 0; c < DV / 2; c += 16) {
+                float v[16];
+                tmem_ld16(to + c, v);
 #pragma unroll
-                    for (int i = 0; i < 16; i += 4) {
-                        float4 a = make_float4(v[i] * inv, v[i + 1] * inv, v[i + 2] * inv, v[i + 3] * inv);
-                        if (M == 2) {
-                            const float4 b = *reinterpret_cast<const float4*>(second + c + i);
-                            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-                            *reinterpret_cast<float4*>(second + c + i) = a;
-                        }
-                        ss += (a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w);
+                for (int i = 0; i < 16; i += 4) {
+                    float4 a = make_float4(v[i] * inv, v[i + 1] * inv, v[i + 2] * inv, v[i + 3] * inv);
+                    if (M == 2) {
+                        const float4 d = *reinterpret_cast<const float4*>(second + c + i);
+                        a.x += d.x; a.y += d.y; a.z += d.z; a.w += d.w;
+                        *reinterpret_cast<float4*>(second + c + i) = a;
                     }
+                    ss += (a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w);
                 }
             }
+        }
+        max_x[0][s][half][r] = ss;
+        pair_meets();
+        ss = max_x[0][s][0][r] + max_x[0][s][1][r];
+        if (writes) {
             float f = p.post_scale;
             if (p.head_norm) f *= rsqrtf(ss / (float)DV + p.eps);
-            bf16* orow = p.out + (size_t)(q0 + r0 + row) * p.out_ld + (size_t)head * DV;
+            bf16* orow = p.out + (size_t)(q0 + r0 + row) * p.out_ld + (size_t)head * DV + half * (DV / 2);
 #pragma unroll
-            for (int c = 0; c < DV; c += 16) {
+            for (int c = 0; c < DV / 2; c += 16) {
                 float v[16];
                 if (M == 2) {
 #pragma unroll
@@ -394,7 +439,7 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
     }
     tcgen05_fence_before();
     __syncthreads();
-    if (warp == 9)
+    if (warp == ISSUER)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" :: "r"(tmem) : "memory");
 }
 
@@ -412,7 +457,8 @@ static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
     const dim3 grid(p.nH, (max_q + ROWS - 1) / ROWS, n_entries);
     if (grid.y > 65535 || grid.z > 65535) return NG_BAD_SIZE;
     const size_t smem = Cfg<M, DV>::smem();
-    NG_LAUNCH((mapped_attention_sm100_kernel<M, DV>), grid, THREADS, smem, stream, mq, mk, mv, p);
+    const int threads = Cfg<M, DV>::THREADS;
+    NG_LAUNCH((mapped_attention_sm100_kernel<M, DV>), grid, threads, smem, stream, mq, mk, mv, p);
     return ng_launch_status();
 }
 
