@@ -419,6 +419,23 @@ def test_attn_decode_bf16(nH, nKV, hd, ps, window, n_splits):
     close(got[keep], want[keep], torch.bfloat16)
 
 
+@pytest.mark.parametrize("hd,nH,nKV", [(64, 32, 8), (16, 3, 1), (48, 16, 1), (128, 8, 2)])
+@pytest.mark.parametrize("n_splits", [2, 7, 8, 9, 33])
+def test_attn_decode_merges_its_splits(hd, nH, nKV, n_splits):
+    """Fewer splits than groups of the merging kernel, and more than its threads walk at once: contexts that leave most splits
+    empty, one key, and one that fills them; a window; the bound is the rounding of weights and output to bfloat16."""
+    q_lens, ctx = [1, 1, 1, 1], [0, 63, 2111, 700]
+    k, v, table, pos, re = _paged_setup(torch.bfloat16, nKV, hd, 16, q_lens, ctx, num_pages=240, seed=9)
+    cu, cb = _cu(q_lens, ctx)
+    q = rnd(4, nH * hd, dtype=torch.bfloat16, seed=15)
+    for window in (None, 600):
+        want, got = torch.empty_like(q), torch.full_like(q, 7.0)
+        ref.attention_generic(q, k, v, table, pos, re, want, nH, window, 1 / math.sqrt(hd))
+        scratch = torch.full((ops().attn_decode_scratch_floats(4, nH, hd, n_splits),), float("nan"), device=DEV)
+        ops().attn_decode_bf16(q, k, v, table, cu, cb, got, scratch, 4, nH, window, 1 / math.sqrt(hd), n_splits, 2112)
+        close(got, want, torch.bfloat16)
+
+
 def test_attn_bf16_finds_a_far_key_and_respects_the_window_edge():
     nH, nKV, hd, ps = 8, 2, 64, 16
     ctx_len, far = 1500, 333
