@@ -1303,8 +1303,12 @@ _GEMM_ARGS = [_c_void_p] * 4 + [_c_int] * 9 + [_c_float, _c_float, _c_void_p, _c
 # Steps of at most FUSE_MAX_ROWS rows (bfloat16, tcgen05 backend) add the products that end a
 # mixer or a feed-forward straight into the float32 residual stream (red.global.add in the
 # epilogue): the norm kernel that follows has no partial sums to read.  Measured on the decode
-# graph of the 1.2B shape: batch 8 0.887 -> 0.852 ms, batch 64 1.329 -> 1.233 ms.
-FUSE_MAX_ROWS = int(os.environ.get("NEUROGRID_B200_FUSE_ROWS", "64"))
+# graph of the 1.2B shape: batch 8 0.887 -> 0.852 ms, batch 64 1.329 -> 1.233 ms.  From 65 to 128 rows, two token tiles of 64
+# and K cut so that the blocks fill the GPU beat the library's product of a feed-forward's second matrix (128 rows; hidden
+# 1,024 / 1,536 / 2,048: 5.2 / 7.8 / 10.6 us against 8.0 / 11.2 / 13.2) and of a mixer's output (3.3 / 4.1 / 5.4 against
+# 3.9 / 4.9 / 6.1), whose result the norm kernel would also have to read; at 256 rows they no longer do (6.3 / 7.6 / 9.8 us
+# against 4.0 / 5.3 / 6.4 for the output).
+FUSE_MAX_ROWS = min(128, int(os.environ.get("NEUROGRID_B200_FUSE_ROWS", "128")))
 FUSE_RED = os.environ.get("NEUROGRID_B200_FUSE_RED", "1") == "1"
 GEMM_BACKEND = os.environ.get("NEUROGRID_B200_GEMM", "sm100")     # "sm100": tcgen05 kernel; "cublas": vendor library
 # Rows up to which the tcgen05 kernel is used.  It streams weights at memory speed, which is the
@@ -1418,14 +1422,15 @@ def linear_to_residual(x: torch.Tensor, weight: torch.Tensor, bias: Optional[tor
     do that, and None is returned: nothing is left for the caller to add."""
     M, K = x.shape
     N = weight.shape[0]
-    if bias is None and M <= 64 and gemm_sm100_ok(x, weight):
-        tiles = -(-N // 128)
+    adds = bias is None and residual is not None and residual_add_fusable(x, weight)
+    if adds or (bias is None and M <= 64 and gemm_sm100_ok(x, weight)):
+        tiles = -(-N // 128) * -(-M // 64)
         want = min(MAX_RESIDUAL_SPLITS, max(1, sm_count(weight.device) // tiles), max(1, -(-K // 64) // 4))
         s = gemm_splits(K, want)
-        if FUSE_RED and residual is not None and M <= FUSE_MAX_ROWS:
+        if adds:
             _f32(residual, "residual")
             f = _fn("gemm_sm100", "ng_gemm_sm100", _GEMM_ARGS)
-            _check(f(_ptr(x), _ptr(weight), None, _ptr(residual), M, N, K, N, N, 3, s, 0, 0, 0.0, 0.0,
+            _check(f(_ptr(x), _ptr(weight), None, _ptr(residual), M, N, K, N, N, 3, s, 0, 64 if M > 64 else 0, 0.0, 0.0,
                      _ptr(_gemm_status(weight.device)), _stream()), "gemm_sm100 (residual add)")
             return None
         if s > 1:
@@ -1460,7 +1465,9 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, ws, name: str):
 
 def residual_add_fusable(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether ``linear_to_residual(x, weight, None, ..., residual=h)`` adds the product into ``h`` itself."""
-    return FUSE_RED and x.shape[0] <= min(64, FUSE_MAX_ROWS) and gemm_sm100_ok(x, weight)
+    M = x.shape[0]
+    return FUSE_RED and M <= FUSE_MAX_ROWS and (gemm_sm100_ok(x, weight) if M <= 64 else
+                                                GEMM_BACKEND == "sm100" and gemm_sm100_takes(x, weight))
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> None:

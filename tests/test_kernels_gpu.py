@@ -691,6 +691,19 @@ def test_tensor_core_kernels_repeat_bit_for_bit():
     assert ops().gemm_status(DEV) == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(64, 1024, 1024), (65, 1024, 4608), (100, 200, 136), (127, 1536, 1536), (128, 2048, 8192), (129, 256, 256)])
+def test_products_into_the_residual(M, N, K):
+    """Steps of up to 64 rows, of two token tiles (65 to 128 rows) and one row more, which the caller adds itself: the sums
+    are float32, in an order that is not fixed (the bound: as many roundings as there are splits and blocks of K)."""
+    x, w, h = rnd(M, K, dtype=torch.bfloat16, seed=1), rnd(N, K, dtype=torch.bfloat16, std=K ** -0.5, seed=2), rnd(M, N, seed=3)
+    want = h.double() + x.double() @ w.double().T
+    taken = ops().residual_add_fusable(x, w)
+    assert taken == (M <= 128)
+    if taken:
+        assert ops().linear_to_residual(x, w, None, None, "out", residual=h) is None
+        assert float((h.double() - want).abs().max()) < 1e-5 * float(want.abs().max())
+
+
 def test_residual_add_epilogue_spread_is_bounded():
     """The epilogue that adds a split-K product into the float32 stream (red.global.add) fixes no
     order for its additions, so runs may differ in the last bits, and by no more: thirty runs from
