@@ -232,11 +232,17 @@ mapped_attention_mma_kernel(const MmaParams p) {
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     lookup(t_begin, 0);
+    if (GROUP) lookup(t_begin + KT, 1);
     __syncthreads();
-    // the first tile, if all its keys are older than the step (an earlier step wrote them), before the wait
-    const int t_old = min(n_keys, t_begin + KT) - 1;
-    const bool old_tile = t_old < t_begin || (t_old < n_sink ? t_old : lo + (t_old - n_sink)) < before;
+    // the first tile, if all its keys are older than the step (an earlier step wrote them), before the wait; of a single
+    // token's run the second one too
+    auto is_old = [&](int t0) {
+        const int t_last = min(n_keys, t0 + KT) - 1;
+        return t_last < t0 || (t_last < n_sink ? t_last : lo + (t_last - n_sink)) < before;
+    };
+    const bool old_tile = is_old(t_begin), old_second = GROUP && old_tile && t_begin + KT < n_keys && is_old(t_begin + KT);
     if (old_tile) copy_tile(0, 0);
+    if (old_second) copy_tile(1, 1);
     ng_pdl_wait();
     const bf16* qg = ng_after_wait(p.q);
     // ---- Q: rows r0.., both maps, into shared memory (rows beyond the entry: zeros)
@@ -260,10 +266,12 @@ mapped_attention_mma_kernel(const MmaParams p) {
         // the lookup of tile it+1 goes to slot (it+1) % 3: slower warps may still read tile it-1's positions (slot
         // (it-1) % 3) and tile it's copies were made from slot it % 3; the slot's last readers (tile it-2) passed the
         // barrier of the iteration before
-        if (more) lookup(t0 + KT, (it + 1) % 3);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        const bool asked = GROUP && it == 0;             // (looked up, and copied if old, in front of the loop)
+        if (more && !asked) lookup(t0 + KT, (it + 1) % 3);
+        if (asked && old_second) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                                 // this tile has landed; the other data buffer is free
-        if (more) copy_tile(buf ^ 1, (it + 1) % 3);
+        if (more && !(asked && old_second)) copy_tile(buf ^ 1, (it + 1) % 3);
         const int* kpos_t = kpos_s[it % 3];
         // does any row of the warp see any key of the tile?  (positions ascend within both parts of the list)
         bool any = warp_live;
@@ -435,40 +443,53 @@ mapped_attention_mma_kernel(const MmaParams p) {
         };
         const bf16* gate = ng_after_wait(p.gate);
         for (int r = blockIdx.x * WARPS + warp; r < n_rows; r += p.n_splits * WARPS) {
-            float v[DV / 32 + 1], ss = 0.f;
-#pragma unroll
-            for (int u = 0; u < DV / 32 + 1; ++u) v[u] = 0.f;
+            constexpr int NU = (DV + 31) / 32;
+            float v[NU], ss = 0.f, f[M], scale[M], acc[M][NU];
+            const int at = r * M * (DV + 2);
+            // a lane per run for the maxima, the factors and the sums; the maps side by side
+            float mr[M], lr[M];
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                const int at = (r * M + m) * (DV + 2);
-                // a lane per run for the maximum, the factors and the sum
-                const float mr = lane < p.n_splits ? state(lane, at) : -INFINITY, lr = lane < p.n_splits ? state(lane, at + 1) : 0.f;
-                const float mt = ng_warp_max(mr);
-                const float f = mr == -INFINITY ? 0.f : exp2f(mr - mt);
-                float l = ng_warp_sum(lr * f);
-                if (p.sinks) l += exp2f(p.sinks[head + r] * 1.4426950408889634f - mt);      // the term without key or value
-                const float scale = (SIGMOID ? 1.f : l > 0.f ? 1.f / l : 0.f) * (m == 1 ? -p.lambda : 1.f);
-                float acc[DV / 32 + 1];
-#pragma unroll
-                for (int u = 0; u < DV / 32 + 1; ++u) acc[u] = 0.f;
-#pragma unroll 4
-                for (int x = 0; x < p.n_splits; ++x) {
-                    const float fx = __shfl_sync(0xffffffffu, f, x);
-#pragma unroll
-                    for (int u = 0; u < DV / 32 + 1; ++u)
-                        if (lane + 32 * u < DV) acc[u] = fmaf(state(x, at + 2 + lane + 32 * u), fx, acc[u]);
-                }
-#pragma unroll
-                for (int u = 0; u < DV / 32 + 1; ++u) v[u] = fmaf(acc[u], scale, v[u]);
+                mr[m] = lane < p.n_splits ? state(lane, at + m * (DV + 2)) : -INFINITY;
+                lr[m] = lane < p.n_splits ? state(lane, at + m * (DV + 2) + 1) : 0.f;
             }
 #pragma unroll
-            for (int u = 0; u < DV / 32 + 1; ++u) ss += v[u] * v[u];
+            for (int m = 0; m < M; ++m) {
+                const float mt = ng_warp_max(mr[m]);
+                f[m] = mr[m] == -INFINITY ? 0.f : exp2f(mr[m] - mt);
+                float l = ng_warp_sum(lr[m] * f[m]);
+                if (p.sinks) l += exp2f(p.sinks[head + r] * 1.4426950408889634f - mt);      // the term without key or value
+                scale[m] = (SIGMOID ? 1.f : l > 0.f ? 1.f / l : 0.f) * (m == 1 ? -p.lambda : 1.f);
+#pragma unroll
+                for (int u = 0; u < NU; ++u) acc[m][u] = 0.f;
+            }
+#pragma unroll 4
+            for (int x = 0; x < p.n_splits; ++x) {
+                float part[M][NU];
+#pragma unroll
+                for (int m = 0; m < M; ++m)
+#pragma unroll
+                    for (int u = 0; u < NU; ++u)
+                        part[m][u] = lane + 32 * u < DV ? state(x, at + m * (DV + 2) + 2 + lane + 32 * u) : 0.f;
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const float fx = __shfl_sync(0xffffffffu, f[m], x);
+#pragma unroll
+                    for (int u = 0; u < NU; ++u) acc[m][u] = fmaf(part[m][u], fx, acc[m][u]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < NU; ++u) {
+                v[u] = acc[0][u] * scale[0];
+                if (M == 2) v[u] = fmaf(acc[M - 1][u], scale[M - 1], v[u]);
+                ss += v[u] * v[u];
+            }
             float k = p.post_scale;
             if (p.gate) k *= rcpf(1.f + ex2f(-1.4426950408889634f * __bfloat162float(gate[(size_t)q0 * p.gate_ld + head + r])));
             if (p.head_norm) k *= rsqrtf(ng_warp_sum(ss) / (float)DV + p.eps);
             bf16* dst = p.out + (size_t)q0 * p.out_ld + (size_t)(head + r) * DV;
 #pragma unroll
-            for (int u = 0; u < DV / 32 + 1; ++u)
+            for (int u = 0; u < NU; ++u)
                 if (lane + 32 * u < DV) dst[lane + 32 * u] = __float2bfloat16_rn(v[u] * k);
         }
         // a block's states stay until every block has read them
