@@ -407,8 +407,8 @@ mapped_attention_kernel(const MaParams p) {
         const int kpos = valid ? (t < n_sink ? t : lo + (t - n_sink)) : pos;
         const int page = trow[kpos / p.page_size];
         const bool ok = valid && page >= 0 && page < p.num_pages;
-        const size_t slot = kpos % p.page_size, pg = ok ? page : 0;
-        const size_t vbase = ((pg * p.nG + g) * p.page_size + slot) * dv;
+        const size_t slot = kpos % p.page_size, pg = ok ? page : 0, none = ~(size_t)0;
+        const size_t vbase = ok ? ((pg * p.nG + g) * p.page_size + slot) * dv : none;
         float pr[M];
 #pragma unroll
         for (int m = 0; m < M; ++m) {
@@ -431,8 +431,8 @@ mapped_attention_kernel(const MaParams p) {
 #pragma unroll
             for (int u = 0; u < DVU; ++u) { acc[m][u][0] *= corr; acc[m][u][1] *= corr; }
         }
-        // eight keys at a time, their values requested before the first is used; a lane beyond the run's end has the
-        // weight 0 and the address of a key that is there (the row's own), so nothing is skipped inside a group
+        // eight keys at a time, their values requested before the first is used; a lane beyond the run's end, or whose key has
+        // no page, has the weight 0 and values of 0 (0 times what some other slot holds may be NaN)
         const int cnt = min(32, t1 - tb);
         for (int j0 = 0; j0 < cnt; j0 += 8) {
             float2 vv[8][DVU];
@@ -445,7 +445,7 @@ mapped_attention_kernel(const MaParams p) {
 #pragma unroll
                 for (int u = 0; u < DVU; ++u) {
                     const int c = 2 * lane + 64 * u;
-                    vv[jj][u] = c < dv ? ma_ld_pair(vp + vb, c, dv, vvec) : make_float2(0.f, 0.f);
+                    vv[jj][u] = vb != none && c < dv ? ma_ld_pair(vp + vb, c, dv, vvec) : make_float2(0.f, 0.f);
                 }
             }
 #pragma unroll

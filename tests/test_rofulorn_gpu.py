@@ -263,6 +263,65 @@ def test_tcgen05_kernel_over_its_forms(M, H, G, vdim, window, keep, softcap, ps,
         assert rel_err(b[:n, :H * vdim], a) < 1.5e-2
 
 
+def _poison(kp, vp, table, lens, befores, window, keep):
+    """NaN and infinities into every slot that no row of any entry sees: behind an entry's last token, between the kept first
+    tokens and its first row's window, and in pages of no entry (host tensors)."""
+    ps, seen = kp.shape[2], torch.zeros(kp.shape[0], kp.shape[2], dtype=torch.bool)
+    for e, (n, b) in enumerate(zip(lens, befores)):
+        for j in range(n + b):
+            if int(table[e, j // ps]) >= 0 and (not window or j > b - window or j < keep):
+                seen[int(table[e, j // ps]), j % ps] = True
+    kp.permute(0, 2, 1, 3)[~seen] = float("nan")
+    vp.permute(0, 2, 1, 3)[~seen] = float("inf")
+    vp[:, :, ::2].permute(0, 2, 1, 3)[~seen[:, ::2]] = float("nan")
+
+
+def _paged_entries(lens, befores, G, M, d, vdim, ps, spare=2):
+    """Random pages (some of no entry, page 0 among them), the table and a step's batch description."""
+    total = [a + b for a, b in zip(lens, befores)]
+    n_pages = spare + sum(-(-t // ps) for t in total)
+    g = torch.Generator().manual_seed(sum(total) + ps)
+    kp = torch.randn(n_pages, G * M, ps, d, generator=g).to(torch.bfloat16)
+    vp = torch.randn(n_pages, G, ps, vdim, generator=g).to(torch.bfloat16)
+    table = torch.full((len(lens), 2 + -(-max(total) // ps)), -1, dtype=torch.int32)
+    perm = (1 + torch.randperm(n_pages - 1, generator=g)).to(torch.int32)
+    at = 0
+    for e, t in enumerate(total):
+        k = -(-t // ps)
+        table[e, :k] = perm[at:at + k]
+        at += k
+    return kp, vp, table, make_ctx(lens, befores, list(range(len(lens))), dtype=torch.bfloat16), g
+
+
+UNSEEN = [(1, 4, 2, 64, None, 0, None, 16), (1, 4, 1, 64, 200, 0, None, 8), (1, 2, 2, 128, 100, 4, 9.0, 32),
+          (2, 2, 1, 128, 130, 4, 30.0, 16), (2, 4, 2, 64, None, 0, None, 64), (2, 2, 2, 128, 20, 150, None, 16),
+          (1, 2, 1, 64, 20, 70, 3.0, 8)]
+UNSEEN_STEPS = [([256], [0]), ([129, 64], [300, 7]), ([1, 385, 40], [130, 0, 641]), ([65], [1023])]
+
+
+@pytest.mark.parametrize("M,H,G,vdim,window,keep,softcap,ps", UNSEEN)
+@pytest.mark.parametrize("lens,befores", UNSEEN_STEPS)
+@pytest.mark.parametrize("kernel", ["rows", "tiles"])
+def test_what_no_row_sees_stays_out(kernel, M, H, G, vdim, window, keep, softcap, ps, lens, befores):
+    """Slots that no row sees hold infinities and NaN, as a request whose values overflowed leaves them in a page that another
+    request is given: the same outputs as with ordinary numbers there, bit for bit."""
+    o = ops()
+    kp, vp, table, ctx, g = _paged_entries(lens, befores, G, M, 64, vdim, ps)
+    n = sum(lens)
+    q = (2 * torch.randn(n, H * M * 64, generator=g)).to(torch.bfloat16).to(DEV)
+    args = (H, M, window, keep, 0.2, softcap or 0.0, 0.4, M == 2, 0.6, 1e-5)
+    got = []
+    for _ in range(2):
+        out, pages = torch.full((n, H * vdim), 7.0, dtype=torch.bfloat16, device=DEV), (q, kp.to(DEV), vp.to(DEV), table.to(DEV))
+        if kernel == "rows":
+            o.mapped_attention(*pages, ctx.positions, ctx.row_entry, out, *args)
+        else:
+            o.mapped_attention_mma(*pages, ctx.cu_q, ctx.ctx_before, out, len(lens), max(lens), *args)
+        got.append(out)
+        _poison(kp, vp, table, lens, befores, window, keep)
+    assert bool(torch.isfinite(got[0].float()).all()) and torch.equal(got[0], got[1])
+
+
 def test_tensor_core_kernel_with_several_entries_in_a_step():
     """Entries of unequal length (one of a single token, one shorter than a tile, one of several tiles), each after
     a context of its own, in one launch; each compared with the row-by-row kernel."""
