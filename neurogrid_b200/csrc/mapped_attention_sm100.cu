@@ -217,6 +217,23 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
             ++n_s[s];
             __syncwarp();
         };
+        // Values that no row of the block sees (behind its last key, in front of the window, between the two) become zeros before
+        // a product reads them: their weights are 0, and 0 times what another request left in a page may be NaN.  They lie in three
+        // tiles at most.  This warp does it while it would wait for the softmax (in the softmax warps the same stores cost 2 to
+        // 10 % of the kernel: registers).
+        const int edge_kept = p.keep_first % BK ? n_sink - 1 : -1, edge_lo = lo_key % BK ? n_sink : -1;
+        const int edge_last = pos_last % BK != BK - 1 ? n_tiles - 1 : -1;
+        auto clear_unseen = [&](int t) {
+            bf16* v = kv_s + (size_t)(t % C::STAGES) * C::STAGE_EL + M * BK * HD;
+            for (int i = lane; i < BK * 8; i += 32) {                 // 128-byte rows whole: the swizzle stays inside
+                const int k = i >> 3, key = tile_of(t) * BK + k;
+                if (key <= pos_last && (key >= lo_key || key < p.keep_first)) continue;
+#pragma unroll
+                for (int c = 0; c < DV / 64; ++c) *reinterpret_cast<uint4*>(v + (c * BK + k) * 64 + (i & 7) * 8) = make_uint4(0u, 0u, 0u, 0u);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+        };
         auto issue_pv = [&](int s, int t) {                                  // O += P V of tile t
             const int b = n_p[s] % C::NB;
             if (!__all_sync(0xffffffffu, mbar_wait(&p_full[s][b], (n_p[s] / C::NB) & 1))) { ok = false; return; }
@@ -240,6 +257,8 @@ mapped_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const _
             __syncwarp();
         };
         for (int t = 0; t <= n_tiles && ok && s_hi < streams; ++t) {
+            // the values of tile t - 1 are there if S of the tile, which has been issued, was one of this warp's
+            if ((t - 1 == edge_last || t - 1 == edge_lo || t - 1 == edge_kept) && t > 0 && (C::ISSUERS == 1 || sees(s_lo, t - 1))) clear_unseen(t - 1);
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
                 if (s < s_lo || s > s_hi || !ok) continue;

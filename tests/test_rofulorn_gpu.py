@@ -301,7 +301,7 @@ UNSEEN_STEPS = [([256], [0]), ([129, 64], [300, 7]), ([1, 385, 40], [130, 0, 641
 
 @pytest.mark.parametrize("M,H,G,vdim,window,keep,softcap,ps", UNSEEN)
 @pytest.mark.parametrize("lens,befores", UNSEEN_STEPS)
-@pytest.mark.parametrize("kernel", ["rows", "tiles"])
+@pytest.mark.parametrize("kernel", ["rows", "tiles", "tcgen05"])
 def test_what_no_row_sees_stays_out(kernel, M, H, G, vdim, window, keep, softcap, ps, lens, befores):
     """Slots that no row sees hold infinities and NaN, as a request whose values overflowed leaves them in a page that another
     request is given: the same outputs as with ordinary numbers there, bit for bit."""
@@ -315,11 +315,13 @@ def test_what_no_row_sees_stays_out(kernel, M, H, G, vdim, window, keep, softcap
         out, pages = torch.full((n, H * vdim), 7.0, dtype=torch.bfloat16, device=DEV), (q, kp.to(DEV), vp.to(DEV), table.to(DEV))
         if kernel == "rows":
             o.mapped_attention(*pages, ctx.positions, ctx.row_entry, out, *args)
-        else:
+        elif kernel == "tiles":
             o.mapped_attention_mma(*pages, ctx.cu_q, ctx.ctx_before, out, len(lens), max(lens), *args)
+        else:
+            o.mapped_attention_sm100(*pages, ctx.cu_q, ctx.ctx_before, out, len(lens), max(lens), *args, ctx.status)
         got.append(out)
         _poison(kp, vp, table, lens, befores, window, keep)
-    assert bool(torch.isfinite(got[0].float()).all()) and torch.equal(got[0], got[1])
+    assert int(ctx.status) == 0 and bool(torch.isfinite(got[0].float()).all()) and torch.equal(got[0], got[1])
 
 
 def test_tensor_core_kernel_with_several_entries_in_a_step():
