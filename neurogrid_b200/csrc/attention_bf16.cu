@@ -67,13 +67,14 @@ struct PrefillSmem {
     bf16 v[2][PF_KEYS][PF_LD];
 };
 
-// Gather one 64-key tile of K and V (keys key0..key0+63 of the entry) into stage s.
+// Gather one 64-key tile of K and V (keys key0..key0+63 of the entry; zeros for those outside [key_lo, kv_end), which no
+// row sees: a weight of 0 times what another request left in a page may be NaN) into stage s.
 // `ptab[(key >> ps_log2) - first_page]` is the page of a key: the block's slice of the table in
 // shared memory when it fits, else the entry's table row itself (first_page 0).
 __device__ __forceinline__ void pf_load_tile(PrefillSmem* sm, int s, const bf16* __restrict__ k_pages,
                                              const bf16* __restrict__ v_pages, const int* __restrict__ ptab,
-                                             int first_page, int key0, int kv_end, int kvh, int nKV, int ps_log2,
-                                             int num_pages) {
+                                             int first_page, int key0, int key_lo, int kv_end, int kvh, int nKV,
+                                             int ps_log2, int num_pages) {
     constexpr int CH = HD / 8;                          // 16-byte chunks per row
 #pragma unroll
     for (int c0 = 0; c0 < PF_KEYS * CH; c0 += PF_THREADS) {
@@ -81,7 +82,7 @@ __device__ __forceinline__ void pf_load_tile(PrefillSmem* sm, int s, const bf16*
         if (PF_KEYS * CH % PF_THREADS != 0 && c >= PF_KEYS * CH) break;
         const int r = c / CH, ch = c % CH;
         const int key = key0 + r;
-        bool ok = key < kv_end;
+        bool ok = key >= key_lo && key < kv_end;
         size_t off = 0;
         if (ok) {
             const int page = ptab[(key >> ps_log2) - first_page];
@@ -141,7 +142,8 @@ attn_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages
             __syncthreads();
         }
     }
-    pf_load_tile(sm, 0, k_pages, v_pages, ptab, first_page, tile0 * PF_KEYS, kv_end, kvh, nKV, ps_log2, num_pages);
+    pf_load_tile(sm, 0, k_pages, v_pages, ptab, first_page, tile0 * PF_KEYS, key_lo, kv_end, kvh, nKV, ps_log2,
+                 num_pages);
     cp_async_commit();
 
     float o[HD / 8][4];
@@ -155,8 +157,8 @@ attn_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages
     for (int tile = tile0; tile <= tile1; ++tile) {
         const int s = (tile - tile0) & 1;
         if (tile < tile1) {
-            pf_load_tile(sm, s ^ 1, k_pages, v_pages, ptab, first_page, (tile + 1) * PF_KEYS, kv_end, kvh, nKV, ps_log2,
-                         num_pages);
+            pf_load_tile(sm, s ^ 1, k_pages, v_pages, ptab, first_page, (tile + 1) * PF_KEYS, key_lo, kv_end, kvh, nKV,
+                         ps_log2, num_pages);
             cp_async_commit();
             cp_async_wait<1>();
         } else {

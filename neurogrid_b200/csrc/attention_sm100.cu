@@ -221,9 +221,23 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
                 }
                 __syncwarp();
             };
+            // Values that no row of the block sees (behind its last key, in front of the window; the last and the first tile may
+            // hold such) become zeros before P V reads them: their weights are 0, and 0 times what another request left in a page
+            // may be NaN.
+            const int edge_last = (tile0 + n_tiles) * BK > kv_end ? n_tiles - 1 : -1, edge_lo = tile0 * BK < key_lo ? 0 : -1;
+            auto clear_unseen = [&](int j) {
+                bf16* v = sm->v[j % KV_STAGES];
+                for (int i = lane; i < BK * HD / 8; i += 32) {      // 128-byte rows whole: the swizzle stays inside
+                    const int key = (tile0 + j) * BK + i / (HD / 8);
+                    if (key < key_lo || key >= kv_end) *reinterpret_cast<uint4*>(v + i * 8) = make_uint4(0u, 0u, 0u, 0u);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+            };
             if (ok) issue_s(0);
             if (ok && n_tiles > 1) issue_s(1);
             for (int j = 0; j < n_tiles && ok; ++j) {
+                if (j == edge_last || j == edge_lo) clear_unseen(j);            // (they are there: S_j has waited for them)
                 ok = __all_sync(0xffffffffu, mbar_wait(&sm->p_full[j & 1], (j >> 1) & 1));   // P_j in tensor memory, O rescaled
                 if (!ok) break;
                 tcgen05_fence_after();

@@ -578,6 +578,43 @@ def test_attn_prefill_sm100(nH, nKV, ps, window):
     close(got2[keep], want[keep], torch.bfloat16)
 
 
+@pytest.mark.parametrize("kernel,hd", [("sm100", 64), ("bf16", 64), ("bf16", 48), ("decode", 64), ("order-fixed", 64)])
+@pytest.mark.parametrize("nH,nKV,ps,window,n_splits", [(4, 2, 16, None, 1), (3, 1, 8, 100, 1), (2, 1, 64, None, 1), (8, 2, 32, 70, 1),
+                                                       (4, 1, 16, None, 3)])
+def test_attention_keeps_out_what_no_row_sees(kernel, hd, nH, nKV, ps, window, n_splits):
+    """Slots behind a request's last token and in front of its window, and pages of nobody, hold infinities and NaN, as a request
+    whose values overflowed leaves them: the same outputs, bit for bit, as with ordinary numbers there."""
+    q_lens, ctx = ([1] * 6, [0, 15, 16, 777, 255, 3300]) if kernel == "decode" else ([3, 1, 150, 128, 2, 129, 400, 70], [0, 37, 5, 64, 63, 131, 77, 3300])
+    k, v, table, pos, re = _paged_setup(torch.bfloat16, nKV, hd, ps, q_lens, ctx, num_pages=6500 // ps + 64)
+    cu, cb = _cu(q_lens, ctx)
+    n = sum(q_lens)
+    q = rnd(n, nH * hd, dtype=torch.bfloat16, seed=12)
+    seen = torch.zeros(k.shape[0], ps, dtype=torch.bool)
+    host = table.cpu()
+    for e, (m, b) in enumerate(zip(q_lens, ctx)):
+        for j in range(0 if window is None else max(0, b - window + 1), m + b):
+            seen[int(host[e, j // ps]), j % ps] = True
+    args, got = (nH, window, 1 / math.sqrt(hd)), []
+    for _ in range(2):
+        out = torch.full_like(q, 7.0)
+        if kernel == "sm100":
+            scratch = torch.empty(max(1, ops().attn_prefill_scratch_floats(n, nH, hd, n_splits)), device=DEV)
+            ops().attn_prefill_sm100(q, k, v, table, cu, cb, out, len(q_lens), max(q_lens), *args, False, None, scratch, n_splits)
+        elif kernel == "bf16":
+            ops().attn_prefill_bf16(q, k, v, table, cu, cb, out, len(q_lens), max(q_lens), *args, False)
+        elif kernel == "decode":
+            scratch = torch.empty(max(1, ops().attn_decode_scratch_floats(n, nH, hd, n_splits)), device=DEV)
+            ops().attn_decode_bf16(q, k, v, table, cu, cb, out, scratch, n, *args, n_splits, max(ctx) + 1)
+        else:
+            ops().attention_generic(q, k, v, table, pos, re, out, *args)
+        got.append(out)
+        k.permute(0, 2, 1, 3)[~seen] = float("nan")
+        v.permute(0, 2, 1, 3)[~seen] = float("inf")
+        v[:, :, ::2].permute(0, 2, 1, 3)[~seen[:, ::2]] = float("nan")
+    assert ops().gemm_status(DEV) == 0
+    assert bool(torch.isfinite(got[0].float()).all()) and torch.equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("n_splits,window", [(2, None), (3, None), (4, None), (2, 2500), (4, 300)])
 def test_attn_prefill_sm100_cut_into_runs_of_keys(n_splits, window):
     """The same kernel with the keys of every block cut into runs that a second kernel merges: a
