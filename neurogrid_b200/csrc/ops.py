@@ -1303,18 +1303,23 @@ _GEMM_ARGS = [_c_void_p] * 4 + [_c_int] * 9 + [_c_float, _c_float, _c_void_p, _c
 # Steps of at most FUSE_MAX_ROWS rows (bfloat16, tcgen05 backend) add the products that end a
 # mixer or a feed-forward straight into the float32 residual stream (red.global.add in the
 # epilogue): the norm kernel that follows has no partial sums to read.  Measured on the decode
-# graph of the 1.2B shape: batch 8 0.887 -> 0.852 ms, batch 64 1.329 -> 1.233 ms.  From 65 to 128 rows, two token tiles of 64
-# and K cut so that the blocks fill the GPU beat the library's product of a feed-forward's second matrix (128 rows; hidden
-# 1,024 / 1,536 / 2,048: 5.2 / 7.8 / 10.6 us against 8.0 / 11.2 / 13.2) and of a mixer's output (3.3 / 4.1 / 5.4 against
-# 3.9 / 4.9 / 6.1), whose result the norm kernel would also have to read; at 256 rows they no longer do (6.3 / 7.6 / 9.8 us
-# against 4.0 / 5.3 / 6.4 for the output).
-FUSE_MAX_ROWS = min(128, int(os.environ.get("NEUROGRID_B200_FUSE_ROWS", "128")))
+# graph of the 1.2B shape: batch 8 0.887 -> 0.852 ms, batch 64 1.329 -> 1.233 ms.
+FUSE_MAX_ROWS = min(64, int(os.environ.get("NEUROGRID_B200_FUSE_ROWS", "64")))
 FUSE_RED = os.environ.get("NEUROGRID_B200_FUSE_RED", "1") == "1"
 GEMM_BACKEND = os.environ.get("NEUROGRID_B200_GEMM", "sm100")     # "sm100": tcgen05 kernel; "cublas": vendor library
 # Rows up to which the tcgen05 kernel is used.  It streams weights at memory speed, which is the
 # whole job when a step has few rows; for long portions the vendor library's product is still
 # faster than this one-tile-per-block kernel, so it stands there.
 SM100_MAX_ROWS = int(os.environ.get("NEUROGRID_B200_GEMM_MAX_ROWS", "64"))
+# From 65 to RESIDUAL_MAX_ROWS rows the products that end a mixer or a feed-forward are this kernel's all the same: two token
+# tiles of 64, K cut so that the blocks fill the GPU, a stack of float32 partial sums that the norm kernel adds up in order (a
+# prompt of so many tokens gives the same bits every time, which red.global.add would not).  128 rows, the norm behind it included, hidden
+# 1,024 / 1,536 / 2,048: second matrix of a feed-forward 8.5 / 11.6 / 13.7 us against 11.1 / 14.3 / 16.2 with the library's product
+# (red.global.add 6.9 / 9.4 / 12.3), a mixer's output 6.2 / 7.9 / 8.2 against 5.8 / 8.0 / 8.8 (5.2 / 5.9 / 6.8).  At 256 rows the
+# library is the faster (4.0 / 5.3 / 6.4 us for the output without the norm against 6.3 / 7.6 / 9.8 of this kernel).
+# NEUROGRID_B200_GEMM_MAX_ROWS, where it is set, bounds these products as well.
+RESIDUAL_MAX_ROWS = 128 if "NEUROGRID_B200_GEMM_MAX_ROWS" not in os.environ else min(128, SM100_MAX_ROWS)
+RESIDUAL_STACK_SPLITS = 8
 _status_word = {}
 
 
@@ -1419,22 +1424,29 @@ def linear_to_residual(x: torch.Tensor, weight: torch.Tensor, bias: Optional[tor
     is a stream of the weights, and splitting K puts every SM on it.
 
     ``residual`` (float32 [M,N]): the product is added straight into it when the kernel can
-    do that, and None is returned: nothing is left for the caller to add."""
+    do that, and None is returned: nothing is left for the caller to add.  (65 to RESIDUAL_MAX_ROWS
+    rows: a stack, in an order that is fixed.)"""
     M, K = x.shape
     N = weight.shape[0]
-    adds = bias is None and residual is not None and residual_add_fusable(x, weight)
-    if adds or (bias is None and M <= 64 and gemm_sm100_ok(x, weight)):
-        tiles = -(-N // 128) * -(-M // 64)
+    if bias is None and residual is not None and M > 64 and residual_product_ours(x, weight):
+        s = gemm_splits(K, min(RESIDUAL_STACK_SPLITS, max(1, sm_count(weight.device) // (-(-N // 128) * 2)), max(1, -(-K // 64) // 4)))
+        # (never more than the partial sums of 64 rows in MAX_RESIDUAL_SPLITS splits)
+        buf = ws.flat(name + "_partials", s * M * N, torch.float32, reserve=MAX_RESIDUAL_SPLITS * min(ws.max_rows, 64) * N)
+        buf = buf[: s * M * N].view(s, M, N)
+        gemm_sm100(x, weight, None, buf, splits=s, token_tile=64)
+        return buf
+    if bias is None and M <= 64 and gemm_sm100_ok(x, weight):
+        tiles = -(-N // 128)
         want = min(MAX_RESIDUAL_SPLITS, max(1, sm_count(weight.device) // tiles), max(1, -(-K // 64) // 4))
         s = gemm_splits(K, want)
-        if adds:
+        if residual is not None and residual_add_fusable(x, weight):
             _f32(residual, "residual")
             f = _fn("gemm_sm100", "ng_gemm_sm100", _GEMM_ARGS)
-            _check(f(_ptr(x), _ptr(weight), None, _ptr(residual), M, N, K, N, N, 3, s, 0, 64 if M > 64 else 0, 0.0, 0.0,
+            _check(f(_ptr(x), _ptr(weight), None, _ptr(residual), M, N, K, N, N, 3, s, 0, 0, 0.0, 0.0,
                      _ptr(_gemm_status(weight.device)), _stream()), "gemm_sm100 (residual add)")
             return None
         if s > 1:
-            # partial sums exist for steps of at most 64 rows only
+            # partial sums in up to MAX_RESIDUAL_SPLITS splits exist for steps of at most 64 rows only
             buf = ws.flat(name + "_partials", s * M * N, torch.float32,
                           reserve=MAX_RESIDUAL_SPLITS * min(ws.max_rows, 64) * N)
             buf = buf[: s * M * N].view(s, M, N)
@@ -1465,9 +1477,15 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, ws, name: str):
 
 def residual_add_fusable(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether ``linear_to_residual(x, weight, None, ..., residual=h)`` adds the product into ``h`` itself."""
+    return FUSE_RED and x.shape[0] <= min(64, FUSE_MAX_ROWS) and gemm_sm100_ok(x, weight)
+
+
+def residual_product_ours(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether ``linear_to_residual(x, weight, None, ..., residual=h)`` is the tcgen05 kernel's: added into ``h`` itself, or a
+    stack of partial sums in a fixed order (65 to RESIDUAL_MAX_ROWS rows)."""
     M = x.shape[0]
-    return FUSE_RED and M <= FUSE_MAX_ROWS and (gemm_sm100_ok(x, weight) if M <= 64 else
-                                                GEMM_BACKEND == "sm100" and gemm_sm100_takes(x, weight))
+    return residual_add_fusable(x, weight) if M <= 64 else (
+        FUSE_RED and M <= RESIDUAL_MAX_ROWS and GEMM_BACKEND == "sm100" and gemm_sm100_takes(x, weight))
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> None:

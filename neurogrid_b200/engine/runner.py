@@ -355,7 +355,7 @@ class ModelRunner:
     def _fuse_rows(self, n_rows: int) -> bool:
         from ..csrc import ops
         return (self._on_cuda and self.dtype == torch.bfloat16 and ops.GEMM_BACKEND == "sm100"
-                and ops.FUSE_RED and n_rows <= ops.FUSE_MAX_ROWS)
+                and ops.FUSE_RED and (n_rows <= ops.FUSE_MAX_ROWS or 64 < n_rows <= ops.RESIDUAL_MAX_ROWS))
 
     def _apply_feed(self, ctx) -> None:
         """Overwrite fed rows of the step's tokens with tokens that are still on the device."""

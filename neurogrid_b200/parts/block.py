@@ -238,7 +238,7 @@ class ParallelBlock:
             return self.ffn.forward(x, ctx) if self.ffn is not None else None
         ka = self.mixer.inner_width()
         inner = ctx.ws.buf("parallel_inner", n, self.w_out.shape[1], self.dtype)
-        fused = ctx.fuse_residual and ops.residual_add_fusable(inner, self.w_out) and \
+        fused = ctx.fuse_residual and ops.residual_product_ours(inner, self.w_out) and \
             (self.b_out is None or getattr(self.norm, "takes_post", False))
         if fused and self.b_out is not None:
             x = self.norm.forward(h, pending, buf, post=self.b_out_f32)
