@@ -603,3 +603,30 @@ NG_EXPORT int ng_mapped_attention(const void* q, const void* k_pages, const void
     if (act_bf16) return n_maps == 2 ? ma_launch<__nv_bfloat16, 2>(p, n_rows, stream) : ma_launch<__nv_bfloat16, 1>(p, n_rows, stream);
     return n_maps == 2 ? ma_launch<float, 2>(p, n_rows, stream) : ma_launch<float, 1>(p, n_rows, stream);
 }
+
+// The runs' states of every (row, head) merged and the heads finished (maps combined, head norm), for states that another
+// kernel left in `partial` (float32 [n_rows, nH, n_splits, n_maps, dv + 2]: maximum, sum, weighted values).  Rows of no
+// entry get zeros.  `sinks` (per head, or null) adds exp(sink) to every head's sum.  `sigmoid`: the weights are not
+// normalised (the states' maxima are 0 and their sums not read); `gate` as above.
+NG_EXPORT int ng_mapped_attention_merge(float* partial, const int* row_entry, void* out, int out_ld, int n_rows, int nH,
+                                        int n_maps, int dv, int n_splits, float lambda, float post_scale, float eps,
+                                        int head_norm, const float* sinks, int sigmoid, const void* gate, int gate_ld, int act_bf16,
+                                        cudaStream_t stream) {
+    if (n_rows <= 0) return NG_OK;
+    if (!partial || dv <= 0 || dv > 64 * MA_DVU || nH <= 0 || nH > 65535 || n_maps < 1 || n_maps > 2 || n_splits < 1 || out_ld < nH * dv ||
+        (sigmoid && (n_maps != 1 || sinks)) || (gate && gate_ld < nH))
+        return NG_BAD_SIZE;
+    MaParams p{nullptr, nullptr, nullptr, nullptr, 0, nullptr, row_entry, out, out_ld, partial, nH, 1, 0, dv, 1, 0, 0, 0, n_splits, 0,
+               0.f, 0.f, lambda, post_scale, eps, head_norm, nullptr, sinks, sigmoid, nullptr, gate, gate_ld};
+    dim3 grid(n_rows, nH);
+    const size_t smem = ((size_t)n_maps * dv + n_splits) * sizeof(float);
+    if (smem > 48 * 1024) return NG_BAD_SIZE;
+    if (act_bf16) {
+        if (n_maps == 2) NG_LAUNCH((mapped_attention_merge_kernel<__nv_bfloat16, 2>), grid, MA_THREADS, smem, stream, p);
+        else NG_LAUNCH((mapped_attention_merge_kernel<__nv_bfloat16, 1>), grid, MA_THREADS, smem, stream, p);
+    } else {
+        if (n_maps == 2) NG_LAUNCH((mapped_attention_merge_kernel<float, 2>), grid, MA_THREADS, smem, stream, p);
+        else NG_LAUNCH((mapped_attention_merge_kernel<float, 1>), grid, MA_THREADS, smem, stream, p);
+    }
+    return ng_launch_status();
+}

@@ -40,7 +40,8 @@ struct MmaParams {
     int nH, nG, page_size, num_pages, window, keep_first;
     int chunk;                         // > 0: a row sees only the keys of its own chunk of that many positions (counted from 0)
     float scale, softcap, lambda, post_scale, eps; int head_norm;
-    int n_splits, n_rows; const int* row_entry;       // GROUP: runs of keys (a cluster's blocks); rows of no entry get zeros
+    int n_splits, n_rows; const int* row_entry;       // runs of keys; CLUSTER: rows of no entry get zeros
+    float* partial;                    // RUNS: the runs' states [row, head, run, map, DV + 2]
     const float* slopes; const float* sinks;    // per head or null: slope * (pos - key position) off every score; exp(sink) in the sum
     const float* score_bias;           // SIGMOID: added to head h's scores, or null
     const bf16* gate; int gate_ld;     // a logit per row and head, rows gate_ld apart, or null
@@ -97,15 +98,19 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t&
     lo = pack2(xr - xm, yr - ym);
 }
 
-// GROUP: for entries that bring one token.  The rows of the tile are then the query heads of one KV group (up to 16; they
-// share keys and values and here also the position), a block takes (run of keys, entry, KV group), the warps of a map
-// take different keys of every tile (each keeps a softmax state of its own; merged in warp order at the end).  The runs of an
-// (entry, KV group) are the blocks of a cluster: each leaves its state (maximum, sum, weighted values) in its shared memory,
-// and the finished heads are dealt over the blocks, which read the states through distributed shared memory and merge
-// them in run order.  A step of single tokens is bound by latency, not by the keys' bytes: keys older than the step's own
-// token are requested before the kernel in front has ended, and there is no second launch to merge the runs.  8 rows behind
-// 512 tokens, inside a step's graph: 10.9 us with two maps (14.4 us and 8.4 us for the merge as a launch), 7.2 us with one
-// (8.7 + 4.2); 13.4 and 8.6 us with only the first tile asked for up front and one map's states read after the other's.
+// CLUSTER and RUNS: for entries that bring one token.  The rows of the tile are then the query heads of one KV group (up to 16;
+// they share keys and values and here also the position), a block takes (run of keys, entry, KV group), the warps of a map
+// take different keys of every tile (each keeps a softmax state of its own; merged in warp order at the end).
+// CLUSTER: the runs of an (entry, KV group), up to eight, are the blocks of a cluster: each leaves its state (maximum, sum,
+// weighted values) in its shared memory, and the finished heads are dealt over the blocks, which read the states through
+// distributed shared memory and merge them in run order.  A short context is bound by latency, not by the keys' bytes: keys
+// older than the step's own token are requested before the kernel in front has ended, and there is no second launch to merge
+// the runs.  8 rows behind 512 tokens, inside a step's graph: 10.9 us with two maps (14.4 us and 8.4 us for the merge as a
+// launch), 7.2 us with one (8.7 + 4.2); 13.4 and 8.6 us with only the first tile asked for up front and one map's states read
+// after the other's.
+// RUNS: the states go to memory, for the kernel that merges them (mapped_attention.cu), in as many runs as the caller asks for.
+// A long context is bound by the tiles each block walks (the figures stand at the rule, parts/mapped_attention.py).
+enum { PORTION = 0, CLUSTER = 1, RUNS = 2 };
 template <int M>
 constexpr size_t smem_bytes() {
     constexpr size_t ROWS = (WARPS / M) * 16;
@@ -117,9 +122,10 @@ constexpr size_t smem_bytes() {
 template <int M>
 constexpr int blocks_per_sm() { return smem_bytes<M>() + 4096 <= 227 * 1024 / 3 ? 3 : 2; }
 
-template <int M, bool GROUP>
+template <int M, int FORM>
 __global__ void __launch_bounds__(THREADS, blocks_per_sm<M>())
 mapped_attention_mma_kernel(const MmaParams p) {
+    constexpr bool GROUP = FORM != PORTION;
     constexpr int ROWS = (WARPS / M) * 16;               // rows of a block
     constexpr int PARTS = GROUP ? WARPS / M : 1;         // warps that share a tile's keys
     constexpr int KW = KT / PARTS;                       // keys of a tile that a warp works on
@@ -137,7 +143,7 @@ mapped_attention_mma_kernel(const MmaParams p) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int q0 = p.cu_q[entry], q_len = p.cu_q[entry + 1] - q0;
     const int r0 = GROUP ? 0 : blockIdx.x * ROWS;        // first row of the block within the entry
-    if (GROUP && blockIdx.x == 0) {                      // rows of no entry: defined output (row r is looked at by entry r mod entries)
+    if (FORM == CLUSTER && blockIdx.x == 0) {            // rows of no entry: defined output (row r is looked at by entry r mod entries)
         const int cols = (p.nH / p.nG) * DV;
         for (int r = entry; r < p.n_rows; r += gridDim.y)
             if (p.row_entry[r] < 0) {
@@ -236,15 +242,15 @@ mapped_attention_mma_kernel(const MmaParams p) {
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     lookup(t_begin, 0);
-    if (GROUP) lookup(t_begin + KT, 1);
+    if (FORM == CLUSTER) lookup(t_begin + KT, 1);
     __syncthreads();
-    // the first tile, if all its keys are older than the step (an earlier step wrote them), before the wait; of a single
-    // token's run the second one too
+    // the first tile, if all its keys are older than the step (an earlier step wrote them), before the wait; of a
+    // cluster's run the second one too
     auto is_old = [&](int t0) {
         const int t_last = min(n_keys, t0 + KT) - 1;
         return t_last < t0 || (t_last < n_sink ? t_last : lo + (t_last - n_sink)) < before;
     };
-    const bool old_tile = is_old(t_begin), old_second = GROUP && old_tile && t_begin + KT < n_keys && is_old(t_begin + KT);
+    const bool old_tile = is_old(t_begin), old_second = FORM == CLUSTER && old_tile && t_begin + KT < n_keys && is_old(t_begin + KT);
     if (old_tile) copy_tile(0, 0);
     if (old_second) copy_tile(1, 1);
     ng_pdl_wait();
@@ -270,7 +276,7 @@ mapped_attention_mma_kernel(const MmaParams p) {
         // the lookup of tile it+1 goes to slot (it+1) % 3: slower warps may still read tile it-1's positions (slot
         // (it-1) % 3) and tile it's copies were made from slot it % 3; the slot's last readers (tile it-2) passed the
         // barrier of the iteration before
-        const bool asked = GROUP && it == 0;             // (looked up, and copied if old, in front of the loop)
+        const bool asked = FORM == CLUSTER && it == 0;             // (looked up, and copied if old, in front of the loop)
         if (more && !asked) lookup(t0 + KT, (it + 1) % 3);
         if (asked && old_second) asm volatile("cp.async.wait_group 1;" ::: "memory");
         else asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -402,9 +408,9 @@ mapped_attention_mma_kernel(const MmaParams p) {
     l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
     l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
     if (GROUP) {
-        // the warps' states through shared memory, over the tiles; then, per head and map, their sum in warp order: maximum,
-        // sum and weighted values of the block's run, in the tiles' place as well
-        float* Rs = Os + (size_t)WARPS * 16 * DV;        // [16][M][DV + 2]
+        // the warps' states through shared memory, over the tiles; then, per head and map, their sum in warp order: maximum
+        // (RUNS: natural logarithm), sum and weighted values of the block's run, in the tiles' place as well or in memory
+        float* Rs = Os + (size_t)WARPS * 16 * DV;        // CLUSTER: [16][M][DV + 2]
         if (tq == 0) {
             part_m[warp][gq] = m_a; part_m[warp][gq + 8] = m_b;
             part_l[warp][gq] = l_a; part_l[warp][gq + 8] = l_b;
@@ -426,8 +432,9 @@ mapped_attention_mma_kernel(const MmaParams p) {
                 f[x] = mx == -INFINITY ? 0.f : ex2f(mx - mt);
                 lt += part_l[m + x * M][r] * f[x];
             }
-            float* ps = Rs + (size_t)rm * (DV + 2);
-            if (lane == 0) { ps[0] = mt; ps[1] = lt; }
+            float* ps = FORM == CLUSTER ? Rs + (size_t)rm * (DV + 2)
+                                        : p.partial + ((((size_t)q0 * p.nH + head + r) * p.n_splits + blockIdx.x) * M + m) * (DV + 2);
+            if (lane == 0) { ps[0] = FORM == CLUSTER ? mt : mt * 0.6931471805599453f; ps[1] = lt; }
             for (int c = lane; c < DV; c += 32) {
                 float a = 0.f;
 #pragma unroll
@@ -435,6 +442,7 @@ mapped_attention_mma_kernel(const MmaParams p) {
                 ps[2 + c] = a;
             }
         }
+        if (FORM == RUNS) return;
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
         // a warp finishes a head: the runs' states in run order, the maps combined, the head's norm and gate
         const uint32_t rs = (uint32_t)__cvta_generic_to_shared(Rs);
@@ -540,19 +548,20 @@ mapped_attention_mma_kernel(const MmaParams p) {
     }
 }
 
-template <int M, bool GROUP>
+template <int M, int FORM>
 static int mma_launch(const MmaParams& p, int n_entries, int max_q, cudaStream_t stream) {
     constexpr int ROWS = (WARPS / M) * 16;
+    constexpr bool GROUP = FORM != PORTION;
     constexpr size_t smem = smem_bytes<M>();
     static bool attr = false;
     if (!attr) {
-        if (cudaFuncSetAttribute(mapped_attention_mma_kernel<M, GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        if (cudaFuncSetAttribute(mapped_attention_mma_kernel<M, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return NG_LAUNCH_FAILED;
         attr = true;
     }
     dim3 grid(GROUP ? p.n_splits : (max_q + ROWS - 1) / ROWS, n_entries, GROUP ? p.nG : p.nH);
     if (grid.y > 65535 || grid.z > 65535) return NG_BAD_SIZE;
-    if (GROUP) {                                         // as ng_launch, the runs as a cluster
+    if (FORM == CLUSTER) {                               // as ng_launch, the runs as a cluster
         cudaLaunchConfig_t cfg;
         memset(&cfg, 0, sizeof(cfg));
         cfg.gridDim = grid;
@@ -568,10 +577,10 @@ static int mma_launch(const MmaParams& p, int n_entries, int max_q, cudaStream_t
         attr2[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr2;
         cfg.numAttrs = ng_pdl_enabled() ? 2 : 1;
-        cudaLaunchKernelEx(&cfg, mapped_attention_mma_kernel<M, GROUP>, MmaParams(p));
+        cudaLaunchKernelEx(&cfg, mapped_attention_mma_kernel<M, FORM>, MmaParams(p));
         return ng_launch_status();
     }
-    NG_LAUNCH((mapped_attention_mma_kernel<M, GROUP>), grid, THREADS, smem, stream, p);
+    NG_LAUNCH((mapped_attention_mma_kernel<M, FORM>), grid, THREADS, smem, stream, p);
     return ng_launch_status();
 }
 
@@ -592,35 +601,40 @@ NG_EXPORT int ng_mapped_attention_mma(const void* q, const void* k_pages, const 
         return NG_BAD_SIZE;
     MmaParams p{(const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, table, table_stride, cu_q, ctx_before, (bf16*)out,
                 out_ld, nH, nG, page_size, num_pages, window, keep_first, chunk, scale, softcap, lambda, post_scale, eps, head_norm,
-                1, 0, nullptr, slopes, sinks, score_bias, (const bf16*)gate, gate_ld};
+                1, 0, nullptr, nullptr, slopes, sinks, score_bias, (const bf16*)gate, gate_ld};
 #if !NG_MA_SIGMOID
-    if (n_maps == 2) return mma_launch<2, false>(p, n_entries, max_q, stream);
+    if (n_maps == 2) return mma_launch<2, PORTION>(p, n_entries, max_q, stream);
 #endif
-    return mma_launch<1, false>(p, n_entries, max_q, stream);
+    return mma_launch<1, PORTION>(p, n_entries, max_q, stream);
 }
 
+// Blocks of the kernel below that an SM holds.
+NG_EXPORT int ng_mapped_attention_group_blocks(int n_maps) { return n_maps == 2 ? blocks_per_sm<2>() : blocks_per_sm<1>(); }
+
 // The same for entries of one token: the heads of a KV group are the rows of a tile (nH / nG <= 16), every row's keys are
-// cut into n_splits runs (at most eight: the blocks of a cluster).  Entries of another length are left alone; the n_rows
-// rows of no entry (row_entry < 0) get zeros.
+// cut into n_splits runs.  Entries of another length are left alone.  Without `partial` the runs (at most eight) are the blocks of
+// a cluster that finish the heads, and the n_rows rows of no entry (row_entry < 0) get zeros.  With `partial` (float32 [N, nH,
+// n_splits, n_maps, DV + 2]: maximum, sum, weighted values) the runs' states go there, for the kernel that merges them and
+// finishes the heads (mapped_attention.cu); out and what belongs to the last step are not touched.
 NG_EXPORT int ng_mapped_attention_group(const void* q, const void* k_pages, const void* v_pages, const int* table,
                                         int table_stride, const int* cu_q, const int* ctx_before, const int* row_entry, void* out,
-                                        int out_ld, int n_rows, int n_entries, int n_splits, int nH, int nG, int n_maps, int d,
-                                        int dv, int page_size, int num_pages, int window, int keep_first, float scale,
+                                        int out_ld, float* partial, int n_rows, int n_entries, int n_splits, int nH, int nG, int n_maps,
+                                        int d, int dv, int page_size, int num_pages, int window, int keep_first, float scale,
                                         float softcap, float lambda, float post_scale, float eps, int head_norm,
                                         const float* slopes, const float* sinks, int chunk, int sigmoid,
                                         const float* score_bias, const void* gate, int gate_ld, cudaStream_t stream) {
     if (n_entries <= 0) return NG_OK;
     if (d != D || dv != DV || nH <= 0 || nG <= 0 || nH % nG || nH / nG > 16 || page_size <= 0 || n_maps < 1 || n_maps > 2 ||
-        window < 0 || keep_first < 0 || chunk < 0 || (chunk > 0 && keep_first > 0) || n_splits < 1 || n_splits > 65535 ||
+        window < 0 || keep_first < 0 || chunk < 0 || (chunk > 0 && keep_first > 0) || n_splits < 1 || n_splits > (partial ? 65535 : 8) ||
         out_ld < nH * dv || ((uintptr_t)q & 15) ||
         ((uintptr_t)k_pages & 15) || ((uintptr_t)v_pages & 15) || (sigmoid != 0) != SIGMOID || (SIGMOID && (n_maps != 1 || sinks)) ||
         (gate && gate_ld < nH))
         return NG_BAD_SIZE;
     MmaParams p{(const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, table, table_stride, cu_q, ctx_before, (bf16*)out,
                 out_ld, nH, nG, page_size, num_pages, window, keep_first, chunk, scale, softcap, lambda, post_scale, eps, head_norm,
-                n_splits > 8 ? 8 : n_splits, n_rows, row_entry, slopes, sinks, score_bias, (const bf16*)gate, gate_ld};
+                n_splits, n_rows, row_entry, partial, slopes, sinks, score_bias, (const bf16*)gate, gate_ld};
 #if !NG_MA_SIGMOID
-    if (n_maps == 2) return mma_launch<2, true>(p, n_entries, 1, stream);
+    if (n_maps == 2) return partial ? mma_launch<2, RUNS>(p, n_entries, 1, stream) : mma_launch<2, CLUSTER>(p, n_entries, 1, stream);
 #endif
-    return mma_launch<1, true>(p, n_entries, 1, stream);
+    return partial ? mma_launch<1, RUNS>(p, n_entries, 1, stream) : mma_launch<1, CLUSTER>(p, n_entries, 1, stream);
 }

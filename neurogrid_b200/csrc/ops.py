@@ -590,6 +590,14 @@ def mapped_attention_sm100(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torc
            "mapped_attention_sm100")
 
 
+MAPPED_CLUSTER_RUNS = 8       # blocks of a cluster
+
+
+def mapped_attention_group_blocks(dim: int, vdim: int, n_maps: int, sigmoid: bool = False) -> int:
+    """Blocks of ``mapped_attention_group`` that an SM holds."""
+    return int(_fn("mapped_attention_mma", "ng_mapped_attention_group_blocks", [_c_int], mapped_attention_mma_defines(dim, vdim, sigmoid))(n_maps))
+
+
 def mapped_attention_group_takes(dim: int, vdim: int, n_heads: int, n_kv_heads: int, dtype) -> bool:
     """Whether single-token entries can run with the heads of a KV group as the rows of a tensor-core tile."""
     return mapped_attention_mma_takes(dim, vdim, dtype) and n_heads // n_kv_heads <= 16
@@ -604,8 +612,10 @@ def mapped_attention_group(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torc
                            sigmoid: bool = False, score_bias: Optional[torch.Tensor] = None,
                            gate: Optional[torch.Tensor] = None) -> None:
     """``mapped_attention`` for a step whose entries bring one token each (bfloat16), on the tensor cores: the query
-    heads of a KV group are the rows of a tile, every row's keys are cut into ``n_splits`` runs (at most eight, the blocks of a
-    cluster, which merge the runs' states, combine the maps and norm the heads).  ``partial`` is not used (None will do)."""
+    heads of a KV group are the rows of a tile, every row's keys are cut into ``n_splits`` runs (a block each).  Without ``partial``
+    the runs (at most eight) are the blocks of a cluster, which merge their states, combine the maps and norm the heads.  With it
+    (float32, n_rows * n_heads * n_splits * n_maps * (vdim + 2) values, also for one run) the states pass through it to a second
+    kernel that does so."""
     n = q.shape[0]
     num_pages, n_k, page_size, dim = k_pages.shape
     n_g, vdim = v_pages.shape[1], v_pages.shape[3]
@@ -613,17 +623,29 @@ def mapped_attention_group(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torc
             or q.dtype != torch.bfloat16 or k_pages.dtype != torch.bfloat16 or v_pages.dtype != torch.bfloat16 \
             or out.dtype != torch.bfloat16 or v_pages.shape[0] != num_pages or v_pages.shape[2] != page_size:
         raise KernelError("mapped_attention_group: shapes or dtypes do not fit")
+    need = n * n_heads * n_splits * n_maps * (vdim + 2)
+    if partial is not None and (partial.dtype != torch.float32 or partial.numel() < need):
+        raise KernelError(f"mapped_attention_group: the runs need {need} float32 values")
+    if partial is None and not 1 <= n_splits <= MAPPED_CLUSTER_RUNS:
+        raise KernelError(f"mapped_attention_group: more than {MAPPED_CLUSTER_RUNS} runs pass through ``partial``")
     _i32(table, "table"), _i32(cu_q, "cu_q"), _i32(ctx_before, "ctx_before"), _i32(row_entry, "row_entry")
     defines = mapped_attention_mma_defines(dim, vdim, sigmoid)
     sig, bias = _sigmoid_args(sigmoid, score_bias, n_maps, sinks, n_heads)
-    f = _fn("mapped_attention_mma", "ng_mapped_attention_group", [_c_void_p] * 4 + [_c_int] + [_c_void_p] * 4 + [_c_int] * 13
-            + [_c_float] * 5 + [_c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p], defines)
+    f = _fn("mapped_attention_mma", "ng_mapped_attention_group", [_c_void_p] * 4 + [_c_int] + [_c_void_p] * 4 + [_c_int, _c_void_p]
+            + [_c_int] * 12 + [_c_float] * 5 + [_c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p], defines)
     _check(f(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(table), table.shape[1], _ptr(cu_q), _ptr(ctx_before), _ptr(row_entry),
-             out.data_ptr(), _column_block(out, "attention out"), n, n_entries, int(n_splits), n_heads, n_g, n_maps, dim, vdim,
+             out.data_ptr(), _column_block(out, "attention out"), _ptr(partial), n, n_entries, int(n_splits), n_heads, n_g, n_maps, dim, vdim,
              page_size, num_pages, int(window or 0), int(keep_first), float(scale), float(softcap or 0.0), float(lam),
              _post(head_norm, post_scale, out_scale), float(eps), int(bool(head_norm)), _slopes(slopes, n_heads),
              _slopes(sinks, n_heads), int(chunk or 0), sig, bias, *_head_gate(gate, q, n_heads), _stream()),
            "mapped_attention_group")
+    if partial is None:
+        return
+    g = _fn("mapped_attention", "ng_mapped_attention_merge", [_c_void_p] * 3 + [_c_int] * 6 + [_c_float] * 3
+            + [_c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p])
+    _check(g(_ptr(partial), _ptr(row_entry), out.data_ptr(), _column_block(out, "attention out"), n, n_heads, n_maps, vdim,
+             int(n_splits), float(lam), _post(head_norm, post_scale, out_scale), float(eps), int(bool(head_norm)), _slopes(sinks, n_heads), sig,
+             *_head_gate(gate, q, n_heads), 1, _stream()), "mapped_attention_merge")
 
 
 # ----------------------------------------------------------------------------- input convolution

@@ -35,7 +35,8 @@ class MappedAttention:
 
     graph_safe = True      # launches depend on device data and on launch-time constants only
     GROUP_MAX_ROWS = 256   # decode-only steps of up to this many rows run the heads of a KV group as a tensor-core tile
-    GROUP_MAX_RUNS = 8     # ... a row's keys in up to this many runs (the blocks of a cluster)
+    GROUP_MAX_RUNS = 512   # ... with rows * runs a row bounded by this
+    GROUP_LONG_KEYS = 3072 # ... rows that may see so many keys may have their runs merged by a second launch
     TILE_MIN_ROWS = 64     # steps with a portion of at least this many rows (half a tile of the tcgen05 kernel) run on it
     SPLIT_MAX_ROWS = 32    # steps of up to this many rows may cut each row's keys into runs
     SPLIT_MIN_KEYS = 128   # ... of at least this many keys (one tile of the kernel)
@@ -154,10 +155,24 @@ class MappedAttention:
         return min(longest, s.window + s.keep_first) if s.window else longest
 
     def _group_splits(self, n_rows, cache):
-        """Runs a row's keys are cut into when single tokens run as tiles of a KV group's heads (tiles of 64 keys)."""
+        """(Runs a row's keys are cut into when single tokens run as tiles of a KV group's heads, tiles of 64 keys; whether a second
+        launch merges them.)  As many runs as the GPU has room for their blocks at once.  In a cluster a power of two of them, since
+        others leave parts of the GPU unused (64 rows x KV heads behind 512 tokens: 9.4 us with 4 runs, 17.4 with 7).  A second launch
+        behind long contexts where the cluster leaves more than a quarter of the room empty (4 rows x KV heads, one map: 8 runs in
+        a cluster 6.9 / 15.3 / 20.1 / 77.8 us behind 1,024 / 3,072 / 4,096 / 16,384 tokens, 16 runs and a second launch 7.4 / 10.7 /
+        12.9 / 40.1; two maps 10.5 / 25.4 / 33.8 / 136 against 15.5 / 22.1 / 26.3 / 77.6), and for one run, whose loop is then the
+        shorter one (512 behind 2,048 tokens, one map: 179 us against 191; two maps 318 against 315)."""
         s = self.spec
-        want = -(-3 * ops.sm_count(self.device) // max(1, n_rows * s.n_kv_heads))
-        return max(1, min(self.GROUP_MAX_RUNS, want, self._longest(cache) // 64))
+        groups = n_rows * s.n_kv_heads
+        most = max(1, ops.sm_count(self.device) * ops.mapped_attention_group_blocks(s.key_dim, s.value_dim, s.n_maps, self.sigmoid) // groups)
+        longest = self._longest(cache)
+        runs = 1 << (max(1, min(ops.MAPPED_CLUSTER_RUNS, most, longest // 64)).bit_length() - 1)
+        many = min(self.MAX_SPLITS, most, self.GROUP_MAX_RUNS // n_rows)
+        if most == 1:
+            return 1, longest >= (self.GROUP_LONG_KEYS if s.n_maps == 2 else self.GROUP_LONG_KEYS // 3)
+        if longest >= self.GROUP_LONG_KEYS and 4 * runs < 3 * many:
+            return many, True
+        return runs, False
 
     # a block arrangement that ends mixer and feed-forward with ONE product calls ``core`` and multiplies itself
     def inner_width(self):
@@ -228,9 +243,15 @@ class MappedAttention:
                      sigmoid=self.sigmoid, score_bias=self.score_bias, gate=head_gate)
         if ctx.max_q == 1 and n <= self.GROUP_MAX_ROWS and not ctx.fixed_launches and \
                 ops.mapped_attention_group_takes(s.key_dim, s.value_dim, s.n_heads, s.n_kv_heads, self.dtype):
-            n_splits = self._group_splits(n, cache)
+            n_splits, second = self._group_splits(n, cache)
+            partial = None
+            if second:       # (scratch whose bound follows from the layer's sizes is named after them: a layer of other sizes has its own)
+                per_run = ops.mapped_attention_partial_floats(1, s.n_heads, s.n_maps, s.value_dim, 2) // 2
+                partial = ctx.ws.flat(f"mattn_group_partial_{s.n_heads}x{s.n_maps}x{s.value_dim}", n * n_splits * per_run,
+                                      torch.float32,
+                                      reserve=max(self.GROUP_MAX_RUNS, min(ctx.ws.max_rows, self.GROUP_MAX_ROWS)) * per_run)
             ops.mapped_attention_group(q, cache.k_pages, cache.v_pages, cache.table, ctx.cu_q, ctx.ctx_before, ctx.row_entry,
-                                       out, None, ctx.n_entries, s.n_heads, s.n_maps, s.window, s.keep_first,
+                                       out, partial, ctx.n_entries, s.n_heads, s.n_maps, s.window, s.keep_first,
                                        s.softmax_scale, s.softcap or 0.0, self.lam, s.n_maps == 2, 1.0 - s.diff, s.eps, n_splits,
                                        **extra)
             return

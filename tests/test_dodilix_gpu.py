@@ -172,6 +172,11 @@ def _run_attention(kind, q, kp, vp, table, ctx, H, chunk, scale, sinks, n_splits
         partial = torch.empty(n * H * n_splits * (vdim + 2), device=DEV)
         ops().mapped_attention_group(q, kp, vp, table, ctx.cu_q, ctx.ctx_before, ctx.row_entry, out, partial, ctx.n_entries,
                                      H, 1, None, 0, scale, 0.0, 0.0, False, 1.0, 1e-6, n_splits, sinks=sinks, chunk=chunk)
+        if n_splits <= 8:                                 # the runs as a cluster: the same but for the last bit of bfloat16
+            again = torch.empty_like(out)
+            ops().mapped_attention_group(q, kp, vp, table, ctx.cu_q, ctx.ctx_before, ctx.row_entry, again, None, ctx.n_entries,
+                                         H, 1, None, 0, scale, 0.0, 0.0, False, 1.0, 1e-6, n_splits, sinks=sinks, chunk=chunk)
+            assert rel_err(again, out) < 2.0 ** -7
     return out
 
 

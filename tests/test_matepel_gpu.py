@@ -185,6 +185,11 @@ def _attend(kind, q, kp, vp, table, ctx, H, scale, sinks, n_splits=1, out_scale=
         partial = torch.empty(n * H * n_splits * (vdim + 2), device=DEV)
         ops().mapped_attention_group(q, kp, vp, table, ctx.cu_q, ctx.ctx_before, ctx.row_entry, out, partial, ctx.n_entries, *args,
                                      n_splits, sinks=sinks, out_scale=out_scale)
+        if n_splits <= 8:                                 # the runs as a cluster: the same but for the last bit of bfloat16
+            again = torch.empty_like(out)
+            ops().mapped_attention_group(q, kp, vp, table, ctx.cu_q, ctx.ctx_before, ctx.row_entry, again, None, ctx.n_entries, *args,
+                                         n_splits, sinks=sinks, out_scale=out_scale)
+            assert rel_err(again, out) < 2.0 ** -7
     return out.double() / out_scale
 
 

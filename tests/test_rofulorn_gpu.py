@@ -355,10 +355,12 @@ def test_tensor_core_kernel_with_several_entries_in_a_step():
 
 @pytest.mark.parametrize("M,H,G,dim,vdim,window,keep,softcap,n_splits", [
     (1, 8, 2, 64, 64, 200, 0, None, 3), (2, 4, 1, 32, 48, 90, 5, 7.0, 1), (2, 6, 3, 16, 128, None, 0, None, 4),
-    (1, 16, 1, 48, 16, 64, 70, 2.0, 16), (2, 3, 3, 64, 32, 33, 2, None, 2)])
-def test_single_tokens_as_tiles_of_a_group(M, H, G, dim, vdim, window, keep, softcap, n_splits):
+    (1, 16, 1, 48, 16, 64, 70, 2.0, 16), (2, 3, 3, 64, 32, 33, 2, None, 2), (1, 8, 4, 64, 128, None, 0, 9.0, 8), (2, 4, 2, 64, 64, None, 0, None, 7)])
+@pytest.mark.parametrize("form", ["cluster", "second launch"])
+def test_single_tokens_as_tiles_of_a_group(form, M, H, G, dim, vdim, window, keep, softcap, n_splits):
     """Entries of one token after contexts of every kind (nothing, less than a tile, across the kept tokens, long), a
-    padding entry between them; runs that are empty; against the row-by-row kernel."""
+    padding entry between them; runs that are empty; against the row-by-row kernel.  Up to eight runs as a cluster, more are
+    refused; any number through memory, where every run leaves its state."""
     dtype, ps = torch.bfloat16, 8
     o = ops()
     befores = [0, 5, 63, 64, 300, 131]
@@ -385,11 +387,36 @@ def test_single_tokens_as_tiles_of_a_group(M, H, G, dim, vdim, window, keep, sof
     a = torch.full((n, H * vdim), 3.0, dtype=dtype, device=DEV)
     b = torch.full((n, H * vdim), 5.0, dtype=dtype, device=DEV)
     o.mapped_attention(q, kp, vp, table, pos, re, a, H, M, window, keep, 0.3, softcap or 0.0, 0.4, M == 2, 0.6, 1e-5)
-    partial = torch.full((n * H * n_splits * M * (vdim + 2),), float("nan"), device=DEV)
-    o.mapped_attention_group(q, kp, vp, table, cu, cb, re, b, partial, 8, H, M, window, keep, 0.3, softcap or 0.0, 0.4, M == 2,
-                             0.6, 1e-5, n_splits)
+    partial = torch.full((n, H * n_splits * M * (vdim + 2)), float("nan"), device=DEV) if form == "second launch" else None
+    args = (8, H, M, window, keep, 0.3, softcap or 0.0, 0.4, M == 2, 0.6, 1e-5, n_splits)
+    if partial is None and n_splits > 8:
+        with pytest.raises(Exception, match="runs"):
+            o.mapped_attention_group(q, kp, vp, table, cu, cb, re, b, partial, *args)
+        return
+    o.mapped_attention_group(q, kp, vp, table, cu, cb, re, b, partial, *args)
+    assert partial is None or (not bool(torch.isnan(partial[:6]).any()) and bool(torch.isnan(partial[6:]).all()))
     assert bool((b[6:] == 0).all()) and not bool(torch.isnan(b.float()).any())
     assert rel_err(b[:6], a[:6]) < 1.5e-2
+
+
+def test_long_contexts_of_few_rows_get_more_runs():
+    """The plan of single tokens' runs: a power of two in a cluster, never more blocks than fit; 16 runs and a second launch for few
+    rows behind a long context without a window (a window keeps it short)."""
+    from neurogrid_b200.csrc import ops as o
+    plan = {}
+    for window in (None, 1024):
+        spec = MappedAttentionSpec(hidden=72, n_heads=16, n_kv_heads=4, key_dim=64, value_dim=64, position=NoPositionSpec(), softmax_scale=0.1,
+                                   window=window)
+        part = build("mixer", spec, dtype=torch.bfloat16, device=DEV)
+        room = o.sm_count(DEV) * o.mapped_attention_group_blocks(64, 64, 1)
+        for tokens in (512, 2048, 16384):
+            kp = torch.empty(1, 4, 16, 64, dtype=torch.bfloat16, device=DEV)
+            view = PagedView(kp, kp, torch.zeros(1, tokens // 16, dtype=torch.int32, device=DEV))
+            for rows in (1, 2, 8, 16, 24, 64, 256):
+                runs, second = plan[window, tokens, rows] = part._group_splits(rows, view)
+                assert runs * rows * 4 <= max(room, rows * 4) and runs <= tokens // 64 and (second or (runs <= 8 and runs & (runs - 1) == 0))
+    assert plan[None, 16384, 1] == plan[None, 16384, 2] == (16, True) and plan[None, 2048, 1] == (8, False)
+    assert plan[1024, 16384, 1] == (8, False) and plan[None, 512, 16] == (4, False) and plan[None, 16384, 256] == (1, True)
 
 
 def _mixer(spec, dtype, seed=0, owns_cache=True):
