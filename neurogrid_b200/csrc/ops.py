@@ -1291,19 +1291,29 @@ def moe_swiglu_scaled(gate_up: torch.Tensor, weights: torch.Tensor, out: torch.T
 # ----------------------------------------------------------------------------- per-layer token input
 def token_side(h: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, w_gate: torch.Tensor,
                w_proj: torch.Tensor, w_norm: torch.Tensor, row_entry: torch.Tensor, eps: float,
-               status: torch.Tensor) -> None:
+               status: torch.Tensor, scratch: Optional[torch.Tensor] = None) -> None:
     """h[N,H] float32 += rmsnorm(W_proj (gelu_tanh(W_gate h) * table[tokens])) * w_norm; all float32.
-    ``w_proj`` is given transposed, [dim, H]."""
+    ``w_proj`` is given transposed, [dim, H].  ``scratch`` (float32, ``token_side_scratch`` values): with it, steps of few rows
+    whose sizes the fast kernels do not take deal their sums to many blocks."""
     n, H = h.shape
     V, dim = table.shape
     if w_gate.shape != (dim, H) or w_proj.shape != (dim, H) or w_norm.numel() != H:
         raise KernelError("token_side: shapes do not fit")
     for t, what in ((h, "residual stream"), (table, "token table"), (w_gate, "gate"), (w_proj, "proj"), (w_norm, "norm")):
         _f32(t, what)
-    _i32(tokens, "tokens"), _i32(row_entry, "row_entry"), _i32(status, "status")
-    f = _fn("token_side", "ng_token_side", [_c_void_p] * 7 + [_c_int] * 4 + [_c_float, _c_void_p, _c_void_p])
+    _i32(tokens, "tokens"), _i32(row_entry, "row_entry"), _i32(status, "status"), _f32(scratch, "scratch")
+    if scratch is not None and scratch.numel() < token_side_scratch(n, H, dim):
+        raise KernelError("token_side: the scratch is too small")
+    f = _fn("token_side", "ng_token_side", [_c_void_p] * 7 + [_c_int] * 4 + [_c_float, _c_void_p, _c_void_p, _c_void_p])
     _check(f(_ptr(h), _ptr(tokens), _ptr(table), _ptr(w_gate), _ptr(w_proj), _ptr(w_norm), _ptr(row_entry), n, H, dim, V,
-             float(eps), _ptr(status), _stream()), "token_side")
+             float(eps), _ptr(status), _ptr(scratch), _stream()), "token_side")
+
+
+def token_side_scratch(n_rows: int, H: int, dim: int) -> int:
+    """float32 values of scratch with which a step of ``n_rows`` rows runs the kernels of few rows (0: none needed)."""
+    if (dim <= 64 and H <= 2048 and H % 4 == 0) or (n_rows >= 128 and 4 * (H + dim) <= 160 * 1024):
+        return 0
+    return n_rows * (dim + H + (H + 127) // 128)
 
 
 # ----------------------------------------------------------------------------- sampling

@@ -74,5 +74,8 @@ class TokenSide:
 
     def forward(self, h, ctx):
         s = self.spec
+        need = ops.token_side_scratch(h.shape[0], s.hidden, s.dim)
+        rows = ctx.ws.max_rows if ops.token_side_scratch(1 << 20, s.hidden, s.dim) else min(ctx.ws.max_rows, 127)
+        scratch = ctx.ws.flat("side_scratch", need, torch.float32, reserve=ops.token_side_scratch(rows, s.hidden, s.dim)) if need else None
         ops.token_side(h, ctx.tokens, self.table, self.w_gate, self.w_proj, self.w_norm, ctx.row_entry,
-                       s.eps, ctx.status)
+                       s.eps, ctx.status, scratch)

@@ -390,6 +390,35 @@ def test_token_side_sizes(rows, H, dim):
     assert int(status) != 0
 
 
+@pytest.mark.parametrize("rows,H,dim", [(1, 2052, 64), (40, 64, 13000), (5, 64, 13000), (100, 4096, 128), (127, 1025, 65), (128, 2304, 64), (300, 4096, 96),
+                                        (600, 2304, 64), (511, 2048, 64), (1184, 2048, 64), (599, 1024, 80), (600, 1024, 80), (399, 1027, 9), (1185, 2048, 64), (600, 3001, 70), (130, 80, 41000)])
+@pytest.mark.parametrize("given", [False, True])
+def test_token_side_of_any_size(given, rows, H, dim):
+    """Sizes beyond what the cluster and the tiles take, with and without scratch, at the edges of the choice between them;
+    rows too long for a block's shared memory run through scratch alone.  The bound: float32 sums of H and dim terms."""
+    V, g = 20, torch.Generator().manual_seed(rows + H)
+    rnd = lambda *s, std=1.0: (torch.randn(*s, generator=g) * std).to(DEV)  # noqa: E731
+    h, table, wg, wp, wn = rnd(rows, H, std=2.0), rnd(V, dim), rnd(dim, H, std=H ** -0.5), rnd(dim, H, std=dim ** -0.5), rnd(H)
+    toks = torch.randint(0, V, (rows,), generator=g).to(torch.int32).to(DEV)
+    entry = torch.zeros(rows, dtype=torch.int32, device=DEV)
+    if rows > 2:
+        entry[rows // 2] = -1
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    need = ops.token_side_scratch(rows, H, dim)
+    scratch = torch.full((need,), float("nan"), device=DEV) if given and need else None
+    got = h.clone()
+    if scratch is None and 4 * (H + dim) > 160 * 1024:
+        with pytest.raises(Exception):
+            ops.token_side(got, toks, table, wg, wp, wn, entry, 1e-5, status)
+        return
+    ops.token_side(got, toks, table, wg, wp, wn, entry, 1e-5, status, scratch)
+    x = h.double()
+    y = (torch.nn.functional.gelu(x @ wg.double().T, approximate="tanh") * table.double()[toks.long()]) @ wp.double()
+    want = x + y * torch.rsqrt((y * y).mean(-1, keepdim=True) + 1e-5) * wn.double()
+    want[entry < 0] = x[entry < 0]
+    assert int(status) == 0 and rel_err(got, want) < 1e-5 and torch.equal(got[entry < 0], h[entry < 0])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n,H,E,top", [(1, 2048, 16, 4), (8, 512, 3, 3), (5, 516, 40, 32), (255, 2052, 17, 2), (256, 1024, 16, 4),
                                        (515, 1540, 33, 7), (3000, 128, 17, 1), (600, 75, 5, 1), (2, 64, 100, 5)])
