@@ -56,13 +56,15 @@ __device__ __forceinline__ void moe_choose(const float* z, float* out, int E, in
 }
 
 // Few rows: bound by latency (a round trip to memory for the dot products, then the choices one after the other).  A
-// block per row, a warp per expert; a lane holds 2,048 columns of the expert's weights in its registers, the first of them
-// requested before the kernel in front has ended, and the choice is a warp's instead of a thread's walk over all experts:
-// 5.1 us a launch of 8 rows of 2,048 and 16 experts inside a step's graph against 14.6 us.  In this kernel and the next a
+// block per row, a warp per expert; HELD: a lane holds 2,048 columns of the expert's weights in its registers, the first
+// of them requested before the kernel in front has ended, and the choice is a warp's instead of a thread's walk over all
+// experts: 5.1 us a launch of 8 rows of 2,048 and 16 experts inside a step's graph against 14.6 us.  So many registers leave an
+// SM one block; where rows come in many rounds of the SMs, four warps a row that read the weights as they go are faster
+// (2,048 rows, 64 experts of 1,024 / 4,096 columns: 53 / 146 us against 139 / 241).  In these kernels and the next a
 // lane adds its columns in ascending order: the logits' bits depend on H alone.
 #define MR_NI 16                            // float4 a lane holds of an expert's weights
-template <typename T>
-__global__ void __launch_bounds__(512)
+template <typename T, bool HELD>
+__global__ void __launch_bounds__(HELD ? 512 : 128)
 moe_router_kernel(const T* __restrict__ x_, const float* __restrict__ wr, const float* __restrict__ br,
                   float* __restrict__ weights, int H, int E, int top_k) {
     extern __shared__ float z[];               // [E]
@@ -70,10 +72,10 @@ moe_router_kernel(const T* __restrict__ x_, const float* __restrict__ wr, const 
     const int row = blockIdx.x;
     const bool wide = H % 4 == 0;              // four columns a lane and load
     const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 w[MR_NI];
+    float4 w[HELD ? MR_NI : 1];
     auto load_w = [&](int e, int i0) {
 #pragma unroll
-        for (int k = 0; k < MR_NI; ++k) {
+        for (int k = 0; k < (HELD ? MR_NI : 0); ++k) {
             const int i = i0 + lane * 4 + 128 * k;
             w[k] = wide && e < E && i < H ? moe_ld4(wr + (size_t)e * H + i) : none;
         }
@@ -84,7 +86,13 @@ moe_router_kernel(const T* __restrict__ x_, const float* __restrict__ wr, const 
     const T* x = ng_after_wait(x_) + (size_t)row * H;
     for (int e = warp; e < E; e += nwarp) {
         float acc = 0.f;
-        if (wide) {
+        if (wide && !HELD) {
+#pragma unroll 4
+            for (int i = lane * 4; i < H; i += 128) {
+                const float4 xv = moe_ld4(x + i), wv = moe_ld4(wr + (size_t)e * H + i);
+                acc = fmaf(xv.x, wv.x, fmaf(xv.y, wv.y, fmaf(xv.z, wv.z, fmaf(xv.w, wv.w, acc))));
+            }
+        } else if (wide) {
             for (int i0 = 0; i0 < H; i0 += 128 * MR_NI) {
 #pragma unroll
                 for (int k = 0; k < MR_NI; ++k) {
@@ -237,9 +245,10 @@ NG_EXPORT int ng_moe_router(const void* x, const float* wr, const float* br, flo
                             int E, int top_k, int act_bf16, cudaStream_t stream) {
     if (n_rows <= 0) return NG_OK;
     if (H <= 0 || E <= 0 || top_k < 1 || top_k > E || top_k > MOE_MAX_TOP || E > 8192) return NG_BAD_SIZE;
-    // from 256 rows on, where W_r fits a block's shared memory (and its rows allow 16-byte copies)
+    // from 256 rows on (512 of more than 2,048 columns: 256 rows, 8 experts of 4,096 16.3 us, a block a row 6.6), where W_r fits a
+    // block's shared memory and its rows allow 16-byte copies
     const size_t held = ((size_t)E * H + (size_t)MRR_WARPS * E) * sizeof(float);
-    if (n_rows >= 256 && H % 4 == 0 && held <= 200 * 1024 && ((uintptr_t)wr & 15) == 0) {
+    if (n_rows >= (H > 2048 ? 512 : 256) && H % 4 == 0 && held <= 200 * 1024 && ((uintptr_t)wr & 15) == 0) {
         int blocks = (n_rows + MRR_WARPS - 1) / MRR_WARPS;
         if (blocks > 148) blocks = 148;
 #define MRR_GO(T)                                                                                                      \
@@ -258,11 +267,17 @@ NG_EXPORT int ng_moe_router(const void* x, const float* wr, const float* br, flo
     }
     const int threads = 32 * (E < 4 ? 4 : E > 16 ? 16 : E);
     const size_t smem = (size_t)E * sizeof(float);
-    if (act_bf16)
-        NG_LAUNCH((moe_router_kernel<__nv_bfloat16>), n_rows, threads, smem, stream, (const __nv_bfloat16*)x, wr, br, weights,
-                  H, E, top_k);
-    else
-        NG_LAUNCH((moe_router_kernel<float>), n_rows, threads, smem, stream, (const float*)x, wr, br, weights, H, E, top_k);
+    // 1,024 rows: 64 experts of 1,024 columns 71 us with held weights, 51 without; of 4,096 121 and 130; 16 of 4,096 45 and 35
+    const int held_rows = H <= 1024 || E <= 16 ? 512 : 1024;
+#define MR_GO(T)                                                                                                       \
+    do {                                                                                                               \
+        if (n_rows <= held_rows)                                                                                       \
+            NG_LAUNCH((moe_router_kernel<T, true>), n_rows, threads, smem, stream, (const T*)x, wr, br, weights, H, E, top_k); \
+        else                                                                                                           \
+            NG_LAUNCH((moe_router_kernel<T, false>), n_rows, 128, smem, stream, (const T*)x, wr, br, weights, H, E, top_k); \
+    } while (0)
+    if (act_bf16) MR_GO(__nv_bfloat16);
+    else MR_GO(float);
     return ng_launch_status();
 }
 

@@ -421,7 +421,8 @@ def test_token_side_of_any_size(given, rows, H, dim):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n,H,E,top", [(1, 2048, 16, 4), (8, 512, 3, 3), (5, 516, 40, 32), (255, 2052, 17, 2), (256, 1024, 16, 4),
-                                       (515, 1540, 33, 7), (3000, 128, 17, 1), (600, 75, 5, 1), (2, 64, 100, 5)])
+                                       (515, 1540, 33, 7), (3000, 128, 17, 1), (600, 75, 5, 1), (2, 64, 100, 5),
+                                       (512, 1024, 64, 4), (513, 1024, 130, 8), (1024, 1028, 64, 3), (1025, 1028, 64, 3), (511, 2052, 8, 2), (512, 2052, 8, 2)])
 def test_moe_router_choice(dtype, n, H, E, top):
     """A block per row and a warp per row (from 256 rows on), widths of one and of several pieces and not divisible by four;
     more experts than a warp has lanes, and than shared memory holds; of equal logits the
