@@ -497,7 +497,7 @@ mapped_attention_mma_kernel(const MmaParams p) {
                 ss += v[u] * v[u];
             }
             float k = p.post_scale;
-            if (p.gate) k *= rcpf(1.f + ex2f(-1.4426950408889634f * __bfloat162float(gate[(size_t)q0 * p.gate_ld + head + r])));
+            if (p.gate) k *= 1.f / (1.f + expf(-__bfloat162float(gate[(size_t)q0 * p.gate_ld + head + r])));      // as the merging kernel
             if (p.head_norm) k *= rsqrtf(ng_warp_sum(ss) / (float)DV + p.eps);
             bf16* dst = p.out + (size_t)q0 * p.out_ld + (size_t)(head + r) * DV;
 #pragma unroll

@@ -185,6 +185,22 @@ def test_attention_without_softmax(kind, dtype, case, H, G, dim, vdim):
         assert float(want[0].abs().max()) < 0.2 * float(v[0].double().abs().max())
 
 
+@pytest.mark.parametrize("n_splits,through_memory", [(1, False), (8, False), (1, True), (16, True)])
+def test_gate_of_single_tokens_is_exact(n_splits, through_memory):
+    """The factor of the gate per head, read off heads whose values are all one: as exact far below zero, where approximate
+    instructions flush it to zero, as anywhere (the bound: the output's rounding to bfloat16, subnormal ones included)."""
+    H, G, d, ps = 8, 2, 64, 16
+    kp, vp = _x((4, G, ps, d), torch.bfloat16), torch.ones(4, G, ps, d, dtype=torch.bfloat16, device=DEV)
+    table, ctx = torch.arange(4, dtype=torch.int32, device=DEV)[None].contiguous(), make_ctx([1], [50], [0], dtype=torch.bfloat16)
+    q, out = _x((1, H * d), torch.bfloat16, seed=1), torch.empty(1, H * d, dtype=torch.bfloat16, device=DEV)
+    gate = torch.tensor([[-88.0, -87.5, -88.5, -10.0, 0.0, 10.0, 60.0, -60.0]], device=DEV).bfloat16()
+    partial = torch.full((H * n_splits * (d + 2),), float("nan"), device=DEV) if through_memory else None
+    ops().mapped_attention_group(q, kp, vp, table, ctx.cu_q, ctx.ctx_before, ctx.row_entry, out, partial, 1, H, 1, None, 0, 0.125, 0.0, 0.0,
+                                 False, 1.0, 1e-6, n_splits, gate=gate)
+    want = torch.sigmoid(gate.double())[0][:, None]
+    assert bool(((out.view(H, d).double() - want).abs() <= 2.0 ** -8 * want + 2.0 ** -133).all())
+
+
 @pytest.mark.parametrize("kind,dtype", KINDS)
 def test_sigmoid_attention_batch_of_unequal_entries(kind, dtype):
     """Entries of several lengths and contexts in one launch, on pages of one pool in a scrambled order; no bias, no gate."""
