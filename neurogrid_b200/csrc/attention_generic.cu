@@ -21,8 +21,9 @@
 #define AG_TILE 8
 #define AG_MAX_J 24     // head_dim <= 768
 
-// MJ: columns a lane holds (head_dim <= 32 * MJ)
-template <typename T, int MJ>
+// MJ: columns a lane holds (head_dim <= 32 * MJ).  Z: more heads than a grid's second dimension has blocks, the third counts on (a form
+// of its own: one more comparison in all of them cost heads of 257 and more a quarter of their speed)
+template <typename T, int MJ, bool Z>
 __global__ void __launch_bounds__(AG_WARPS * 32)
 attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pages, const T* __restrict__ v_pages,
                          const int* __restrict__ table, int table_stride, const int* __restrict__ positions,
@@ -31,7 +32,8 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pages,
     __shared__ float acc_s[AG_WARPS][32 * MJ], ml_s[2][AG_WARPS];
     ng_pdl_trigger();
     ng_pdl_wait();
-    const int row = blockIdx.x, head = blockIdx.y;
+    const int row = blockIdx.x, head = Z ? blockIdx.z * gridDim.y + blockIdx.y : blockIdx.y;
+    if (Z && head >= nH) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T* o = out + ((size_t)row * nH + head) * hd;
     const int entry = row_entry[row];
@@ -140,18 +142,19 @@ NG_EXPORT int ng_attention_generic(const void* q, const void* k_pages, const voi
                                    float scale, const float* slopes, int act_bf16, cudaStream_t stream) {
     if (n_rows <= 0) return NG_OK;
     if (hd <= 0 || hd > 32 * AG_MAX_J || nH <= 0 || nKV <= 0 || nH % nKV || page_size <= 0) return NG_BAD_SIZE;
-    if (nH > 65535) return NG_BAD_SIZE;
-    dim3 grid(n_rows, nH);
-#define AG_LAUNCH(TT, MJ)                                                                                              \
-    NG_LAUNCH((attention_generic_kernel<TT, MJ>), grid, AG_WARPS * 32, 0, stream, (const TT*)q, (const TT*)k_pages,    \
+    dim3 grid(n_rows, nH < 65535 ? nH : 65535, (nH + 65534) / 65535);
+    if (grid.z > 65535) return NG_BAD_SIZE;
+#define AG_LAUNCH(TT, MJ, Z)                                                                                           \
+    NG_LAUNCH((attention_generic_kernel<TT, MJ, Z>), grid, AG_WARPS * 32, 0, stream, (const TT*)q, (const TT*)k_pages, \
               (const TT*)v_pages, table, table_stride, positions, row_entry, (TT*)out, nH, nKV, hd, page_size, num_pages, \
               window, scale, slopes)
 #define AG_SIZES(TT)                                                                                                   \
     do {                                                                                                               \
-        if (hd <= 64) AG_LAUNCH(TT, 2);                                                                                \
-        else if (hd <= 128) AG_LAUNCH(TT, 4);                                                                          \
-        else if (hd <= 256) AG_LAUNCH(TT, 8);                                                                          \
-        else AG_LAUNCH(TT, 24);                                                                                        \
+        if (grid.z > 1) AG_LAUNCH(TT, 24, true);                                                                       \
+        else if (hd <= 64) AG_LAUNCH(TT, 2, false);                                                                    \
+        else if (hd <= 128) AG_LAUNCH(TT, 4, false);                                                                   \
+        else if (hd <= 256) AG_LAUNCH(TT, 8, false);                                                                   \
+        else AG_LAUNCH(TT, 24, false);                                                                                 \
     } while (0)
     if (act_bf16) AG_SIZES(__nv_bfloat16);
     else AG_SIZES(float);

@@ -316,6 +316,18 @@ def test_attention_generic_row_alone(hd):
             assert torch.equal(one[0], whole[r]), (window, r)
 
 
+@pytest.mark.parametrize("nH", [65535, 65536, 131075])
+def test_attention_generic_of_very_many_heads(nH):
+    """More heads than one dimension of a grid has blocks; the bound: float32 sums of four terms and of 21 weights."""
+    hd, ctx = 4, 20
+    k, v, table, pos, re = _paged_setup(torch.float32, 1, hd, 16, [1], [ctx], num_pages=8)
+    q = rnd(1, nH * hd, seed=3)
+    out = torch.empty_like(q)
+    ops().attention_generic(q, k, v, table, pos, re, out, nH, None, 0.5)
+    kk, vv = (torch.stack([p[int(table[0, j // 16]), 0, j % 16] for j in range(ctx + 1)]).double() for p in (k, v))
+    close(out.view(nH, hd), torch.softmax(q.view(nH, hd).double() @ kk.T * 0.5, -1) @ vv, torch.float32)
+
+
 def test_attention_finds_a_far_key():
     """One key among hundreds, on another page, carries a score that stands out: the output
     must be its value row.  Random pages elsewhere would hide a wrong page or a wrong slot."""
