@@ -522,18 +522,22 @@ attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages,
     }
 }
 
-// out[row, head, :] = sum_s o_s * 2^(m_s - m) / sum_s l_s * 2^(m_s - m).  A block per (row, head), DCC_GROUPS threads a column:
-// group g adds splits g, g + DCC_GROUPS, ... in ascending order, the groups' sums are added in order.  A long context in few
+// out[row, head, :] = sum_s o_s * 2^(m_s - m) / sum_s l_s * 2^(m_s - m).  A block per (row, head), G threads a column:
+// group g adds splits g, g + G, ... in ascending order, the groups' sums are added in order.  A long context in few
 // rows has fifty splits and more, which one thread a column walked one after the other (21 us at 16,384 tokens, one row, 24 heads;
-// now 5.9 us inside a step's graph).  (Splits as the
-// blocks of a cluster, merged there without this launch, took 16.5 us a layer where the two kernels take 15.9: 8 rows, 7 splits.).
+// 5.9 us inside a step's graph with G = 4).  (Splits as the
+// blocks of a cluster, merged there without this launch, took 16.5 us a layer where the two kernels take 15.9: 8 rows, 7 splits.)
 #define DCC_GROUPS 4
-#define DCC_THREADS (HD * DCC_GROUPS)
-static_assert(DCC_THREADS <= 1024, "a column of the head has a thread in every group");
-__global__ void __launch_bounds__(DCC_THREADS)
+template <int G>
+struct Dcc {
+    static constexpr int THREADS = (HD * G + 31) / 32 * 32;
+    static_assert(THREADS <= 1024 && (G == 1 || THREADS == HD * G), "a column of the head has a thread in every group");
+};
+template <int G>
+__global__ void __launch_bounds__(Dcc<G>::THREADS)
 attn_combine_kernel(const float* __restrict__ scratch, const int* __restrict__ cu_q,
                     bf16* __restrict__ out, int nH, int n_splits, int n_rows) {
-    __shared__ float top[(DCC_THREADS + 31) / 32], part[DCC_GROUPS][HD], part_l[DCC_GROUPS];
+    constexpr int THREADS = Dcc<G>::THREADS;
     ng_pdl_trigger();
     const int e = blockIdx.y, head = blockIdx.x;
     const int row = cu_q[e];                                     // the batch description: older than the step's kernels
@@ -543,31 +547,51 @@ attn_combine_kernel(const float* __restrict__ scratch, const int* __restrict__ c
     scratch = ng_after_wait(scratch);
     const float* rec = scratch + ((size_t)row * nH + head) * n_splits * DC_REC;
     const int d = threadIdx.x % HD, g = threadIdx.x / HD;
-    float m = -INFINITY;
-    for (int s = threadIdx.x; s < n_splits; s += DCC_THREADS) m = fmaxf(m, rec[(size_t)s * DC_REC]);
+    float m = -INFINITY, l = 0.f, acc = 0.f;
+    if constexpr (G == 1) {                                      // at most DCC_GROUPS splits: all of them requested at once
+        if (g > 0) return;
+        float ms[DCC_GROUPS], ls[DCC_GROUPS], os[DCC_GROUPS];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = m;
-    __syncthreads();
-    m = top[0];
-#pragma unroll
-    for (int w = 1; w < (DCC_THREADS + 31) / 32; ++w) m = fmaxf(m, top[w]);
-    float l = 0.f, acc = 0.f;
-    if (m > -INFINITY) {
-#pragma unroll 8
-        for (int s = g; s < n_splits; s += DCC_GROUPS) {
-            const float f = exp2f(rec[(size_t)s * DC_REC] - m);
-            l += rec[(size_t)s * DC_REC + 1] * f;
-            acc += rec[(size_t)s * DC_REC + 2 + d] * f;
+        for (int s = 0; s < DCC_GROUPS; ++s) {
+            const float* r = rec + (size_t)s * DC_REC;
+            ms[s] = s < n_splits ? r[0] : -INFINITY;
+            ls[s] = s < n_splits ? r[1] : 0.f;
+            os[s] = s < n_splits ? r[2 + d] : 0.f;
+            m = fmaxf(m, ms[s]);
         }
-    }
-    part[g][d] = acc;
-    if (d == 0) part_l[g] = l;
-    __syncthreads();
-    if (g > 0) return;
-    for (int k = 1; k < DCC_GROUPS; ++k) {
-        l += part_l[k];
-        acc += part[k][d];
+        if (m > -INFINITY)
+#pragma unroll
+            for (int s = 0; s < DCC_GROUPS; ++s) {
+                const float f = exp2f(ms[s] - m);
+                l += ls[s] * f;
+                acc += os[s] * f;
+            }
+    } else {
+        __shared__ float top[THREADS / 32], part[G][HD], part_l[G];
+        for (int s = threadIdx.x; s < n_splits; s += THREADS) m = fmaxf(m, rec[(size_t)s * DC_REC]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = m;
+        __syncthreads();
+        m = top[0];
+#pragma unroll
+        for (int w = 1; w < THREADS / 32; ++w) m = fmaxf(m, top[w]);
+        if (m > -INFINITY) {
+#pragma unroll 8
+            for (int s = g; s < n_splits; s += G) {
+                const float f = exp2f(rec[(size_t)s * DC_REC] - m);
+                l += rec[(size_t)s * DC_REC + 1] * f;
+                acc += rec[(size_t)s * DC_REC + 2 + d] * f;
+            }
+        }
+        part[g][d] = acc;
+        if (d == 0) part_l[g] = l;
+        __syncthreads();
+        if (g > 0) return;
+        for (int k = 1; k < G; ++k) {
+            l += part_l[k];
+            acc += part[k][d];
+        }
     }
     out[((size_t)row * nH + head) * HD + d] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
 }
@@ -606,9 +630,16 @@ static int attn_decode_launch(const void* q, const void* k_pages, const void* v_
         (const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, table, table_stride, cu_q, ctx_before,
         (bf16*)out, scratch, nH, nKV, ps_log2, num_pages, window, scale * 1.4426950408889634f, n_splits, per,
         table_in_smem, n_rows, slopes);
-    if (n_splits > 1)
-        NG_LAUNCH((attn_combine_kernel), dim3(nH, n_entries), DCC_THREADS, 0, stream, scratch, cu_q, (bf16*)out, nH,
-                                                                                   n_splits, n_rows);
+    if (n_splits > 1) {
+        // up to two splits one thread a column is enough, and three or four are worth four only where they are few (32 heads of
+        // 64, 64 rows, 2 splits: 15.4 us with the attention in front against 18.0; 8 rows, 3 splits 7.4 against 6.5; 16 heads of
+        // 128, 8 rows, 4 splits 7.1 against 8.5)
+        if (n_splits > 4 || (n_splits > 2 && (long long)n_splits * nH * n_entries * HD * DCC_GROUPS <= 200000))
+            NG_LAUNCH((attn_combine_kernel<DCC_GROUPS>), dim3(nH, n_entries), Dcc<DCC_GROUPS>::THREADS, 0, stream, scratch, cu_q, (bf16*)out,
+                      nH, n_splits, n_rows);
+        else
+            NG_LAUNCH((attn_combine_kernel<1>), dim3(nH, n_entries), Dcc<1>::THREADS, 0, stream, scratch, cu_q, (bf16*)out, nH, n_splits, n_rows);
+    }
     return ng_launch_status();
 }
 
