@@ -385,7 +385,11 @@ NG_EXPORT int ng_shortconv(const void* p, const float* w, const float* bias, flo
     dim3 grid((H + CONV_THREADS - 1) / CONV_THREADS, (max_q + CONV_TILE - 1) / CONV_TILE, n_entries);
     if (grid.y > 65535 || grid.z > 65535) return NG_BAD_SIZE;
     const size_t ps = (size_t)partial_stride;
-    if (max_q == 1 && n_entries <= 65535) {
+    const bool pairs = act_bf16 && n_partials <= 1 && H % 2 == 0 && ((uintptr_t)p & 3) == 0 && ((uintptr_t)out & 3) == 0 && ((uintptr_t)state & 7) == 0;
+    // single tokens: where a step is large enough to be bound by its accesses, and the input is one tensor, two channels a thread
+    // are faster (L = 3, 64 and 256 rows of 2,048: 2.3 and 4.4 us against 2.7 and 6.1; 64 of 1,024 2.1 each; L = 4: 3.4 and 7.1
+    // against 2.8 and 6.2)
+    if (max_q == 1 && n_entries <= 65535 && !(pairs && NG_CONV_L <= 3 && (long long)n_entries * H > 65536)) {
         dim3 g1((H + CONV_THREADS - 1) / CONV_THREADS, n_entries);
 #define CONV_TOKEN(TI, T, NP, PS)                                                                                      \
     NG_LAUNCH((shortconv_token_kernel<TI, T, NG_CONV_L>), g1, CONV_THREADS, 0, stream, (const TI*)p, w, bias, state, (T*)out, \
@@ -403,8 +407,7 @@ NG_EXPORT int ng_shortconv(const void* p, const float* w, const float* bias, flo
                   (__nv_bfloat16*)out, cu_q, ctx_before, slots, H);
         return ng_launch_status();
     }
-    if (act_bf16 && n_partials <= 1 && H % 2 == 0 && ((uintptr_t)p & 3) == 0 && ((uintptr_t)out & 3) == 0 &&
-        ((uintptr_t)state & 7) == 0) {
+    if (pairs) {
         dim3 g2((H / 2 + CONV_THREADS - 1) / CONV_THREADS, grid.y, grid.z);
         NG_LAUNCH((shortconv_bf16x2_kernel<NG_CONV_L>), g2, CONV_THREADS, 0, stream, (const __nv_bfloat16*)p, w, bias, state,
                   (__nv_bfloat16*)out, cu_q, ctx_before, slots, H);

@@ -179,6 +179,24 @@ def test_shortconv_single_tokens(dtype, L, H, parts):
     assert all(torch.equal(st1[i], st2[i]) for i in (4, 6, 7))             # slots without a token stay
 
 
+@pytest.mark.parametrize("n,L,H", [(64, 3, 1024), (65, 3, 1024), (65, 4, 1024), (200, 2, 514), (130, 3, 515)])
+def test_shortconv_single_tokens_of_many_rows(n, L, H):
+    """Both sides of the size from which two channels a thread take a step of single tokens, widths that do not pair, entries
+    without a token between the others."""
+    lens = [i % 7 != 3 for i in range(n)]
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32).to(DEV)
+    cb, slots = torch.tensor([i % 5 for i in range(n)], dtype=torch.int32, device=DEV), torch.randperm(n, generator=torch.Generator().manual_seed(1)).to(torch.int32).to(DEV)
+    m = sum(lens)
+    p, w, b = rnd(m, 3 * H, dtype=torch.bfloat16, seed=4, std=0.5), rnd(H, L, seed=5, std=0.3), rnd(H, seed=6, std=0.1)
+    st1 = rnd(n, L - 1, H, seed=7)
+    st2 = st1.clone()
+    o1, o2 = (torch.zeros(m, H, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    ops().shortconv(p, w, b, st1, o1, cu, cb, slots, n, 1)
+    ref.shortconv(p, w, b, st2, o2, cu, cb, slots, n, 1)
+    close(o1, o2, torch.bfloat16)
+    close(st1, st2, torch.float32)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H", [4, 132, 1024, 2044, 2048, 4100, 8192, 333, 4102])
 @pytest.mark.parametrize("kind", ["plain", "delta", "stack", "post", "rows"])
