@@ -36,14 +36,16 @@
 // OWN_V: value heads are normed or mixed (a form of its own: the others' values are copied as they are).  PAIRS: pairs of
 // a head a lane holds (d <= 64 * PAIRS).  HB: heads a warp takes at a time, their loads in flight together (steps of
 // many rows, where one block walks all heads of its row).  `wide`: neighbouring pairs, and values in pieces of 16 bytes,
-// lie where one access reaches them.  2,048 rows of 32 + 8 heads of 64: 21.3 us (38.9 us with loads of one element, one
+// lie where one access reaches them; TWO: neighbouring pairs by one access (with eight pairs a
+// lane only where more blocks than fit are launched: 255 rows of 8 + 2 heads of 256 4.1 us against 5.9, but 8 rows 3.5 against 3.0 and
+// 2,048 rows 21.5 against 18.0).  2,048 rows of 32 + 8 heads of 64: 21.3 us (38.9 us with loads of one element, one
 // head at a time and eight pairs' worth of predicated code); 8 rows inside a step's graph: 2.7 us (5.2 us).
 __device__ __forceinline__ float2 prep_ld2(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
 __device__ __forceinline__ float2 prep_ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ void prep_st2(__nv_bfloat16* p, float a, float b) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b); }
 __device__ __forceinline__ void prep_st2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
 
-template <typename T, bool OWN_V, int PAIRS, int HB>
+template <typename T, bool OWN_V, int PAIRS, int HB, bool TWO>
 __global__ void __launch_bounds__(MA_THREADS)
 qkv_prep_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, const float* __restrict__ qw,
                 const float* __restrict__ kw, const float* __restrict__ inv_freq, int rot_dims,
@@ -111,7 +113,7 @@ qkv_prep_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, const float* _
                 if (i < half) {
                     // pair i: (2i, 2i+1), or with half pairing (i, i + rot_dims/2) inside the rotated coordinates
                     const bool hp = half_pairing && i < half_rot;
-                    if (wide && !hp) {
+                    if (TWO && wide && !hp) {
                         const float2 f = prep_ld2(src + 2 * i);
                         x1[hb][u] = f.x;
                         x2[hb][u] = f.y;
@@ -157,7 +159,7 @@ qkv_prep_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, const float* _
                         const float z1 = y1 * c - y2 * s, z2 = y2 * c + y1 * s;
                         y1 = z1; y2 = z2;
                     }
-                    if (wide && !hp) {
+                    if (TWO && wide && !hp) {
                         prep_st2(dst + c1, y1, y2);
                     } else {
                         ng_st(dst + c1, y1);
@@ -237,16 +239,17 @@ NG_EXPORT int ng_qkv_prep(const void* qkv, void* q_out, const float* qw, const f
     const int el = act_bf16 ? 8 : 4;
     const bool wide = d % el == 0 && dv % el == 0 && ld % el == 0 &&
                       (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0;
-#define PREP_LAUNCH(TT, OWN, PAIRS, HB)                                                                                \
-    NG_LAUNCH((qkv_prep_kernel<TT, OWN, PAIRS, HB>), grid, MA_THREADS, smem, stream, (const TT*)qkv, (TT*)q_out, qw, kw, \
+#define PREP_LAUNCH(TT, OWN, PAIRS, HB, TWO)                                                                                \
+    NG_LAUNCH((qkv_prep_kernel<TT, OWN, PAIRS, HB, TWO>), grid, MA_THREADS, smem, stream, (const TT*)qkv, (TT*)q_out, qw, kw, \
               inv_freq, rot_dims, (TT*)k_pages, (TT*)v_pages, table, table_stride, positions, row_entry, nQ, nK, nV, d, dv, \
               page_size, num_pages, eps, status, whole, temp_coef, temp_every, ld, half_pairing, unit_norm, v_is_k,    \
               rot_mag, v_norm, v_mode, v_lambda, v_first, (int)wide)
 #define PREP_SIZES(TT, OWN)                                                                                            \
     do {                                                                                                               \
-        if (d <= 64) { if (head_blocks == 1) PREP_LAUNCH(TT, OWN, 1, 4); else PREP_LAUNCH(TT, OWN, 1, 1); }            \
-        else if (d <= 128) { if (head_blocks == 1) PREP_LAUNCH(TT, OWN, 2, 4); else PREP_LAUNCH(TT, OWN, 2, 1); }      \
-        else PREP_LAUNCH(TT, OWN, MA_MAX_PAIRS, 1);                                                                    \
+        if (d <= 64) { if (head_blocks == 1) PREP_LAUNCH(TT, OWN, 1, 4, true); else PREP_LAUNCH(TT, OWN, 1, 1, true); }            \
+        else if (d <= 128) { if (head_blocks == 1) PREP_LAUNCH(TT, OWN, 2, 4, true); else PREP_LAUNCH(TT, OWN, 2, 1, true); }      \
+        else if (head_blocks > 1 && n_rows * head_blocks > 3 * 148) PREP_LAUNCH(TT, OWN, MA_MAX_PAIRS, 1, true);        \
+        else PREP_LAUNCH(TT, OWN, MA_MAX_PAIRS, 1, false);                                                                    \
     } while (0)
     const bool own_v = (v_norm || v_mode) && nV > 0;
     if (act_bf16) {
