@@ -21,16 +21,17 @@ __device__ __forceinline__ void ng_st(__nv_bfloat16* p, float v) { *p = __float2
 // An input that is either one tensor of type TI, or n_part float32 partial sums `stride`
 // elements apart (split-K products).  The sum is taken in ascending order and rounded to TO, the
 // type the unsplit product would have been stored in, so both routes round at the same place.
-template <typename TO, typename TI>
+// AHEAD: partial sums requested at a time (one at a time, each waits for memory; four at a time cost registers).
+template <typename TO, int AHEAD = 4, typename TI>
 __device__ __forceinline__ float ng_ld_sum(const TI* p, size_t idx, int n_part, size_t stride) {
-    if (n_part <= 1) return ng_ld(p + idx);
+    if (sizeof(TI) < 4 || n_part <= 1) return ng_ld(p + idx);          // (only float32 comes in parts)
     float v = 0.f;
-    for (int s0 = 0; s0 < n_part; s0 += 4) {            // four loads in flight; one at a time, each waits for memory
-        float f[4];
+    for (int s0 = 0; s0 < n_part; s0 += AHEAD) {
+        float f[AHEAD];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) f[k] = s0 + k < n_part ? ng_ld(p + (s0 + k) * stride + idx) : 0.f;
+        for (int k = 0; k < AHEAD; ++k) f[k] = s0 + k < n_part ? ng_ld(p + (s0 + k) * stride + idx) : 0.f;
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < AHEAD; ++k)
             if (s0 + k < n_part) v += f[k];
     }
     TO r;

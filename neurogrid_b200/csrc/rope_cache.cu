@@ -24,16 +24,16 @@ __device__ __forceinline__ float2 rc_ld2(const __nv_bfloat16* q) {
     return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(q));
 }
 __device__ __forceinline__ float2 rc_ld2(const float* q) { return *reinterpret_cast<const float2*>(q); }
-template <typename TO, typename TI>
+template <typename TO, int AHEAD, typename TI>
 __device__ __forceinline__ void rc_load_pair(const TI* __restrict__ qkv, size_t ia, size_t ib, bool adjacent, int n_part,
                                              size_t pstride, float& x1, float& x2) {
     if (!adjacent) {
-        x1 = ng_ld_sum<TO>(qkv, ia, n_part, pstride);
-        x2 = ng_ld_sum<TO>(qkv, ib, n_part, pstride);
+        x1 = ng_ld_sum<TO, AHEAD>(qkv, ia, n_part, pstride);
+        x2 = ng_ld_sum<TO, AHEAD>(qkv, ib, n_part, pstride);
         return;
     }
     float2 f = rc_ld2(qkv + ia);
-    if (n_part > 1) {
+    if (sizeof(TI) == 4 && n_part > 1) {
         f.x += 0.f; f.y += 0.f;
         for (int s = 1; s < n_part; ++s) {
             const float2 g = rc_ld2(qkv + ia + (size_t)s * pstride);
@@ -56,8 +56,14 @@ __device__ __forceinline__ void rc_store_pair(float* dst, int a, int b, bool adj
 
 // HB heads per warp and pass: their loads are all issued before the first is used.  With few
 // rows HB = 1 and a warp per head (parallelism); with many, HB = 4 (loads in flight).
-// ``wide``: pairs are adjacent and every row and page is aligned for two-element accesses.
-template <typename TI, typename T, int HB, int PAIRS>
+// ``wide``: pairs are adjacent and every row and page is aligned for two-element accesses.  HELD: a lane holds its norm weights,
+// requested before the wait (heads of up to 128): 8 rows 1.5 to 1.7 us against 1.8 to 2.1; 256 rows of heads of 128 4.1 against
+// 5.3; from HELD_ROWS on their registers cost more (2,048 rows 18.2 against 16.3).  AHEAD: partial sums requested at a time; up to
+// AHEAD_ROWS rows four (8 rows of 32 + 16 heads of 64, 2 parts 2.0 us against 2.5), beyond them one in heads of up to 64 (64 rows, 4
+// parts 3.2 against 2.7; heads of 128, 2 parts 3.1 against 3.6).
+#define HELD_ROWS 1024
+#define AHEAD_ROWS 32
+template <typename TI, typename T, int HB, int PAIRS, bool HELD, int AHEAD>
 __global__ void __launch_bounds__(RC_THREADS)
 rope_cache_kernel(const TI* __restrict__ qkv, T* __restrict__ q_out, const float* __restrict__ qw,
                   const float* __restrict__ kw, const float* __restrict__ inv_freq, int half_pairing,
@@ -102,8 +108,7 @@ rope_cache_kernel(const TI* __restrict__ qkv, T* __restrict__ q_out, const float
         cs[u] = 1.f;
         if (inv_freq && i < half) sincosf(pf * inv_freq[i], &sn[u], &cs[u]);
     }
-    // and the norms' weights, as far as registers allow
-    constexpr bool HELD = PAIRS <= 2;
+    // and the norms' weights
     float nw[2][HELD ? PAIRS : 1][2];
     if constexpr (HELD)
 #pragma unroll
@@ -127,7 +132,7 @@ rope_cache_kernel(const TI* __restrict__ qkv, T* __restrict__ q_out, const float
                 // unconditional (indices clamped into the row), so that all loads are in flight together
                 const int ic = min(i, half - 1);
                 const int a = half_pairing ? ic : 2 * ic, b = half_pairing ? ic + half : 2 * ic + 1;
-                rc_load_pair<T>(qkv, src + a, src + b, adjacent, n_part, pstride, x1[hb][u], x2[hb][u]);
+                rc_load_pair<T, AHEAD>(qkv, src + a, src + b, adjacent, n_part, pstride, x1[hb][u], x2[hb][u]);
                 if (i >= half) x1[hb][u] = x2[hb][u] = 0.f;
             }
         }
@@ -292,8 +297,12 @@ NG_EXPORT int ng_rope_cache(const void* qkv, void* q_out, const float* qw, const
 #define RC_ARGS(TIN, TT) (const TIN*)qkv, (TT*)q_out, qw, kw, inv_freq, half_pairing, pos_scale, (TT*)k_pages, \
         (TT*)v_pages, table, table_stride, positions, row_entry, nH, nKV, hd, page_size, num_pages, eps, status
 #define RC_GO2(TIN, TT, NP, PS, PAIRS) \
-    do { if (bulk) NG_LAUNCH((rope_cache_kernel<TIN, TT, 4, PAIRS>), grid, RC_THREADS, 0, stream, RC_ARGS(TIN, TT), NP, PS, wide); \
-         else NG_LAUNCH((rope_cache_kernel<TIN, TT, 1, PAIRS>), grid, RC_THREADS, 0, stream, RC_ARGS(TIN, TT), NP, PS, wide); } while (0)
+    do { if (bulk && (PAIRS > 2 || n_rows >= HELD_ROWS))                                                               \
+             NG_LAUNCH((rope_cache_kernel<TIN, TT, 4, PAIRS, false, 1>), grid, RC_THREADS, 0, stream, RC_ARGS(TIN, TT), NP, PS, wide); \
+         else if (bulk) NG_LAUNCH((rope_cache_kernel<TIN, TT, 4, PAIRS, (PAIRS <= 2), 1>), grid, RC_THREADS, 0, stream, RC_ARGS(TIN, TT), NP, PS, wide); \
+         else if (sizeof(TIN) == 4 && (PAIRS > 1 || n_rows <= AHEAD_ROWS))                                             \
+             NG_LAUNCH((rope_cache_kernel<TIN, TT, 1, PAIRS, (PAIRS <= 2), 4>), grid, RC_THREADS, 0, stream, RC_ARGS(TIN, TT), NP, PS, wide); \
+         else NG_LAUNCH((rope_cache_kernel<TIN, TT, 1, PAIRS, (PAIRS <= 2), 1>), grid, RC_THREADS, 0, stream, RC_ARGS(TIN, TT), NP, PS, wide); } while (0)
 #define RC_GO(TIN, TT, NP, PS) RC_GO2(TIN, TT, NP, PS, NG_ROPE_PAIRS)
     if (act_bf16 && n_partials > 1) RC_GO(float, bf, n_partials, ps);
     else if (act_bf16) RC_GO(bf, bf, 1, 0);
