@@ -58,19 +58,42 @@ retention_kernel(const T* __restrict__ x, const float* __restrict__ inv_freq, in
     for (int i = dk + tid; i < dkp; i += blockDim.x) qs[i] = ks[i] = 0.f;
     ng_pdl_wait();
     x = ng_after_wait(x);
-    for (int t = 0; t < qlen; ++t) {
+    // a thread's inputs of one token: its coordinate of q and k with the coordinate it turns with, its value and gate.  The next
+    // token's are requested while this one is worked on (a token waits for memory otherwise: 8 portions of
+    // 15 tokens, 8 heads of 64 x 128 26.0 us against 27.9; float32, 300 tokens 367 against 395)
+    struct In { float q, k, qm, km, v, g; };
+    auto fetch = [&](int t, int i) {
         const T* row = x + (size_t)(q0 + t) * ld;
+        In in = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (i < dk) {
+            in.q = ng_ld(row + off_q + i);
+            in.k = ng_ld(row + off_k + i);
+            if (i < rot_dims) {
+                const int mate = i < half ? i + half : i - half;
+                in.qm = ng_ld(row + off_q + mate);
+                in.km = ng_ld(row + off_k + mate);
+            }
+        }
+        if (i == tid) {
+            in.v = live ? ng_ld(row + off_v + j) : 0.f;
+            in.g = tid < dv ? ng_ld(row + off_g + tid) : 0.f;
+        }
+        return in;
+    };
+    constexpr bool AHEAD = R < 64;                 // (larger states leave no registers)
+    In next = fetch(0, tid);
+    for (int t = 0; t < qlen; ++t) {
         const float pos = (float)(ctx + t);
-        const float vj = live ? ng_ld(row + off_v + j) : 0.f;
-        const float gate = tid < dv ? ng_ld(row + off_g + tid) : 0.f;
+        if (!AHEAD && t > 0) next = fetch(t, tid);
+        const float vj = next.v, gate = next.g;
         for (int i = tid; i < dk; i += blockDim.x) {
-            float qv = ng_ld(row + off_q + i), kv = ng_ld(row + off_k + i);
+            const In in = i == tid ? next : fetch(t, i);
+            float qv = in.q, kv = in.k;
             if (i < rot_dims) {
                 const int p = i < half ? i : i - half;
                 float sn, cs;
                 sincosf(pos * inv_freq[p], &sn, &cs);
-                const int mate = i < half ? i + half : i - half;
-                const float qm = ng_ld(row + off_q + mate), km = ng_ld(row + off_k + mate);
+                const float qm = in.qm, km = in.km;
                 // the pair (a, b) = (x[p], x[p + half]) becomes (a cos - b sin, b cos + a sin)
                 qv = i < half ? qv * cs - qm * sn : qv * cs + qm * sn;
                 kv = i < half ? kv * cs - km * sn : kv * cs + km * sn;
@@ -78,6 +101,7 @@ retention_kernel(const T* __restrict__ x, const float* __restrict__ inv_freq, in
             qs[i] = qv;
             ks[i] = kv * kscale;
         }
+        if (AHEAD && t + 1 < qlen) next = fetch(t + 1, tid);
         __syncthreads();
         if (live) {
             float acc = 0.f;
