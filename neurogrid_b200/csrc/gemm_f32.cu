@@ -235,10 +235,8 @@ static int gf_rows(const float* A, const float* W, const float* bias, float* C, 
                    int ldc, cudaStream_t stream) {
     const int pieces = (K + GR_K - 1) / GR_K, stages = pieces < GR_STAGES ? pieces : GR_STAGES;
     constexpr int STAGE = GR_COLS * GR_WROW + MR * GR_XROW, PART = 2 * GR_CH * MR * GR_COLS;
-    static bool set = false;
-    if (!set && cudaFuncSetAttribute(gemm_f32_rows_kernel<MR, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (GR_STAGES * STAGE + PART) * 4) != cudaSuccess) return NG_LAUNCH_FAILED;
-    set = true;
+    static std::atomic<unsigned long long> done{0};
+    if (!ng_allow_smem(done, gemm_f32_rows_kernel<MR, AL>, (GR_STAGES * STAGE + PART) * 4)) return NG_LAUNCH_FAILED;
     dim3 grid((N + GR_COLS - 1) / GR_COLS, (M + MR - 1) / MR);
     if (grid.y > 65535) return NG_BAD_SIZE;
     NG_LAUNCH((gemm_f32_rows_kernel<MR, AL>), grid, GR_COLS * GR_CH, (size_t)(stages * STAGE + PART) * 4, stream, A, W,
@@ -250,10 +248,8 @@ template <int BM, int BN, int TM, int TN, bool AL>
 static int gf_tile(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
                    int ldc, cudaStream_t stream) {
     constexpr int BYTES = GT_STAGES * (BM + BN) * GT_ROW * 4;
-    static bool set = false;
-    if (!set && cudaFuncSetAttribute(gemm_f32_tile_kernel<BM, BN, TM, TN, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     BYTES) != cudaSuccess) return NG_LAUNCH_FAILED;
-    set = true;
+    static std::atomic<unsigned long long> done{0};
+    if (!ng_allow_smem(done, gemm_f32_tile_kernel<BM, BN, TM, TN, AL>, BYTES)) return NG_LAUNCH_FAILED;
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return NG_BAD_SIZE;
     NG_LAUNCH((gemm_f32_tile_kernel<BM, BN, TM, TN, AL>), grid, 128, BYTES, stream, A, W, bias, C, M, N, K, lda, ldw, ldc);

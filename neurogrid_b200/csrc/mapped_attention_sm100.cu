@@ -466,13 +466,8 @@ template <int M, int DV>
 static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const Params& p, int n_entries, int max_q,
                   cudaStream_t stream) {
     constexpr int ROWS = M == 2 ? BQ : 2 * BQ;
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(mapped_attention_sm100_kernel<M, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)Cfg<M, DV>::smem()) != cudaSuccess)
-            return NG_LAUNCH_FAILED;
-        attr = true;
-    }
+    static std::atomic<unsigned long long> done{0};
+    if (!ng_allow_smem(done, mapped_attention_sm100_kernel<M, DV>, (int)Cfg<M, DV>::smem())) return NG_LAUNCH_FAILED;
     const dim3 grid(p.nH, (max_q + ROWS - 1) / ROWS, n_entries);
     if (grid.y > 65535 || grid.z > 65535) return NG_BAD_SIZE;
     const size_t smem = Cfg<M, DV>::smem();

@@ -253,12 +253,8 @@ NG_EXPORT int ng_moe_router(const void* x, const float* wr, const float* br, flo
         if (blocks > 148) blocks = 148;
 #define MRR_GO(T)                                                                                                      \
     do {                                                                                                               \
-        static bool configured = false;                                                                                \
-        if (!configured) {                                                                                             \
-            if (cudaFuncSetAttribute(moe_router_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) \
-                return NG_LAUNCH_FAILED;                                                                               \
-            configured = true;                                                                                         \
-        }                                                                                                              \
+        static std::atomic<unsigned long long> done{0};                                                                \
+        if (!ng_allow_smem(done, moe_router_rows_kernel<T>, 200 * 1024)) return NG_LAUNCH_FAILED;                      \
         NG_LAUNCH((moe_router_rows_kernel<T>), blocks, MRR_WARPS * 32, held, stream, (const T*)x, wr, br, weights, n_rows, H, E, top_k); \
         return ng_launch_status();                                                                                     \
     } while (0)

@@ -109,6 +109,14 @@ static inline void ng_launch(void (*kernel)(KP...), dim3 grid, dim3 block, size_
     cfg.numAttrs = ng_pdl_enabled() ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, KP(args)...);
 }
+// The kernel may use so much dynamic shared memory, on the device that is current (`done` is the call site's own, static).
+#include "ng_device_once.h"
+template <typename K>
+static inline bool ng_allow_smem(std::atomic<unsigned long long>& done, K kernel, int bytes) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    return ng_once_per_device(done, device, [&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; });
+}
 #define NG_LAUNCH(kernel, grid, block, smem, stream, ...) ng_launch((kernel), dim3(grid), dim3(block), (smem), (stream), __VA_ARGS__)
 
 #include <cstdio>

@@ -704,15 +704,11 @@ NG_EXPORT int ng_retention_chunked(const void* x, const float* inv_freq, int rot
     if (grid.y > 65535 || grid.z > 65535 || sgrid.y > 65535 || sgrid.z > 65535) return NG_BAD_SIZE;
     // 16-byte accesses to rows of the activation type and to the chunks' states
     if (dk == R1_D && dv == R1_D && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)u_scratch) & 15) == 0) {
-        static bool set[2] = {false, false};
+        static std::atomic<unsigned long long> done[2];
         dim3 hgrid(n_entries, grid.y, nH);
 #define R1_GO(T)                                                                                                       \
     do {                                                                                                               \
-        if (!set[which]) {                                                                                             \
-            if (cudaFuncSetAttribute(retention_out128_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, R1_OUT_SMEM) != cudaSuccess) \
-                return NG_LAUNCH_FAILED;                                                                               \
-            set[which] = true;                                                                                         \
-        }                                                                                                              \
+        if (!ng_allow_smem(done[which], retention_out128_kernel<T>, R1_OUT_SMEM)) return NG_LAUNCH_FAILED;             \
         NG_LAUNCH((retention_local128_kernel<T>), hgrid, R1_THREADS, 0, stream, (const T*)x, inv_freq, decay, u_scratch, cu_q, \
                   ctx_before, nH, rot_dims);                                                                           \
         NG_LAUNCH((retention_scan_kernel), sgrid, 256, 0, stream, u_scratch, state, decay, cu_q, ctx_before, slots, nH, dk, dv); \
