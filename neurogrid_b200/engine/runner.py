@@ -627,7 +627,7 @@ class ModelRunner:
             bits |= ops.gemm_status(self.device)
         if bits:
             self.status.zero_()
-            raise StepError(f"a kernel reported status bits {bits:#x} (1 bad token, 2 bad page, 4 bad position, 8 a bounded wait of the tensor-core product ran out)")
+            raise StepError(f"a kernel reported status bits {bits:#x} (1 bad token, 2 bad page, 4 bad position, 8 a bounded wait of the tensor-core product ran out, 16 one of the tensor-core attention)")
 
     def graph_kernel_nodes(self) -> Dict[tuple, int]:
         """Kernel nodes of every captured graph, asked from the CUDA runtime (``keep_graphs`` must

@@ -9,6 +9,7 @@ import kernel_refs
 import plain_lfm2
 from helpers import make_runner, rel_err, run_cuts
 from neurogrid_b200.engine import StepEntry
+from neurogrid_b200.engine.runner import StepError
 from tiny_configs import PAGE_SIZE, TINY
 
 
@@ -31,6 +32,15 @@ def test_whole_prompt_matches_plain(model_dirs, name):
         got = run_cuts(runner, "r", toks, [T])
         assert rel_err(got, plain_lfm2.forward(cfg, w, toks)) < 2e-5
     runner.cache.check()
+
+
+def test_status_names_the_attention_kernels_timeout(model_dirs):
+    """What the attention kernels report when a bounded wait runs out (16) is named beside the other bits."""
+    runner = make_runner(model_dirs["A"], page_size=PAGE_SIZE["A"])
+    runner.status.fill_(16)
+    with pytest.raises(StepError, match="0x10 .*16 .*attention"):
+        runner.check_status()
+    runner.check_status()
 
 
 @pytest.mark.parametrize("name", ["A", "B", "C", "D"])
