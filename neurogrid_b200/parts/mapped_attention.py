@@ -37,7 +37,10 @@ class MappedAttention:
     GROUP_MAX_ROWS = 256   # decode-only steps of up to this many rows run the heads of a KV group as a tensor-core tile
     GROUP_MAX_RUNS = 512   # ... with rows * runs a row bounded by this
     GROUP_LONG_KEYS = 3072 # ... rows that may see so many keys may have their runs merged by a second launch
-    TILE_MIN_ROWS = 64     # steps with a portion of at least this many rows (half a tile of the tcgen05 kernel) run on it
+    # steps with a portion of at least this many rows (half a tile of the tcgen05 kernel) run on it, single tokens beside it too, and
+    # padded mixed steps, whose longest portion counts as all of their rows: it was the faster one in every mix tried (heads of 64, one
+    # map: 63 single tokens beside 64 rows behind 500 tokens 104 us against 141; 15 beside 48 behind 2,000 85 against 187)
+    TILE_MIN_ROWS = 64
     SPLIT_MAX_ROWS = 32    # steps of up to this many rows may cut each row's keys into runs
     SPLIT_MIN_KEYS = 128   # ... of at least this many keys (one tile of the kernel)
     MAX_SPLITS = 16
@@ -141,7 +144,8 @@ class MappedAttention:
     def _plain_scores(self):
         """Softmax over scores without a bias per head, sinks, chunks or a gate per head: what the tcgen05 kernel forms."""
         s = self.spec
-        return not self.sigmoid and not getattr(s, "sinks", False) and not getattr(s, "chunk", None) and not getattr(s, "head_gate", False)
+        return not self.sigmoid and not getattr(s, "sink", False) and not getattr(s, "unit_sink", False) and \
+            not getattr(s, "chunk", None) and not getattr(s, "head_gate", False)
 
     def scratch_bytes_per_row(self):
         s = self.spec

@@ -16,6 +16,17 @@ from neurogrid_b200.engine import StepEntry
 from neurogrid_b200.models import declare_tensors
 
 
+@pytest.mark.parametrize("kw,tiles", [({}, True), (dict(window=100, keep_first=3, softcap=9.0), True), (dict(sink=True), False),
+                                      (dict(unit_sink=True), False), (dict(weights="sigmoid"), False), (dict(head_gate=True), False)])
+def test_only_plain_scores_ask_for_the_tile_kernel(kw, tiles):
+    """A layer whose scores the tcgen05 kernel does not form does not have it built: sinks, sigmoid weights, a gate per head."""
+    from neurogrid_b200.config import MappedAttentionSpec, NoPositionSpec
+    from neurogrid_b200.parts import build
+    spec = MappedAttentionSpec(hidden=64, n_heads=4, n_kv_heads=2, key_dim=64, value_dim=64, position=NoPositionSpec(), softmax_scale=0.1, **kw)
+    part = build("mixer", spec, dtype=torch.bfloat16, device="cpu")
+    assert ("mapped_attention_sm100" in [name for name, _ in part.kernels()]) == tiles
+
+
 def test_spec_and_declared_tensors():
     spec = config_from_dict(rm.ROFU_S).model_spec()
     assert spec.architecture == "Rofulorn" and spec.embed_scale == 1.7 and spec.vocab_size == 157
