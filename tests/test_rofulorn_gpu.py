@@ -1,6 +1,7 @@
 """Rofulorn on the GPU against the plain implementation: each mechanism alone, then whole models under every way of
 cutting the work, then generation through the engine's own entry point and the replay program."""
 import json
+import math
 import os
 import subprocess
 import sys
@@ -322,6 +323,64 @@ def test_what_no_row_sees_stays_out(kernel, M, H, G, vdim, window, keep, softcap
         got.append(out)
         _poison(kp, vp, table, lens, befores, window, keep)
     assert int(ctx.status) == 0 and bool(torch.isfinite(got[0].float()).all()) and torch.equal(got[0], got[1])
+
+
+def _cancelling(M, vdim, lam, seed):
+    """Scores (base 2) of four keys and values whose weighted sum almost cancels: (scores [M, 4], values [4, vdim], the exact sum, the sum
+    of the sizes of its terms, how far a sum whose weights are two bfloat16 terms each is off at most, relative to the latter)."""
+    bf = lambda x: x.to(torch.bfloat16).to(x.dtype)  # noqa: E731
+    g = torch.Generator().manual_seed(seed)
+    scores = torch.tensor([0.0, 4.0, 13.0, 13.0]) + torch.randint(0, 64, (M, 4), generator=g) / 64
+    e = 2.0 ** (scores - scores.amax(-1, keepdim=True)).double()
+    signs = torch.tensor([1.0, -lam], dtype=torch.float64)[:M, None] / e.sum(-1, keepdim=True)
+    w, v = (signs * e).sum(0), torch.zeros(4, vdim, dtype=torch.float64)
+    for j in (0, 1):
+        v[j] = bf(0.3 * (1 + torch.rand(vdim, generator=g)).double() / w[j].abs())
+    for j in (2, 3):
+        v[j] = bf(-(w[:j, None] * v[:j]).sum(0) / w[j])
+    want, size = (w[:, None] * v).sum(0), ((signs * e).abs().sum(0)[:, None] * v.abs()).sum(0)
+    two = bf(e) + bf(e - bf(e))
+    miss = ((signs * two).sum(0)[:, None] * v).sum(0) - want
+    return scores, v, want, size, float((miss.abs() / size).max())
+
+
+@pytest.mark.parametrize("kernel", ["tcgen05", "tiles", "cluster", "second launch"])
+@pytest.mark.parametrize("M,vdim", [(1, 64), (1, 128), (2, 64), (2, 128)])
+def test_weights_enter_as_three_terms(kernel, M, vdim):
+    """Four keys in three tiles, in scores that rise by more than 2^8 (the reference point moves and O is rescaled), with values
+    whose weighted sum is 2^-17 of its terms: what is left of the weights shows whole.  The bound is what float32 weights (the
+    exponential to 2 units of the last place) and sums of a few terms leave; two bfloat16 terms a weight miss it threefold and
+    more, one term a thousandfold."""
+    d, ps, T, lam, H, G = 64, 16, 300, 0.5, 2, 1
+    scores, v4, want, size, miss = _cancelling(M, vdim, lam, 41)
+    bound = 2.0 ** -20.3
+    assert miss > 3 * bound
+    k, v, q = torch.zeros(T, G * M, d), torch.zeros(T, G, vdim), torch.zeros(T, H, M, d)
+    k[:, :, 0], q[..., :3] = -64.0, 1.0
+    for i, j in enumerate((5, 70, 140, 141)):
+        k[j, :, 0], k[j, :, 1], k[j, :, 2] = 0.0, scores[:, i].floor(), scores[:, i] - scores[:, i].floor()
+        v[j, 0] = v4[i].float()
+    n_pages = -(-T // ps)
+    perm = torch.randperm(n_pages, generator=torch.Generator().manual_seed(1))
+    kp, vp = torch.zeros(n_pages, G * M, ps, d), torch.zeros(n_pages, G, ps, vdim)
+    for t in range(T):
+        kp[perm[t // ps], :, t % ps], vp[perm[t // ps], :, t % ps] = k[t], v[t]
+    b = lambda t: t.to(torch.bfloat16).to(DEV)  # noqa: E731
+    args = (H, M, None, 0, math.log(2.0), 0.0, lam, False, 1.0, 1e-5)
+    if kernel in ("tcgen05", "tiles"):
+        ctx, rows = make_ctx([T], [0], [0], dtype=torch.bfloat16), list(range(150, T))
+        out = torch.empty(T, H * vdim, dtype=torch.bfloat16, device=DEV)
+        call = (b(q.reshape(T, -1)), b(kp), b(vp), perm.to(torch.int32)[None].contiguous().to(DEV), ctx.cu_q, ctx.ctx_before, out, 1, T) + args
+        ops().mapped_attention_sm100(*call, ctx.status) if kernel == "tcgen05" else ops().mapped_attention_mma(*call)
+    else:
+        at = [141, 142, 200, 299]
+        ctx, rows = make_ctx([1] * 4, at, list(range(4)), dtype=torch.bfloat16), list(range(4))
+        out = torch.empty(4, H * vdim, dtype=torch.bfloat16, device=DEV)
+        partial = torch.empty(4 * H * 4 * M * (vdim + 2), device=DEV) if kernel == "second launch" else None
+        ops().mapped_attention_group(b(q[:4].reshape(4, -1)), b(kp), b(vp), perm.to(torch.int32)[None].repeat(4, 1).to(DEV), ctx.cu_q, ctx.ctx_before,
+                                     ctx.row_entry, out, partial, 4, *args, 4)
+    assert int(ctx.status) == 0
+    assert float(((out.view(-1, H, vdim)[rows].double().cpu() - want).abs() / size).max()) < bound
 
 
 def test_tensor_core_kernel_with_several_entries_in_a_step():
