@@ -164,3 +164,16 @@ def test_float32_follows_plain_at_real_sizes(runners, plain_weights):
     got = _run(runners[torch.float32], {"a": toks}, lambda n: [n], 6)["a"]
     want = plain_lfm2.forward(CFG, plain_weights, toks, rows=list(range(290 - 7, 290)))
     assert rel_err(got, want) < 1e-4, rel_err(got, want)
+
+
+@pytest.mark.parametrize("n", [65, 100, 128, 300])
+def test_prompts_of_more_than_64_tokens_repeat_bit_for_bit(runners, n):
+    """Steps of up to 64 rows add products into the residual stream in an order that is not fixed; longer ones do not: the same
+    prompt gives the same logits every time, from the eager step, the captured one and its replays."""
+    runner, toks, first = runners[torch.bfloat16], _tokens(n, 40 + n), None
+    for k in range(6):
+        got = runner.step([StepEntry("p", toks, sorted({*range(0, n, 9), n - 1}))]).clone()
+        runner.finish("p")
+        first = got if first is None else first
+        assert torch.equal(got, first), k
+    runner.check_status()
