@@ -2,19 +2,42 @@
 //
 // FFMA only: no tensor cores, no TF32.  The order of the additions depends on K alone: k is cut into chunks of 64; a
 // chunk has two sums, of its even and of its odd k, each in ascending order (the two halves of one packed FMA), which
-// are added; the chunks' sums are added in ascending order.  Both kernels below form exactly that, so a row's result
-// does not depend on M, on the other rows of the batch or on where the row sits in it, and shorter chains of
-// additions are a little nearer to 64 bits than one chain over k.  The reference calls cuBLAS for every contraction
+// are added; the sums of 16 chunks are added in ascending order to a group's, the groups' sums likewise.  Both kernels
+// below form exactly that, so a row's result does not depend on M, on the other rows of the batch or on where the row
+// sits in it, and shorter chains of additions are a little nearer to 64 bits than one chain over k.  The groups of a
+// long K (2 to 8 of them) are the blocks of a cluster, which add their sums through shared memory in that order.  The reference calls cuBLAS for every contraction
 // (gpu/cuda/matmul.cu:316-355) and has no float32 path.
 //
 // Few rows (single tokens) are bound by the weights' bytes: `gemm_f32_rows_kernel`.  More rows are bound by the FMA
 // pipe: `gemm_f32_tile_kernel`.  Measured on the 350M LFM2 shape, two prompts of 96 tokens and 8 decode steps, where
 // one kernel of 64 x 64 tiles (4 x 4 elements a thread, synchronous loads) took 109 ms of the pass: the products of
-// the decode steps now take 3.8 ms (7.4 us each, the weights at 3.0 TB/s), those of the prompts' step of 256 padded
-// rows 6.3 ms (gate/up, 256 x 9216 x 1024: 138 us, 35 of 74 TFLOP/s).
+// the decode steps took 3.8 ms, those of the prompts' step of 256 padded rows 6.3 ms; with the groups of a long K side
+// by side and 192 rows the pass takes 10.7 ms instead of 13.0 (192 x 1024 x 4608: 75 us instead of 223; 2 rows: 6.2
+// instead of 10.8; 192 x 9216 x 1024: 107 us, 34 of 74 TFLOP/s).
 #include "ng_common.cuh"
 
 #define GF_CHUNK 64
+#define GF_GROUP (16 * GF_CHUNK)                 // k of a group
+// Few rows: the groups are a cluster's blocks where the launch has no more blocks than this without (1 / 2 / 8 rows, us: 1,024 x
+// 4,608 5.6 / 6.2 / 12.9 against 8.3 / 10.8 / 16.4 in one block; 2,048 x 8,192 17.5 / 19.6 / 37.8 against 17.3 / 35.4 / 53.7)
+#define GF_ROWS_FEW 600
+#define GF_MAX_CLUSTER 8                         // groups that are blocks of a cluster; a longer K walks its groups in one block
+
+__device__ __forceinline__ uint32_t gf_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void gf_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the float at `p` of this block's shared memory, in block `rank` of the cluster
+__device__ __forceinline__ float gf_peer(const float* p, int rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    float v;
+    asm volatile("{\n\t.reg .u32 r;\n\tmapa.shared::cluster.u32 r, %1, %2;\n\tld.shared::cluster.f32 %0, [r];\n\t}" : "=f"(v) : "r"(a), "r"(rank) : "memory");
+    return v;
+}
 
 __device__ __forceinline__ uint64_t gf_fma2(uint64_t a, uint64_t b, uint64_t c) {
     uint64_t d;
@@ -48,16 +71,17 @@ __device__ __forceinline__ void gf_wait() { asm volatile("cp.async.wait_group %0
 // ---- few rows --------------------------------------------------------------------------------------------------
 // A block owns 8 columns (weight rows) and up to MR rows of A and walks k in pieces of 16 chunks.  A thread owns one
 // column and one chunk of the piece for all MR rows; the 16 chunk sums of a (row, column) are then added in order by
-// one thread.  Eight columns a block keep 128 blocks busy at N = 1,024; the pieces' copies (33 KB of weights) run
-// GR_STAGES deep, and the first weights are requested before the kernel in front has ended.
+// one thread: a group's sum.  Eight columns a block keep 128 blocks busy at N = 1,024, and a cluster's blocks share the
+// pieces of a long K; otherwise the pieces' copies (33 KB of weights) run GR_STAGES deep.  The first weights are
+// requested before the kernel in front has ended.
 #define GR_COLS 8
 #define GR_CH 16
-#define GR_K (GR_CH * GF_CHUNK)
+#define GR_K GF_GROUP                            // a piece is a group
 #define GR_WROW (GR_K + 4)                       // 4 mod 32 words: eight columns read 16 bytes each without conflicts
 #define GR_XROW (GR_CH * (GF_CHUNK + 4))         // chunks 68 words apart: the four chunks a warp reads lie in other banks
 #define GR_STAGES 3
 
-template <int MR, bool AL>
+template <int MR, bool AL, bool CLUSTER>
 __global__ void __launch_bounds__(GR_COLS* GR_CH)
 gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                      float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int stages) {
@@ -66,12 +90,13 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, c
     float* part = gr_smem + (size_t)stages * STAGE;                // [2][chunk][MR * GR_COLS]
     const int tid = threadIdx.x, col = tid % GR_COLS, ch = tid / GR_COLS;
     const int n0 = blockIdx.x * GR_COLS, m0 = blockIdx.y * MR;
-    const int pieces = (K + GR_K - 1) / GR_K;
+    const int rank = CLUSTER ? gf_rank() : 0;                      // (the cluster's blocks are those of blockIdx.z)
+    const int pieces = CLUSTER ? 1 : (K + GR_K - 1) / GR_K;        // this block's: in a cluster the one of its rank
     ng_pdl_trigger();
 
     auto load_w = [&](int p) {
         float* s = gr_smem + (size_t)(p % stages) * STAGE;
-        const int k0 = p * GR_K;
+        const int k0 = (rank + p) * GR_K;
         for (int i = tid; i < GR_COLS * (GR_K / 4); i += GR_COLS * GR_CH) {
             const int r = i / (GR_K / 4), k = (i % (GR_K / 4)) * 4;
             if (k0 + k >= ((K + GF_CHUNK - 1) / GF_CHUNK) * GF_CHUNK) continue;
@@ -81,7 +106,7 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, c
     };
     auto load_x = [&](int p, const float* a) {
         float* s = gr_smem + (size_t)(p % stages) * STAGE + GR_COLS * GR_WROW;
-        const int k0 = p * GR_K;
+        const int k0 = (rank + p) * GR_K;
         for (int i = tid; i < MR * (GR_K / 4); i += GR_COLS * GR_CH) {
             const int r = i / (GR_K / 4), k = (i % (GR_K / 4)) * 4;
             if (k0 + k >= ((K + GF_CHUNK - 1) / GF_CHUNK) * GF_CHUNK) continue;
@@ -104,7 +129,7 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, c
         gf_wait<GR_STAGES - 1>();
         __syncthreads();
         const float* s = gr_smem + (size_t)(p % stages) * STAGE;
-        const int chunks = min(GR_CH, (K - p * GR_K + GF_CHUNK - 1) / GF_CHUNK);
+        const int chunks = min(GR_CH, (K - (rank + p) * GR_K + GF_CHUNK - 1) / GF_CHUNK);
         float* pp = part + (p & 1) * GR_CH * MR * GR_COLS;
         if (ch < chunks) {
             uint64_t acc[MR];
@@ -130,8 +155,21 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, c
             load_x(p + stages, a);
         }
         gf_commit();
-        if (tid < MR * GR_COLS)
-            for (int c = 0; c < chunks; ++c) total += pp[c * MR * GR_COLS + tid];
+        if (tid < MR * GR_COLS) {
+            float group = 0.f;
+            for (int c = 0; c < chunks; ++c) group += pp[c * MR * GR_COLS + tid];
+            total += group;
+        }
+    }
+    if constexpr (CLUSTER) {
+        if (tid < MR * GR_COLS) part[GR_CH * MR * GR_COLS + tid] = total;        // (the half that was not used)
+        gf_cluster_sync();
+        if (rank == 0 && tid < MR * GR_COLS) {
+            total = 0.f;
+            for (int r = 0; r < (int)gridDim.z; ++r) total += gf_peer(part + GR_CH * MR * GR_COLS + tid, r);
+        }
+        gf_cluster_sync();                                       // a block's shared memory is there until it has been read
+        if (rank != 0) return;
     }
     const int m = m0 + tid / GR_COLS, n = n0 + col;
     if (tid < MR * GR_COLS && m < M && n < N) C[(size_t)m * ldc + n] = total + (bias ? bias[n] : 0.f);
@@ -144,7 +182,8 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, c
 #define GT_ROW (GT_BK + 4)
 #define GT_STAGES 4
 
-template <int BM, int BN, int TM, int TN, bool AL>
+// GROUPS: K is one group (0), the groups of this block's walk one after the other (1), or the blocks of a cluster (2).
+template <int BM, int BN, int TM, int TN, bool AL, int GROUPS>
 __global__ void __launch_bounds__(128)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                      float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc) {
@@ -154,14 +193,16 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
     const int tid = threadIdx.x, tr = tid % TR, tc = tid / TR;
     const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
     // the order of the sums has whole chunks: an odd number of stages ends with one of zeros
-    const int stages = 2 * ((K + GF_CHUNK - 1) / GF_CHUNK);
+    const int rank = GROUPS == 2 ? gf_rank() : 0, kbase = rank * GF_GROUP;
+    const int klen = GROUPS == 2 ? min(K - kbase, GF_GROUP) : K;
+    const int stages = 2 * ((klen + GF_CHUNK - 1) / GF_CHUNK);
     ng_pdl_trigger();
 
     auto load_w = [&](int t) {
         float* s = gt_smem + (t % GT_STAGES) * STAGE + BM * GT_ROW;
 #pragma unroll
         for (int i = tid; i < BN * (GT_BK / 4); i += 128) {
-            const int r = i / (GT_BK / 4), k = (i % (GT_BK / 4)) * 4, kk = t * GT_BK + k;
+            const int r = i / (GT_BK / 4), k = (i % (GT_BK / 4)) * 4, kk = kbase + t * GT_BK + k;
             const int have = n0 + r < N ? K - kk : 0;
             gf_copy4<AL>(s + r * GT_ROW + k, have > 0 ? W + (size_t)(n0 + r) * ldw + kk : W, have);
         }
@@ -170,7 +211,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
         float* s = gt_smem + (t % GT_STAGES) * STAGE;
 #pragma unroll
         for (int i = tid; i < BM * (GT_BK / 4); i += 128) {
-            const int r = i / (GT_BK / 4), k = (i % (GT_BK / 4)) * 4, kk = t * GT_BK + k;
+            const int r = i / (GT_BK / 4), k = (i % (GT_BK / 4)) * 4, kk = kbase + t * GT_BK + k;
             const int have = m0 + r < M ? K - kk : 0;
             gf_copy4<AL>(s + r * GT_ROW + k, have > 0 ? a + (size_t)(m0 + r) * lda + kk : a, have);
         }
@@ -183,11 +224,14 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
         gf_commit();
     }
     uint64_t acc[TM][TN];
-    float total[TM][TN];
+    float total[TM][TN], before[GROUPS == 1 ? TM : 1][GROUPS == 1 ? TN : 1];     // of the group, of the groups before it
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0ull, total[i][j] = 0.f;
+        for (int j = 0; j < TN; ++j) {
+            acc[i][j] = 0ull, total[i][j] = 0.f;
+            if constexpr (GROUPS == 1) before[i][j] = 0.f;
+        }
 
     for (int t = 0; t < stages; ++t) {
         gf_wait<GT_STAGES - 2>();
@@ -216,7 +260,41 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) total[i][j] += gf_both(acc[i][j]), acc[i][j] = 0ull;
+            if constexpr (GROUPS == 1)
+                if ((t + 1) % (GF_GROUP / GT_BK) == 0 || t + 1 == stages)        // a group's end
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+#pragma unroll
+                        for (int j = 0; j < TN; ++j) before[i][j] += total[i][j], total[i][j] = 0.f;
         }
+    }
+    if constexpr (GROUPS == 1)
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) total[i][j] = before[i][j];
+    if constexpr (GROUPS == 2) {                                 // the blocks of a cluster: each adds up some rows of the tile
+        static_assert(BM * BN <= GT_STAGES * STAGE, "the tile's sums fit where the stages were");
+        __syncthreads();                                         // every stage has been read
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) gt_smem[(tr + i * TR) * BN + tc + j * TC] = total[i][j];
+        gf_cluster_sync();
+        const int blocks = gridDim.z;
+        for (int e = tid; e < ((BM - rank + blocks - 1) / blocks) * BN; e += 128) {
+            const int r = rank + e / BN * blocks, c = e % BN, m = m0 + r, n = n0 + c;
+            if (m >= M || n >= N) continue;
+            float v[GF_MAX_CLUSTER], sum = 0.f;
+#pragma unroll
+            for (int b = 0; b < GF_MAX_CLUSTER; ++b) v[b] = b < blocks ? gf_peer(gt_smem + r * BN + c, b) : 0.f;
+#pragma unroll
+            for (int b = 0; b < GF_MAX_CLUSTER; ++b)
+                if (b < blocks) sum += v[b];
+            C[(size_t)m * ldc + n] = sum + (bias ? bias[n] : 0.f);
+        }
+        gf_cluster_sync();
+        return;
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
@@ -230,30 +308,73 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
     }
 }
 
+// as ng_launch, the blocks of one (x, y) as a cluster
+template <typename... KP, typename... A>
+static int gf_launch_cluster(void (*kernel)(KP...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    memset(attr, 0, sizeof(attr));
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = grid.z;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ng_pdl_enabled() ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, KP(args)...);
+    return ng_launch_status();
+}
+static inline int gf_groups(int K) { return (K + GF_GROUP - 1) / GF_GROUP; }
+
+template <int MR, bool AL, bool CLUSTER>
+static int gf_rows_as(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
+                      int ldc, cudaStream_t stream) {
+    const int groups = gf_groups(K), stages = CLUSTER ? 1 : groups < GR_STAGES ? groups : GR_STAGES;
+    constexpr int STAGE = GR_COLS * GR_WROW + MR * GR_XROW, PART = 2 * GR_CH * MR * GR_COLS;
+    static std::atomic<unsigned long long> done{0};
+    if (!ng_allow_smem(done, gemm_f32_rows_kernel<MR, AL, CLUSTER>, (GR_STAGES * STAGE + PART) * 4)) return NG_LAUNCH_FAILED;
+    dim3 grid((N + GR_COLS - 1) / GR_COLS, (M + MR - 1) / MR, CLUSTER ? groups : 1);
+    if (grid.y > 65535) return NG_BAD_SIZE;
+    const size_t smem = (size_t)(stages * STAGE + PART) * 4;
+    if (CLUSTER) return gf_launch_cluster(gemm_f32_rows_kernel<MR, AL, CLUSTER>, grid, GR_COLS * GR_CH, smem, stream, A, W, bias, C, M, N, K, lda, ldw, ldc, stages);
+    NG_LAUNCH((gemm_f32_rows_kernel<MR, AL, CLUSTER>), grid, GR_COLS * GR_CH, smem, stream, A, W, bias, C, M, N, K, lda, ldw, ldc, stages);
+    return ng_launch_status();
+}
 template <int MR, bool AL>
 static int gf_rows(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
                    int ldc, cudaStream_t stream) {
-    const int pieces = (K + GR_K - 1) / GR_K, stages = pieces < GR_STAGES ? pieces : GR_STAGES;
-    constexpr int STAGE = GR_COLS * GR_WROW + MR * GR_XROW, PART = 2 * GR_CH * MR * GR_COLS;
-    static std::atomic<unsigned long long> done{0};
-    if (!ng_allow_smem(done, gemm_f32_rows_kernel<MR, AL>, (GR_STAGES * STAGE + PART) * 4)) return NG_LAUNCH_FAILED;
-    dim3 grid((N + GR_COLS - 1) / GR_COLS, (M + MR - 1) / MR);
-    if (grid.y > 65535) return NG_BAD_SIZE;
-    NG_LAUNCH((gemm_f32_rows_kernel<MR, AL>), grid, GR_COLS * GR_CH, (size_t)(stages * STAGE + PART) * 4, stream, A, W,
-              bias, C, M, N, K, lda, ldw, ldc, stages);
-    return ng_launch_status();
+    // a cluster where the blocks alone are few: GF_ROWS_FEW
+    const int groups = gf_groups(K);
+    const long long blocks = (long long)((N + GR_COLS - 1) / GR_COLS) * ((M + MR - 1) / MR);
+    if (groups > 1 && groups <= GF_MAX_CLUSTER && blocks <= GF_ROWS_FEW)
+        return gf_rows_as<MR, AL, true>(A, W, bias, C, M, N, K, lda, ldw, ldc, stream);
+    return gf_rows_as<MR, AL, false>(A, W, bias, C, M, N, K, lda, ldw, ldc, stream);
 }
 
-template <int BM, int BN, int TM, int TN, bool AL>
-static int gf_tile(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
-                   int ldc, cudaStream_t stream) {
+template <int BM, int BN, int TM, int TN, bool AL, int GROUPS>
+static int gf_tile_as(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
+                      int ldc, cudaStream_t stream) {
     constexpr int BYTES = GT_STAGES * (BM + BN) * GT_ROW * 4;
     static std::atomic<unsigned long long> done{0};
-    if (!ng_allow_smem(done, gemm_f32_tile_kernel<BM, BN, TM, TN, AL>, BYTES)) return NG_LAUNCH_FAILED;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+    if (!ng_allow_smem(done, gemm_f32_tile_kernel<BM, BN, TM, TN, AL, GROUPS>, BYTES)) return NG_LAUNCH_FAILED;
+    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, GROUPS == 2 ? gf_groups(K) : 1);
     if (grid.y > 65535) return NG_BAD_SIZE;
-    NG_LAUNCH((gemm_f32_tile_kernel<BM, BN, TM, TN, AL>), grid, 128, BYTES, stream, A, W, bias, C, M, N, K, lda, ldw, ldc);
+    if (GROUPS == 2) return gf_launch_cluster(gemm_f32_tile_kernel<BM, BN, TM, TN, AL, GROUPS>, grid, 128, BYTES, stream, A, W, bias, C, M, N, K, lda, ldw, ldc);
+    NG_LAUNCH((gemm_f32_tile_kernel<BM, BN, TM, TN, AL, GROUPS>), grid, 128, BYTES, stream, A, W, bias, C, M, N, K, lda, ldw, ldc);
     return ng_launch_status();
+}
+template <int BM, int BN, int TM, int TN, bool AL>
+static int gf_tile(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
+                   int ldc, cudaStream_t s) {
+    const int groups = gf_groups(K);
+    if (groups == 1) return gf_tile_as<BM, BN, TM, TN, AL, 0>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+    if (groups <= GF_MAX_CLUSTER) return gf_tile_as<BM, BN, TM, TN, AL, 2>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+    return gf_tile_as<BM, BN, TM, TN, AL, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
 }
 
 // Rows up to which the few-rows kernel takes the product: it reads the weights once per 8 rows (from the L2 after the
@@ -269,9 +390,12 @@ static int gf_dispatch(const float* A, const float* W, const float* bias, float*
         if (M <= 4) return gf_rows<4, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
         return gf_rows<8, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
     }
-    auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
+    const int split = gf_groups(K) <= GF_MAX_CLUSTER ? gf_groups(K) : 1;
+    auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn) * split; };
+    // 192 and 256 rows, us: 9,216 x 1,024 106.8 / 136.8 with 64 x 64 tiles (106.2 / 139.6 with 32 x 64); 3,072 x 1,024 67.5 / 69.9
+    // (58.8 / 71.7); 1,024 x 1,024 34.5 / 48.4 with 32 x 64 (96 and 128 blocks), 50.8 / 61.4 with 32 x 32
     if (blocks(64, 64) >= 2 * 148) return gf_tile<64, 64, 8, 4, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
-    if (blocks(32, 64) >= 148) return gf_tile<32, 64, 4, 4, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+    if (blocks(32, 64) >= 64) return gf_tile<32, 64, 4, 4, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
     return gf_tile<32, 32, 4, 2, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
 }
 

@@ -107,6 +107,23 @@ def test_gemm_f32_one_order(M, N, K):
         assert torch.equal(part, out[M - min(n, M):]), n
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 24, 1025), (8, 4801, 2048), (2, 9, 8192), (5, 17, 9000), (33, 40, 1100), (64, 2300, 4608),
+                                   (192, 4700, 2050), (70, 65, 8193), (200, 130, 3073)])
+def test_gemm_f32_groups(M, N, K):
+    """K of more than one group: the blocks of a cluster, or (more than eight groups) one block, in one order.  The bound: a
+    chunk's products and sums, then the additions of 16 chunks and of the groups, 2^-24 each."""
+    a, w, b = rnd(M, K, seed=1), rnd(N, K, seed=2), rnd(N, seed=3)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    ops().gemm_f32(a, w, b, out)
+    want = a.double() @ w.double().T + b.double()
+    size = a.double().abs() @ w.double().abs().T + b.double().abs()
+    assert bool(((out.double() - want).abs() <= (64 + 16 + -(-K // 1024) + 3) * 2.0 ** -24 * size).all())
+    for n in sorted({1, min(M, 8), min(M, 40)}):
+        part = torch.empty(n, N, device=DEV)
+        ops().gemm_f32(a[M - n:].contiguous(), w, b, part)
+        assert torch.equal(part, out[M - n:]), n
+
+
 def _ragged(q_lens, ctx):
     cu = [0]
     for q in q_lens:
