@@ -135,7 +135,7 @@ mapped_attention_mma_kernel(const MmaParams p) {
     bf16* Vs = Ks + 2 * M * KT * KP;                                     // [2][KT][VP]
     float* Os = reinterpret_cast<float*>(Ks);                            // epilogue: [M][ROWS][DV], over the tiles
     __shared__ int kpos_s[3][KT];                                        // per tile in flight or in use (three: see the loop)
-    __shared__ long long koff_s[3][KT];
+    __shared__ int page_s[3][KT], slot_s[3][KT];                         // a key's page (-1: none) and its place in it
     __shared__ int tile_bad_s[3][2];                                     // a key of the tile has no page
     __shared__ float part_m[WARPS][16], part_l[WARPS][16];               // GROUP: the warps' states per row
     ng_pdl_trigger();
@@ -204,21 +204,24 @@ mapped_attention_mma_kernel(const MmaParams p) {
     const int* trow = p.table + (size_t)entry * p.table_stride;
 
     // Two buffers: while the warps work on a tile, the next one is on its way (cp.async, 16 bytes a copy; a key that
-    // is not there is filled with zeros).  A tile's page slots are looked up one iteration ahead of its copies.
+    // is not there is filled with zeros).  A tile's page slots are looked up one iteration ahead of its copies, once a key; a
+    // division by the page size in front of every copy was a microsecond a launch (8 rows behind 512 tokens, 16 layers, a decode
+    // step: 560 -> 545 us).
     auto lookup = [&](int t0, int b) {
         if (tid < KT) {
             const int t = t0 + tid;
-            int kpos = -1;
-            long long off = -1;
+            int kpos = -1, page = -1, slot = 0;
             if (t < n_keys) {
                 kpos = t < n_sink ? t : lo + (t - n_sink);
-                const int page = trow[kpos / p.page_size];
-                if (page >= 0 && page < p.num_pages) off = (long long)page * p.page_size + (kpos % p.page_size);
-                else kpos = -1;
+                const int at = kpos / p.page_size;
+                page = trow[at];
+                slot = kpos - at * p.page_size;
+                if (page < 0 || page >= p.num_pages) page = kpos = -1;
             }
             kpos_s[b][tid] = kpos;
-            koff_s[b][tid] = off;
-            const unsigned bad = __ballot_sync(0xffffffffu, t < n_keys && off < 0);      // KT = 64: warps 0 and 1, whole
+            page_s[b][tid] = page;
+            slot_s[b][tid] = slot;
+            const unsigned bad = __ballot_sync(0xffffffffu, t < n_keys && page < 0);     // KT = 64: warps 0 and 1, whole
             if (lane == 0) tile_bad_s[b][warp] = bad != 0u;
         }
     };
@@ -227,17 +230,15 @@ mapped_attention_mma_kernel(const MmaParams p) {
         bf16* vb = Vs + (size_t)b * KT * VP;
         for (int i = tid; i < M * KT * (D / 8); i += THREADS) {
             const int ch = i % (D / 8), key = (i / (D / 8)) % KT, m = i / ((D / 8) * KT);
-            const long long off = koff_s[mb][key];
-            const long long page = off >= 0 ? off / p.page_size : 0, slot = off >= 0 ? off % p.page_size : 0;
+            const int page = max(page_s[mb][key], 0), slot = slot_s[mb][key];
             cp_async16(kb + ((size_t)m * KT + key) * KP + ch * 8,
-                       p.k_pages + (((size_t)page * p.nG * M + (size_t)g * M + m) * p.page_size + slot) * D + ch * 8, off >= 0);
+                       p.k_pages + (((size_t)page * p.nG * M + (size_t)g * M + m) * p.page_size + slot) * D + ch * 8, page_s[mb][key] >= 0);
         }
         for (int i = tid; i < KT * (DV / 8); i += THREADS) {
             const int ch = i % (DV / 8), key = i / (DV / 8);
-            const long long off = koff_s[mb][key];
-            const long long page = off >= 0 ? off / p.page_size : 0, slot = off >= 0 ? off % p.page_size : 0;
+            const int page = max(page_s[mb][key], 0), slot = slot_s[mb][key];
             cp_async16(vb + (size_t)key * VP + ch * 8,
-                       p.v_pages + (((size_t)page * p.nG + g) * p.page_size + slot) * DV + ch * 8, off >= 0);
+                       p.v_pages + (((size_t)page * p.nG + g) * p.page_size + slot) * DV + ch * 8, page_s[mb][key] >= 0);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
