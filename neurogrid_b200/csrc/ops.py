@@ -664,6 +664,31 @@ def input_conv(u: torch.Tensor, weight: torch.Tensor, state: torch.Tensor, out: 
              max_q, H, L, _act_flag(u, "conv input"), _stream()), "input_conv")
 
 
+def norm_input_conv_takes(h: torch.Tensor, delta: Optional[torch.Tensor], norm_weight: torch.Tensor, weight: torch.Tensor,
+                          state: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether ``norm_input_conv`` takes a stream of this width, a convolution of this many taps and these operands."""
+    return (h.shape[1] % 4 == 0 and h.shape[1] <= 2048 and 2 <= weight.shape[1] <= 4
+            and all(t is None or t.data_ptr() % 16 == 0 for t in (h, delta, norm_weight, weight, state, out)))
+
+
+def norm_input_conv(h: torch.Tensor, delta: Optional[torch.Tensor], norm_weight: torch.Tensor, eps: float, weight: torch.Tensor,
+                    state: torch.Tensor, out: torch.Tensor, row_entry: torch.Tensor, ctx_before: torch.Tensor,
+                    slots: torch.Tensor) -> None:
+    """``add_rmsnorm`` and ``input_conv`` over its output in one launch, for a step whose entries bring one token each (bit for
+    bit what the two give); rows of no entry (``row_entry`` -1) get the norm."""
+    n, H = out.shape
+    L = weight.shape[1]
+    act = _act_flag(out, "conv out")
+    if h.shape != out.shape or weight.shape[0] != H or norm_weight.numel() != H or state.shape[1:] != (L - 1, H):
+        raise KernelError("norm_input_conv: shapes do not fit")
+    _f32(h, "residual stream"), _f32(norm_weight, "norm weight"), _f32(weight, "conv weight"), _f32(state, "conv state")
+    _i32(row_entry, "row_entry"), _i32(ctx_before, "ctx_before"), _i32(slots, "slots")
+    d32, n_part, stride = _partials(delta, h, act)
+    f = _fn("input_conv", "ng_norm_input_conv", [_c_void_p] * 9 + [_c_int] * 3 + [_c_float] + [_c_int] * 3 + [_c_ll, _c_void_p])
+    _check(f(_ptr(h), _ptr(delta), _ptr(norm_weight), _ptr(weight), _ptr(state), _ptr(out), _ptr(row_entry), _ptr(ctx_before),
+             _ptr(slots), n, H, L, float(eps), act, d32, n_part, stride, _stream()), "norm_input_conv")
+
+
 # ----------------------------------------------------------------------------- retention
 def retention(x: torch.Tensor, inv_freq: Optional[torch.Tensor], rot_dims: int, decay: torch.Tensor,
               state: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, ctx_before: torch.Tensor,

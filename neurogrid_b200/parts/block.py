@@ -142,14 +142,16 @@ class PreNormConvSideBlock:
         mixer_cache = views.pop(0)
         buf = ctx.ws.buf("normed", n, H, self.dtype)
         ctx.residual = h if ctx.fuse_residual else None
-        x = self.mixer_norm.forward(h, pending, buf)
         if self.mixer_conv is not None:
-            x = self.mixer_conv.forward(x, ctx, views.pop(0), ctx.ws.buf("conv_out", n, H, self.dtype))
+            x = self.mixer_conv.forward_normed(self.mixer_norm, h, pending, ctx, views.pop(0), buf, ctx.ws.buf("conv_out", n, H, self.dtype))
+        else:
+            x = self.mixer_norm.forward(h, pending, buf)
         out = self.mixer.forward(x, ctx, mixer_cache)
         if self.ffn is not None:
-            x = self.ffn_norm.forward(h, out, buf)
             if self.ffn_conv is not None:
-                x = self.ffn_conv.forward(x, ctx, views.pop(0), ctx.ws.buf("conv_out", n, H, self.dtype))
+                x = self.ffn_conv.forward_normed(self.ffn_norm, h, out, ctx, views.pop(0), buf, ctx.ws.buf("conv_out", n, H, self.dtype))
+            else:
+                x = self.ffn_norm.forward(h, out, buf)
             out = self.ffn.forward(x, ctx)
         if self.side is None:
             return out

@@ -6,6 +6,7 @@ import torch
 from ..cache.manager import SlotNeed
 from ..csrc import ops
 from ..weights.decl import TensorDecl
+from .norm import RMSNorm
 
 
 class InputConv:
@@ -36,6 +37,16 @@ class InputConv:
     def forward(self, u, ctx, cache, out):
         ops.input_conv(u, self.weight, cache.state, out, ctx.cu_q, ctx.ctx_before, ctx.slots, ctx.n_entries, ctx.max_q)
         return out
+
+    def forward_normed(self, norm, h, pending, ctx, cache, buf, out):
+        """The same for u = norm(h + pending); ``buf`` holds u where the two are launches of their own."""
+        # one launch for single tokens: rows of no entry are the norm's alone there, so every row is written either way
+        if ctx.max_q == 1 and not ctx.fixed_launches and type(norm).forward is RMSNorm.forward and \
+                ops.norm_input_conv_takes(h, pending, norm.weight, self.weight, cache.state, out):
+            ops.norm_input_conv(h, pending, norm.weight, norm.spec.eps, self.weight, cache.state, out, ctx.row_entry,
+                                ctx.ctx_before, ctx.slots)
+            return out
+        return self.forward(norm.forward(h, pending, buf), ctx, cache, out)
 
 
 class TokenSide:

@@ -104,6 +104,29 @@ def test_input_conv_whole_cut_and_slot_reuse(dtype, taps):
     assert rel_err(o2[T:], plain.input_conv(y.double().cpu(), w[""].double())) < TOL[dtype]
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("H,taps,delta", [(4, 2, "none"), (512, 3, "act"), (516, 4, "none"), (1024, 4, "act"), (2048, 4, "stack"), (2044, 2, "stack")])
+def test_norm_and_input_conv_in_one_launch(dtype, H, taps, delta):
+    """Single tokens: bit for bit the norm's launch and the convolution's, requests at their first positions and a row of no
+    entry among them."""
+    from neurogrid_b200.csrc import ops
+    n, ctx = 6, [0, 1, 2, 40, 7]
+    h = _x(n, H, torch.float32, scale=3.0)
+    d = None if delta == "none" else _x(n, H, dtype, seed=2) if delta == "act" else torch.stack([_x(n, H, torch.float32, seed=k) for k in (3, 4, 5)])
+    nw, w = 1 + 0.1 * _x(1, H, torch.float32, seed=6)[0], _x(H, taps, torch.float32, seed=7)
+    state = torch.randn(7, taps - 1, H, device=DEV)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    cu, cb, slots = torch.tensor([0, 1, 2, 3, 4, 5], **i32), torch.tensor(ctx, **i32), torch.tensor([3, 0, 6, 2, 5], **i32)
+    h1, s1, u1, o1 = h.clone(), state.clone(), torch.empty(n, H, dtype=dtype, device=DEV), torch.zeros(n, H, dtype=dtype, device=DEV)
+    ops.add_rmsnorm(h1, d, nw, u1, 1e-5)
+    ops.input_conv(u1, w, s1, o1, cu, cb, slots, 5, 1)
+    h2, s2, o2 = h.clone(), state.clone(), torch.zeros(n, H, dtype=dtype, device=DEV)
+    assert ops.norm_input_conv_takes(h2, d, nw, w, s2, o2)
+    ops.norm_input_conv(h2, d, nw, 1e-5, w, s2, o2, torch.tensor([0, 1, 2, 3, 4, -1], **i32), cb, slots)
+    assert torch.equal(h1, h2) and torch.equal(s1, s2)
+    assert torch.equal(o1[:5], o2[:5]) and torch.equal(u1[5], o2[5])
+
+
 def _retention(spec, dtype, seed=0, gains=None):
     part = build("mixer", spec, dtype=dtype, device=DEV)
     w = _mats({k: d.shape for k, d in part.tensors().items()}, seed, gains)
