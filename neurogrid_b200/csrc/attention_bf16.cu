@@ -18,6 +18,8 @@
 // head, context <= 4096 (gpu/cuda/paged_attention.cu:278-387); its prefill materialises
 // [heads, S, S] scores in HBM with K/V expanded to every query head
 // (gpu/cuda/attention.cu:332-363,369-500).
+#include <type_traits>
+
 #include "ng_common.cuh"
 
 #ifndef NG_HEAD_DIM
@@ -336,14 +338,72 @@ __device__ __forceinline__ uint32_t ld_b32(const bf16* p) {
 // tiles are in flight while one is computed; each warp owns 16 keys of a tile and keeps its
 // own online-softmax state over all query heads of the group (the 16 MMA rows); the four
 // states are merged through shared memory at the end.
+//
+// TI not void: the rows come as the q|k|v projection left them (one tensor of TI, or n_part float32 partial sums), and the
+// block forms its group's query rows itself: norm per head, rotation, the one rounding to bfloat16, in the arithmetic and
+// order of rope_cache.cu (the same bits).  The block whose run ends with the step's own token forms that key and value
+// too, writes them to their page and puts them into its last tile by hand, so no block reads from memory what this
+// launch writes, and every key that is read is old: all first tiles are on their way before the wait.  A launch less a layer
+// (the figures stand at the rule, parts/attention.py).
+struct DecodePrep {
+    const void* qkv; int n_part; size_t pstride;
+    const float* qw; const float* kw; const float* inv_freq; int half_pairing; float pos_scale, eps;
+    bf16* k_pages; bf16* v_pages; int* status;
+};
+constexpr int DC_PAIRS = (HD / 2 + 31) / 32;
+template <typename TI>
+__device__ __forceinline__ void dc_prep_load(const TI* qkv, size_t head_at, const DecodePrep& pr, float (&x1)[DC_PAIRS], float (&x2)[DC_PAIRS]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int u = 0; u < DC_PAIRS; ++u) {
+        const int i = lane + 32 * u, ic = min(i, HD / 2 - 1);
+        x1[u] = ng_ld_sum<bf16>(qkv, head_at + (pr.half_pairing ? ic : 2 * ic), pr.n_part, pr.pstride);
+        x2[u] = ng_ld_sum<bf16>(qkv, head_at + (pr.half_pairing ? ic + HD / 2 : 2 * ic + 1), pr.n_part, pr.pstride);
+        if (i >= HD / 2) x1[u] = x2[u] = 0.f;
+    }
+}
+// the head's norm (if it has one) and rotation; into dst, and dst2 if there is one
+__device__ __forceinline__ void dc_prep_store(const DecodePrep& pr, const float (&w1)[DC_PAIRS], const float (&w2)[DC_PAIRS], bool norm, bool turn,
+                                              const float (&sn)[DC_PAIRS], const float (&cs)[DC_PAIRS], const float (&x1)[DC_PAIRS],
+                                              const float (&x2)[DC_PAIRS], bf16* dst, bf16* dst2) {
+    const int lane = threadIdx.x & 31;
+    float r = 1.f;
+    if (norm) {
+        float ss = 0.f;
+#pragma unroll
+        for (int u = 0; u < DC_PAIRS; ++u) ss += x1[u] * x1[u] + x2[u] * x2[u];
+        r = rsqrtf(ng_warp_sum(ss) / (float)HD + pr.eps);
+    }
+#pragma unroll
+    for (int u = 0; u < DC_PAIRS; ++u) {
+        const int i = lane + 32 * u;
+        if (i >= HD / 2) continue;
+        const int a = pr.half_pairing ? i : 2 * i, b = pr.half_pairing ? i + HD / 2 : 2 * i + 1;
+        float y1 = x1[u], y2 = x2[u];
+        if (norm) { y1 = y1 * r * w1[u]; y2 = y2 * r * w2[u]; }
+        if (turn) {
+            const float z1 = y1 * cs[u] - y2 * sn[u], z2 = y1 * sn[u] + y2 * cs[u];
+            y1 = z1; y2 = z2;
+        }
+        dst[a] = __float2bfloat16(y1);
+        dst[b] = __float2bfloat16(y2);
+        if (dst2) { dst2[a] = dst[a]; dst2[b] = dst[b]; }
+    }
+}
+
+template <typename TI>
 __global__ void __launch_bounds__(DC_THREADS)
 attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages, const bf16* __restrict__ v_pages,
                    const int* __restrict__ table, int table_stride, const int* __restrict__ cu_q,
                    const int* __restrict__ ctx_before, bf16* __restrict__ out, float* __restrict__ scratch,
                    int nH, int nKV, int ps_log2, int num_pages, int window, float scale_log2, int n_splits,
-                   int keys_per_split, int table_in_smem, int n_rows, const float* __restrict__ slopes) {
+                   int keys_per_split, int table_in_smem, int n_rows, const float* __restrict__ slopes, const DecodePrep pr) {
+    constexpr bool PREP = !std::is_void<TI>::value;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(16) bf16 own[PREP ? 2 : 1][HD];
     DecodeSmem* sm = reinterpret_cast<DecodeSmem*>(smem_raw);
+    // PREP: the group's query rows lie where no tile is on its way yet (in 2.5 KB of their own they cost an SM its third block)
+    bf16 (*prep_q)[PF_LD] = sm->k[DC_STAGES - 1];
     ng_pdl_trigger();
     // What the previous kernel of the step writes is this step's query rows and, in the cache, the key and value at
     // each entry's own position.  The batch description (written by the step's host copy before its first kernel) and
@@ -376,21 +436,63 @@ attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages,
         __syncthreads();
     }
     // the tile that holds this step's own key (position `pos`), if it is among the ones asked for up front, is not old
-    const bool own_key_early = pos >= k_begin && pos < k_begin + (DC_STAGES - 1) * DC_TILE;
+    // (PREP: that key does not come from memory)
+    const bool own_key_early = !PREP && pos >= k_begin && pos < k_begin + (DC_STAGES - 1) * DC_TILE;
+    const bool has_own = PREP && n_tiles > 0 && k_end == kv_end;
+    const int load_end = has_own ? pos : k_end;                  // keys that come from the pages
     if (own_key_early) ng_pdl_wait();
 #pragma unroll
     for (int s = 0; s < DC_STAGES - 1; ++s) {
         if (s < n_tiles)
-            dc_load_tile(sm, s, k_pages, v_pages, ptab, first_page, k_begin + s * DC_TILE, key_lo, k_end, kvh, nKV,
+            dc_load_tile(sm, s, k_pages, v_pages, ptab, first_page, k_begin + s * DC_TILE, key_lo, load_end, kvh, nKV,
                          ps_log2, num_pages);
         cp_async_commit();
     }
-    if (!own_key_early) ng_pdl_wait();
+    if constexpr (PREP) {
+        // the angles and the norms' weights do not depend on the projection either
+        float sn[DC_PAIRS], cs[DC_PAIRS], w1[2][DC_PAIRS], w2[2][DC_PAIRS];
+        const float pf = (float)pos / pr.pos_scale;
+#pragma unroll
+        for (int u = 0; u < DC_PAIRS; ++u) {
+            const int i = lane + 32 * u, ic = min(i, HD / 2 - 1);
+            const int a = pr.half_pairing ? ic : 2 * ic, b = pr.half_pairing ? ic + HD / 2 : 2 * ic + 1;
+            sn[u] = 0.f;
+            cs[u] = 1.f;
+            if (pr.inv_freq && i < HD / 2) sincosf(pf * pr.inv_freq[i], &sn[u], &cs[u]);
+            w1[0][u] = pr.qw ? pr.qw[a] : 1.f; w2[0][u] = pr.qw ? pr.qw[b] : 1.f;
+            w1[1][u] = pr.kw ? pr.kw[a] : 1.f; w2[1][u] = pr.kw ? pr.kw[b] : 1.f;
+        }
+        const int own_page = has_own ? ptab[(pos >> ps_log2) - first_page] : 0;
+        const bool page_ok = own_page >= 0 && own_page < num_pages;
+        ng_pdl_wait();
+        if (n_tiles > 0) {
+            const TI* in = ng_after_wait(reinterpret_cast<const TI*>(pr.qkv));
+            const size_t at = (size_t)row * (nH + 2 * nKV) * HD;
+            const size_t slot = ((((size_t)(page_ok ? own_page : 0) * nKV + kvh) << ps_log2) + (pos & ((1 << ps_log2) - 1))) * HD;
+            // units: the group's query heads, then the own key and value; a warp takes every fourth
+            const int units = G + (has_own ? 2 : 0);
+            for (int x = warp; x < units; x += DC_WARPS) {
+                const int head = x < G ? kvh * G + x : nH + (x - G) * nKV + kvh;
+                float x1[DC_PAIRS], x2[DC_PAIRS];
+                dc_prep_load(in, at + (size_t)head * HD, pr, x1, x2);
+                if (x < G) dc_prep_store(pr, w1[0], w2[0], pr.qw != nullptr, pr.inv_freq != nullptr, sn, cs, x1, x2, prep_q[x], nullptr);
+                else if (x == G) dc_prep_store(pr, w1[1], w2[1], pr.kw != nullptr, pr.inv_freq != nullptr, sn, cs, x1, x2, own[0], page_ok ? pr.k_pages + slot : nullptr);
+                else dc_prep_store(pr, w1[1], w2[1], false, false, sn, cs, x1, x2, own[1], page_ok ? pr.v_pages + slot : nullptr);
+            }
+            if (has_own && !page_ok) {                           // no page, no key: zeros, as the loads of such keys give
+                if (threadIdx.x == 0) atomicOr(pr.status, NG_STATUS_BAD_PAGE);
+                __syncthreads();
+                for (int i = threadIdx.x; i < 2 * HD; i += DC_THREADS) own[i / HD][i % HD] = __float2bfloat16(0.f);
+            }
+        }
+        __syncthreads();
+    } else if (!own_key_early) ng_pdl_wait();
     // Q fragments (A operand): rows = the group's query heads, rows >= G are zero
     uint32_t qa[HD / 16][4];
     {
-        const bf16* qr_lo = q + ((size_t)row * nH + kvh * G + g) * HD;
-        const bf16* qr_hi = qr_lo + (size_t)8 * HD;
+        const bf16* qr_lo = PREP ? prep_q[PREP ? g : 0] : q + ((size_t)row * nH + kvh * G + g) * HD;
+        const bf16* qr_hi = PREP ? prep_q[PREP ? g + 8 : 0] : qr_lo + (size_t)8 * HD;
+        auto ld_b32 = [](const bf16* p) { return PREP ? *reinterpret_cast<const uint32_t*>(p) : ::ld_b32(p); };
 #pragma unroll
         for (int b = 0; b < HD / 16; ++b) {
             const int d = 16 * b + 2 * t;
@@ -400,6 +502,7 @@ attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages,
             qa[b][3] = g + 8 < G ? ld_b32(qr_hi + d + 8) : 0u;
         }
     }
+    if (PREP) __syncthreads();                                   // every warp has its rows: the stage may be filled
     float o[HD / 8][4];
 #pragma unroll
     for (int i = 0; i < HD / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
@@ -411,12 +514,20 @@ attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages,
     for (int tile = 0; tile < n_tiles; ++tile) {
         const int nxt = tile + DC_STAGES - 1;
         if (nxt < n_tiles)
-            dc_load_tile(sm, nxt % DC_STAGES, k_pages, v_pages, ptab, first_page, k_begin + nxt * DC_TILE, key_lo, k_end,
+            dc_load_tile(sm, nxt % DC_STAGES, k_pages, v_pages, ptab, first_page, k_begin + nxt * DC_TILE, key_lo, load_end,
                          kvh, nKV, ps_log2, num_pages);
         cp_async_commit();
         cp_async_wait<DC_STAGES - 1>();                         // tile `tile` has landed
         __syncthreads();
         const int s = tile % DC_STAGES;
+        if (PREP && has_own && tile == n_tiles - 1) {            // the step's own key and value, over the zeros in their place
+            const int r = pos - (k_begin + tile * DC_TILE);
+            for (int i = threadIdx.x; i < HD; i += DC_THREADS) {
+                sm->k[s][r][i] = own[0][i];
+                sm->v[s][r][i] = own[PREP ? 1 : 0][i];
+            }
+            __syncthreads();
+        }
         const int key0 = k_begin + tile * DC_TILE + warp * 16;   // this warp's 16 keys
         if (key0 < k_end) {
             float sc[2][4];
@@ -602,7 +713,7 @@ static int attn_decode_launch(const void* q, const void* k_pages, const void* v_
                               int table_stride, const int* cu_q, const int* ctx_before, void* out,
                               float* scratch, int n_rows, int n_entries, int nH, int nKV, int hd, int page_size,
                               int num_pages, int window, float scale, int n_splits, int max_ctx,
-                              const float* slopes, cudaStream_t stream) {
+                              const float* slopes, const DecodePrep* prep, cudaStream_t stream) {
     if (n_entries <= 0) return NG_OK;
     if (hd != HD || nH <= 0 || nKV <= 0 || nH % nKV || nH / nKV > 16 || page_size <= 0 || n_splits < 1 ||
         n_splits > 65535 || n_entries > 65535 || (n_splits > 1 && !scratch))
@@ -618,18 +729,19 @@ static int attn_decode_launch(const void* q, const void* k_pages, const void* v_
     const size_t tab_bytes = ((size_t)per / page_size + 2) * sizeof(int);
     const int table_in_smem = tab_bytes <= 16 * 1024;
     const size_t smem = sizeof(DecodeSmem) + (table_in_smem ? tab_bytes : 0);
-    static size_t smem_set = 0;
-    if (smem > smem_set) {
-        if (cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(DecodeSmem) + 16 * 1024)) != cudaSuccess)
-            return NG_LAUNCH_FAILED;
-        smem_set = sizeof(DecodeSmem) + 16 * 1024;
-    }
     dim3 grid(nKV, n_entries, n_splits);
-    NG_LAUNCH((attn_decode_kernel), grid, DC_THREADS, smem, stream, 
-        (const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, table, table_stride, cu_q, ctx_before,
-        (bf16*)out, scratch, nH, nKV, ps_log2, num_pages, window, scale * 1.4426950408889634f, n_splits, per,
-        table_in_smem, n_rows, slopes);
+#define DC_GO(TI)                                                                                                          \
+    do {                                                                                                                   \
+        static std::atomic<unsigned long long> once{0};                                                                    \
+        if (!ng_allow_smem(once, attn_decode_kernel<TI>, (int)(sizeof(DecodeSmem) + 16 * 1024))) return NG_LAUNCH_FAILED;  \
+        NG_LAUNCH((attn_decode_kernel<TI>), grid, DC_THREADS, smem, stream, (const bf16*)q, (const bf16*)k_pages,          \
+                  (const bf16*)v_pages, table, table_stride, cu_q, ctx_before, (bf16*)out, scratch, nH, nKV, ps_log2,      \
+                  num_pages, window, scale * 1.4426950408889634f, n_splits, per, table_in_smem, n_rows, slopes,            \
+                  prep ? *prep : DecodePrep{});                                                                            \
+    } while (0)
+    if (!prep) DC_GO(void);
+    else if (prep->n_part > 0) DC_GO(float);
+    else DC_GO(bf16);
     if (n_splits > 1) {
         // up to two splits one thread a column is enough, and three or four are worth four only where they are few (32 heads of
         // 64, 64 rows, 2 splits: 15.4 us with the attention in front against 18.0; 8 rows, 3 splits 7.4 against 6.5; 16 heads of
@@ -650,8 +762,23 @@ NG_EXPORT int ng_attn_decode_bf16(const void* q, const void* k_pages, const void
                                   int num_pages, int window, float scale, int n_splits, int max_ctx,
                                   const float* slopes, cudaStream_t stream) {
     return attn_decode_launch(q, k_pages, v_pages, table, table_stride, cu_q, ctx_before, out, scratch, 0x7fffffff,
-                              n_entries, nH, nKV, hd, page_size, num_pages, window, scale, n_splits, max_ctx, slopes,
+                              n_entries, nH, nKV, hd, page_size, num_pages, window, scale, n_splits, max_ctx, slopes, nullptr,
                               stream);
+}
+
+// ng_rope_cache and ng_attn_decode_bf16 in one launch (and the merge of the splits), for a step whose entries bring one token
+// each: qkv [n_rows, (nH + 2 nKV) hd] in bfloat16, or n_partials > 0 float32 partial sums of it partial_stride apart.
+NG_EXPORT int ng_attn_decode_prep_bf16(const void* qkv, int n_partials, long long partial_stride, const float* qw, const float* kw,
+                                       const float* inv_freq, int half_pairing, float pos_scale, float eps, int* status,
+                                       void* k_pages, void* v_pages, const int* table, int table_stride, const int* cu_q,
+                                       const int* ctx_before, void* out, float* scratch, int n_rows, int n_entries, int nH,
+                                       int nKV, int hd, int page_size, int num_pages, int window, float scale, int n_splits,
+                                       int max_ctx, const float* slopes, cudaStream_t stream) {
+    if (HD % 2 || !status || n_partials < 0 || pos_scale == 0.f) return NG_BAD_SIZE;
+    const DecodePrep pr{qkv, n_partials, (size_t)partial_stride, qw, kw, inv_freq, half_pairing, pos_scale, eps, (bf16*)k_pages,
+                        (bf16*)v_pages, status};
+    return attn_decode_launch(nullptr, k_pages, v_pages, table, table_stride, cu_q, ctx_before, out, scratch, n_rows, n_entries,
+                              nH, nKV, hd, page_size, num_pages, window, scale, n_splits, max_ctx, slopes, &pr, stream);
 }
 
 NG_EXPORT int ng_attn_decode_scratch_floats(int n_rows, int nH, int n_splits) {
@@ -707,5 +834,5 @@ NG_EXPORT int ng_attn_decode_bf16_noalloc(const void* q, const void* k_pages, co
     // the capacity check above counted, and skip an entry whose row lies beyond them
     return attn_decode_launch(q, k_pages, v_pages, table, table_stride, cu_q, ctx_before, out, scratch, n_rows,
                               n_entries, nH, nKV, hd, page_size, num_pages, window, scale, n_splits, max_ctx, nullptr,
-                              stream);
+                              nullptr, stream);
 }

@@ -400,6 +400,36 @@ def attn_decode_bf16(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
              float(scale), int(n_splits), int(max_ctx), _slopes(slopes, n_heads), _stream()), "attn_decode_bf16")
 
 
+def attn_decode_prep_bf16(qkv: torch.Tensor, q_weight: Optional[torch.Tensor], k_weight: Optional[torch.Tensor],
+                          inv_freq: Optional[torch.Tensor], half_pairing: bool, pos_scale: float, eps: float, status: torch.Tensor,
+                          k_pages: torch.Tensor, v_pages: torch.Tensor, table: torch.Tensor, cu_q: torch.Tensor,
+                          ctx_before: torch.Tensor, out: torch.Tensor, scratch: Optional[torch.Tensor], n_entries: int, n_heads: int,
+                          window: Optional[int], scale: float, n_splits: int, max_ctx: int,
+                          slopes: Optional[torch.Tensor] = None) -> None:
+    """``rope_cache`` and ``attn_decode_bf16`` in one launch, for a step whose entries bring one token each: qkv [N, (n_heads +
+    2 n_kv) * hd] (or a float32 stack of partial sums) as the projection left it; keys and values go to their pages."""
+    num_pages, n_kv, page_size, hd = k_pages.shape
+    n = out.shape[0]
+    if k_pages.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or v_pages.dtype != torch.bfloat16:
+        raise KernelError("attn_decode_prep_bf16 takes bfloat16 tensors")
+    if out.shape != (n, n_heads * hd) or v_pages.shape != k_pages.shape:
+        raise KernelError("attn_decode_prep_bf16: shapes do not fit")
+    n_part, stride = _stack(qkv, (n, (n_heads + 2 * n_kv) * hd), out.dtype, "attn_decode_prep_bf16 input")
+    need = attn_decode_scratch_floats(n, n_heads, hd, n_splits)
+    if need and (scratch is None or scratch.numel() < need or scratch.dtype != torch.float32):
+        raise KernelError(f"attn_decode_prep_bf16 needs {need} float32 values of scratch")
+    _f32(q_weight, "q norm weight"), _f32(k_weight, "k norm weight"), _f32(inv_freq, "inv_freq")
+    _i32(table, "table"), _i32(cu_q, "cu_q"), _i32(ctx_before, "ctx_before"), _i32(status, "status")
+    f = _fn("attention_bf16", "ng_attn_decode_prep_bf16",
+            [_c_void_p, _c_int, _c_ll] + [_c_void_p] * 3 + [_c_int, _c_float, _c_float] + [_c_void_p] * 4 + [_c_int] + [_c_void_p] * 4
+            + [_c_int] * 8 + [_c_float, _c_int, _c_int, _c_void_p, _c_void_p], {"NG_HEAD_DIM": hd})
+    _check(f(_ptr(qkv), n_part if qkv.dtype == torch.float32 else 0, stride, _ptr(q_weight), _ptr(k_weight), _ptr(inv_freq),
+             int(half_pairing), float(pos_scale), float(eps), _ptr(status), _ptr(k_pages), _ptr(v_pages), _ptr(table), table.shape[1],
+             _ptr(cu_q), _ptr(ctx_before), _ptr(out), _ptr(scratch), n, n_entries, n_heads, n_kv, hd, page_size, num_pages,
+             int(window or 0), float(scale), int(n_splits), int(max_ctx), _slopes(slopes, n_heads), _stream()),
+           "attn_decode_prep_bf16")
+
+
 # ----------------------------------------------------------------------------- attention with float32 weights
 def qkv_prep(qkv: torch.Tensor, q_out: torch.Tensor, q_weight: Optional[torch.Tensor], k_weight: Optional[torch.Tensor],
              inv_freq: Optional[torch.Tensor], k_pages: Optional[torch.Tensor], v_pages: Optional[torch.Tensor],

@@ -108,10 +108,18 @@ class Attention:
             qkv_q = ctx.ws.buf("attn_qonly", n, s.n_heads * s.head_dim, self.dtype)
             qkv_q.copy_(qkv[:, : s.n_heads * s.head_dim])
             qkv, n_kv = qkv_q, 0
+        a = ctx.ws.buf("attn_out", n, s.n_heads * s.head_dim, self.dtype)
+        plan = self._decode_plan(cache, ctx, n) if n_kv and self._one_launch(ctx) else None
+        if plan is not None and ctx.n_entries * n_kv * plan[1] <= sm_count(self.device):
+            # single tokens in few blocks: the attention prepares its rows itself
+            scratch, n_splits, max_ctx = plan
+            ops.attn_decode_prep_bf16(qkv, self.q_norm, self.k_norm, inv_freq, half, pos_scale, s.qk_norm_eps, ctx.status,
+                                      cache.k_pages, cache.v_pages, cache.table, ctx.cu_q, ctx.ctx_before, a, scratch,
+                                      ctx.n_entries, s.n_heads, s.window, self.scale, n_splits, max_ctx, pa.score_slopes)
+            return ops.linear_to_residual(a, self.w_o, self.b_o, ctx.ws, "mixer_out", residual=ctx.residual)
         ops.rope_cache(qkv, q, self.q_norm, self.k_norm, inv_freq, half, pos_scale,
                        cache.k_pages if n_kv else None, cache.v_pages if n_kv else None, cache.table,
                        ctx.positions, ctx.row_entry, s.n_heads, n_kv, s.head_dim, s.qk_norm_eps, ctx.status)
-        a = ctx.ws.buf("attn_out", n, s.n_heads * s.head_dim, self.dtype)
         self.attend(q, cache, ctx, a, pa.score_slopes)
         return ops.linear_to_residual(a, self.w_o, self.b_o, ctx.ws, "mixer_out", residual=ctx.residual)
 
@@ -149,18 +157,36 @@ class Attention:
                 ops.attn_prefill_bf16(q, cache.k_pages, cache.v_pages, cache.table, ctx.cu_q, ctx.ctx_before, out,
                                       ctx.n_entries, ctx.max_q, s.n_heads, s.window, self.scale, bool(singles), slopes)
         if singles:
-            max_ctx = ctx.decode_max_ctx or max(singles)
-            n_splits = decode_splits(ctx.decode_batch or len(singles), s.n_kv_heads, max_ctx, s.window, self.device)
-            floats = ops.attn_decode_scratch_floats(q.shape[0], s.n_heads, s.head_dim, n_splits)
-            scratch = None
-            if floats or ctx.ws.fixed:
-                # upper bound over every batch size: splits <= 3 * SMs / (rows * n_kv_heads) + 1, or 2, or
-                # what the longest context a request can have asks (one per 2,048 keys)
-                per_row = max(2, -(-(cache.table.shape[1] * cache.k_pages.shape[2]) // 2048))
-                bound = (3 * sm_count(self.device) // s.n_kv_heads + per_row * ctx.ws.max_rows + 2) * s.n_heads * (s.head_dim + 2)
-                scratch = ctx.ws.flat("attn_split_scratch", floats, torch.float32, reserve=bound)
+            scratch, n_splits, max_ctx = self._decode_plan(cache, ctx, q.shape[0], singles)
             ops.attn_decode_bf16(q, cache.k_pages, cache.v_pages, cache.table, ctx.cu_q, ctx.ctx_before, out,
                                  scratch, ctx.n_entries, s.n_heads, s.window, self.scale, n_splits, max_ctx, slopes)
+
+    def _one_launch(self, ctx):
+        """Whether the step is single tokens alone, in bfloat16, with heads that the decode kernel takes: then one launch may
+        prepare the rows and attend.  It is the faster where no SM has two of its blocks (every block prepares its group's
+        rows anew): a decode step of 1 row behind 19 tokens, 16 / 8 heads, 8 blocks a launch, 394 -> 381 us; behind 300 tokens,
+        32 / 8 heads, 32 blocks, 634 both; 32 rows, 256 blocks, 627 -> 628; 64 rows, 512 blocks, 851 -> 862; 8 rows behind
+        2,048, 448 blocks, 724 -> 732."""
+        s = self.spec
+        return (torch.device(self.device).type == "cuda" and self.dtype == torch.bfloat16 and ctx.max_q == 1 and not ctx.fixed_launches and s.n_heads // s.n_kv_heads <= 16
+                and s.head_dim % 2 == 0 and 1 in ctx.q_lens)
+
+    def _decode_plan(self, cache, ctx, n, singles=None):
+        """(scratch, splits, longest context) of the decode kernel over a step of ``n`` rows."""
+        s = self.spec
+        if singles is None:
+            singles = [c + 1 for c, k in zip(ctx.ctx_lens, ctx.q_lens) if k == 1]
+        max_ctx = ctx.decode_max_ctx or max(singles)
+        n_splits = decode_splits(ctx.decode_batch or len(singles), s.n_kv_heads, max_ctx, s.window, self.device)
+        floats = ops.attn_decode_scratch_floats(n, s.n_heads, s.head_dim, n_splits)
+        scratch = None
+        if floats or ctx.ws.fixed:
+            # upper bound over every batch size: splits <= 3 * SMs / (rows * n_kv_heads) + 1, or 2, or
+            # what the longest context a request can have asks (one per 2,048 keys)
+            per_row = max(2, -(-(cache.table.shape[1] * cache.k_pages.shape[2]) // 2048))
+            bound = (3 * sm_count(self.device) // s.n_kv_heads + per_row * ctx.ws.max_rows + 2) * s.n_heads * (s.head_dim + 2)
+            scratch = ctx.ws.flat("attn_split_scratch", floats, torch.float32, reserve=bound)
+        return scratch, n_splits, max_ctx
 
 
 def _product_library(dtype):

@@ -509,6 +509,46 @@ def test_attn_bf16_finds_a_far_key_and_respects_the_window_edge():
                 assert (d < 0.05) == hit, (single, window, h, d)
 
 
+@pytest.mark.parametrize("nH,nKV,hd,half,norm,parts,window,n_splits", [
+    (32, 8, 64, True, True, 3, None, 1), (16, 8, 64, False, True, 0, None, 5), (4, 4, 16, True, False, 2, 70, 2), (32, 2, 128, False, True, 2, None, 3),
+    (6, 1, 256, True, True, 0, 200, 4), (8, 8, 48, False, False, 6, None, 1)])
+def test_attn_decode_prep_bf16(nH, nKV, hd, half, norm, parts, window, n_splits):
+    """Bit for bit the launch that prepares the rows and the attention behind it: first tokens, tokens at the edges of tiles
+    and pages, an entry without rows, one whose page is not there; the pages written alike."""
+    ps, ctx = 16, [0, 1, 63, 64, 500, 127, 15, 333]
+    R, n = len(ctx), len(ctx)
+    per = 40
+    i32 = dict(dtype=torch.int32, device=DEV)
+    table = torch.randperm(R * per, device=DEV).to(torch.int32).view(R, per)
+    table[6, 0] = -1                                             # the page of entry 6's own token
+    cu = torch.tensor(list(range(R + 1)) + [R], **i32)           # ... and an entry without a row
+    cb, re = torch.tensor(ctx + [9], **i32), torch.arange(R, **i32)
+    table = torch.cat([table, table[:1]])
+    width = (nH + 2 * nKV) * hd
+    qkv = rnd(parts, n, width, seed=1) if parts else rnd(n, width, dtype=torch.bfloat16, seed=1)
+    qw, kw = (1 + 0.1 * rnd(hd, seed=2), 1 + 0.1 * rnd(hd, seed=3)) if norm else (None, None)
+    inv = (1e4 ** (-torch.arange(hd // 2, device=DEV) * 2.0 / hd)).float()
+    k0, v0 = (rnd(R * per, nKV, ps, hd, dtype=torch.bfloat16, seed=s) for s in (4, 5))
+    slopes = 0.01 * rnd(nH, seed=6).abs()
+    got = []
+    for fused in (False, True):
+        k, v, st = k0.clone(), v0.clone(), torch.zeros(1, **i32)
+        out = torch.full((n, nH * hd), 7.0, dtype=torch.bfloat16, device=DEV)
+        scratch = torch.empty(max(1, ops().attn_decode_scratch_floats(n, nH, hd, n_splits)), device=DEV)
+        if fused:
+            ops().attn_decode_prep_bf16(qkv, qw, kw, inv, half, 1.0, 1e-5, st, k, v, table, cu, cb, out, scratch, R + 1, nH, window,
+                                        1 / math.sqrt(hd), n_splits, 512, slopes)
+        else:
+            q = torch.empty(n, nH * hd, dtype=torch.bfloat16, device=DEV)
+            ops().rope_cache(qkv, q, qw, kw, inv, half, 1.0, k, v, table, cb[:R], re, nH, nKV, hd, 1e-5, st)
+            ops().attn_decode_bf16(q, k, v, table, cu, cb, out, scratch, R + 1, nH, window, 1 / math.sqrt(hd), n_splits, 512, slopes)
+        got.append((k, v, st, out))
+    (k1, v1, s1, o1), (k2, v2, s2, o2) = got
+    assert torch.equal(k1, k2) and torch.equal(v1, v2) and int(s1) == int(s2) != 0
+    keep = [i for i in range(n) if i != 6]                       # (a key without a page counts with a score of 0 in both)
+    assert torch.equal(o1[keep], o2[keep]) and torch.equal(o1[6], o2[6])
+
+
 # ----------------------------------------------------------------------------- tcgen05 products
 def _mm_ref(x, w, bias=None):
     r = x.double() @ w.double().T
