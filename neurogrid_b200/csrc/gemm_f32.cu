@@ -5,7 +5,8 @@
 // are added; the sums of 16 chunks are added in ascending order to a group's, the groups' sums likewise.  Both kernels
 // below form exactly that, so a row's result does not depend on M, on the other rows of the batch or on where the row
 // sits in it, and shorter chains of additions are a little nearer to 64 bits than one chain over k.  The groups of a
-// long K (2 to 8 of them) are the blocks of a cluster, which add their sums through shared memory in that order.  The reference calls cuBLAS for every contraction
+// long K (2 to 8 of them) are walked by one block, or, where that is the faster (gemm_f32_form.h), they are the blocks of a
+// cluster, which add their sums through shared memory in the same order.  The reference calls cuBLAS for every contraction
 // (gpu/cuda/matmul.cu:316-355) and has no float32 path.
 //
 // Few rows (single tokens) are bound by the weights' bytes: `gemm_f32_rows_kernel`.  More rows are bound by the FMA
@@ -14,14 +15,8 @@
 // the decode steps took 3.8 ms, those of the prompts' step of 256 padded rows 6.3 ms; with the groups of a long K side
 // by side and 192 rows the pass takes 10.7 ms instead of 13.0 (192 x 1024 x 4608: 75 us instead of 223; 2 rows: 6.2
 // instead of 10.8; 192 x 9216 x 1024: 107 us, 34 of 74 TFLOP/s).
+#include "gemm_f32_form.h"
 #include "ng_common.cuh"
-
-#define GF_CHUNK 64
-#define GF_GROUP (16 * GF_CHUNK)                 // k of a group
-// Few rows: the groups are a cluster's blocks where the launch has no more blocks than this without (1 / 2 / 8 rows, us: 1,024 x
-// 4,608 5.6 / 6.2 / 12.9 against 8.3 / 10.8 / 16.4 in one block; 2,048 x 8,192 17.5 / 19.6 / 37.8 against 17.3 / 35.4 / 53.7)
-#define GF_ROWS_FEW 600
-#define GF_MAX_CLUSTER 8                         // groups that are blocks of a cluster; a longer K walks its groups in one block
 
 __device__ __forceinline__ uint32_t gf_rank() {
     uint32_t r;
@@ -74,7 +69,6 @@ __device__ __forceinline__ void gf_wait() { asm volatile("cp.async.wait_group %0
 // one thread: a group's sum.  Eight columns a block keep 128 blocks busy at N = 1,024, and a cluster's blocks share the
 // pieces of a long K; otherwise the pieces' copies (33 KB of weights) run GR_STAGES deep.  The first weights are
 // requested before the kernel in front has ended.
-#define GR_COLS 8
 #define GR_CH 16
 #define GR_K GF_GROUP                            // a piece is a group
 #define GR_WROW (GR_K + 4)                       // 4 mod 32 words: eight columns read 16 bytes each without conflicts
@@ -329,7 +323,6 @@ static int gf_launch_cluster(void (*kernel)(KP...), dim3 grid, int threads, size
     cudaLaunchKernelEx(&cfg, kernel, KP(args)...);
     return ng_launch_status();
 }
-static inline int gf_groups(int K) { return (K + GF_GROUP - 1) / GF_GROUP; }
 
 template <int MR, bool AL, bool CLUSTER>
 static int gf_rows_as(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
@@ -348,10 +341,7 @@ static int gf_rows_as(const float* A, const float* W, const float* bias, float* 
 template <int MR, bool AL>
 static int gf_rows(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
                    int ldc, cudaStream_t stream) {
-    // a cluster where the blocks alone are few: GF_ROWS_FEW
-    const int groups = gf_groups(K);
-    const long long blocks = (long long)((N + GR_COLS - 1) / GR_COLS) * ((M + MR - 1) / MR);
-    if (groups > 1 && groups <= GF_MAX_CLUSTER && blocks <= GF_ROWS_FEW)
+    if (gf_rows_cluster(M, N, K))
         return gf_rows_as<MR, AL, true>(A, W, bias, C, M, N, K, lda, ldw, ldc, stream);
     return gf_rows_as<MR, AL, false>(A, W, bias, C, M, N, K, lda, ldw, ldc, stream);
 }
@@ -385,10 +375,12 @@ template <bool AL>
 static int gf_dispatch(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,
                        int ldw, int ldc, cudaStream_t s) {
     if (M <= GF_ROWS_MAX) {
-        if (M == 1) return gf_rows<1, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
-        if (M == 2) return gf_rows<2, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
-        if (M <= 4) return gf_rows<4, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
-        return gf_rows<8, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+        switch (gf_rows_of_block(M)) {
+            case 1: return gf_rows<1, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+            case 2: return gf_rows<2, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+            case 4: return gf_rows<4, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+            default: return gf_rows<8, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+        }
     }
     const int split = gf_groups(K) <= GF_MAX_CLUSTER ? gf_groups(K) : 1;
     auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn) * split; };

@@ -124,6 +124,22 @@ def test_gemm_f32_groups(M, N, K):
         assert torch.equal(part, out[M - n:]), n
 
 
+@pytest.mark.parametrize("N,K", [(40, 2050), (592, 2048), (600, 1540), (1184, 2048), (1192, 2047), (2376, 1600), (1040, 3072), (1536, 4100), (1544, 4100),
+                                 (24, 8191), (2400, 2049), (4104, 1537)])
+def test_gemm_f32_forms_of_few_rows_give_the_same_bits(N, K):
+    """1 to 32 rows at sizes around the lines between a cluster and one block: a row alone, in two, four and eight.  The bound
+    of the sums as above."""
+    a, w, b = rnd(32, K, seed=1), rnd(N, K, seed=2), rnd(N, seed=3)
+    whole = torch.full((32, N), float("nan"), device=DEV)
+    ops().gemm_f32(a, w, b, whole)
+    want, size = a.double() @ w.double().T + b.double(), a.double().abs() @ w.double().abs().T + b.double().abs()
+    assert bool(((whole.double() - want).abs() <= (64 + 16 + -(-K // 1024) + 3) * 2.0 ** -24 * size).all())
+    for n in (1, 2, 3, 4, 8, 9):
+        part = torch.full((n, N), float("nan"), device=DEV)
+        ops().gemm_f32(a[:n].contiguous(), w, b, part)
+        assert torch.equal(part, whole[:n]), n
+
+
 def _ragged(q_lens, ctx):
     cu = [0]
     for q in q_lens:
