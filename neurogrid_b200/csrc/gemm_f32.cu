@@ -361,9 +361,8 @@ static int gf_tile_as(const float* A, const float* W, const float* bias, float* 
 template <int BM, int BN, int TM, int TN, bool AL>
 static int gf_tile(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw,
                    int ldc, cudaStream_t s) {
-    const int groups = gf_groups(K);
-    if (groups == 1) return gf_tile_as<BM, BN, TM, TN, AL, 0>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
-    if (groups <= GF_MAX_CLUSTER) return gf_tile_as<BM, BN, TM, TN, AL, 2>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+    if (gf_groups(K) == 1) return gf_tile_as<BM, BN, TM, TN, AL, 0>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+    if (gf_tile_cluster(M, N, K)) return gf_tile_as<BM, BN, TM, TN, AL, 2>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
     return gf_tile_as<BM, BN, TM, TN, AL, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
 }
 
@@ -382,13 +381,11 @@ static int gf_dispatch(const float* A, const float* W, const float* bias, float*
             default: return gf_rows<8, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
         }
     }
-    const int split = gf_groups(K) <= GF_MAX_CLUSTER ? gf_groups(K) : 1;
-    auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn) * split; };
-    // 192 and 256 rows, us: 9,216 x 1,024 106.8 / 136.8 with 64 x 64 tiles (106.2 / 139.6 with 32 x 64); 3,072 x 1,024 67.5 / 69.9
-    // (58.8 / 71.7); 1,024 x 1,024 34.5 / 48.4 with 32 x 64 (96 and 128 blocks), 50.8 / 61.4 with 32 x 32
-    if (blocks(64, 64) >= 2 * 148) return gf_tile<64, 64, 8, 4, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
-    if (blocks(32, 64) >= 64) return gf_tile<32, 64, 4, 4, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
-    return gf_tile<32, 32, 4, 2, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+    switch (gf_tile_size(M, N, K)) {
+        case 0: return gf_tile<64, 64, 8, 4, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+        case 1: return gf_tile<32, 64, 4, 4, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+        default: return gf_tile<32, 32, 4, 2, AL>(A, W, bias, C, M, N, K, lda, ldw, ldc, s);
+    }
 }
 
 NG_EXPORT int ng_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,

@@ -140,6 +140,21 @@ def test_gemm_f32_forms_of_few_rows_give_the_same_bits(N, K):
         assert torch.equal(part, whole[:n]), n
 
 
+@pytest.mark.parametrize("N,K", [(3072, 1540), (1537, 1536), (2100, 2048), (1030, 4608), (2050, 3071), (700, 9000)])
+def test_gemm_f32_forms_of_tiles_give_the_same_bits(N, K):
+    """Rows on both sides of the lines between a cluster and one block and between the tiles: the first rows of a longer
+    product are those of a shorter one, and of a row alone."""
+    a, w, b = rnd(1100, K, seed=1), rnd(N, K, seed=2), rnd(N, seed=3)
+    whole = torch.full((1100, N), float("nan"), device=DEV)
+    ops().gemm_f32(a, w, b, whole)
+    want, size = a[:200].double() @ w.double().T + b.double(), a[:200].double().abs() @ w.double().abs().T + b.double().abs()
+    assert bool(((whole[:200].double() - want).abs() <= (64 + 16 + -(-K // 1024) + 3) * 2.0 ** -24 * size).all())
+    for n in (1, 33, 64, 96, 200, 384, 640):
+        part = torch.full((n, N), float("nan"), device=DEV)
+        ops().gemm_f32(a[:n].contiguous(), w, b, part)
+        assert torch.equal(part, whole[:n]), n
+
+
 def _ragged(q_lens, ctx):
     cu = [0]
     for q in q_lens:
