@@ -79,7 +79,11 @@ input_conv_kernel(const T* __restrict__ u, const float* __restrict__ w, float* _
 // thread NV x 4 channels, the residual sum in front as in add_rmsnorm, whose arithmetic and order this is, and the
 // convolution's of the kernel above.  A step of few rows is a chain of launches that wait for one another: two of them in
 // one, everything but the stream (weights, taps, the slot) read before the wait.  A row of no entry gets its norm.
-// 8 rows of 2,048 behind 256 tokens, 16 layers of two norms each, a decode step: 1,171 -> 1,128 us.
+// The next launch may begin only after the wait: with a product that began earlier, beside it, the token input in front (a
+// cluster, token_side.cu) took 12.3 us instead of 7.6, more than the product's head start gave.  Decode steps of 16
+// layers behind 40 tokens, two launches / one that lets the next begin at its top / this one, us: width 2,048, 1 row 1,097 /
+// 1,199 / 1,046, 4 rows 1,134 / 1,206 / 1,064, 8 rows 1,160 / 1,094 / 1,087, 64 rows 1,868 / 1,774 / 1,753; width 1,024, 1 row 843 /
+// 765 / 693, 8 rows 854 / 802 / 722, 64 rows 1,231 / 1,159 / 1,131.
 __device__ __forceinline__ float4 ic_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 ic_ld4(const __nv_bfloat16* p) {
     const uint2 u = *reinterpret_cast<const uint2*>(p);
@@ -107,7 +111,6 @@ norm_conv_token_kernel(float* __restrict__ h, const TD* __restrict__ delta, cons
                        const int* __restrict__ ctx_before, const int* __restrict__ slots, int H, float eps, int n_partials,
                        size_t partial_stride) {
     __shared__ float red[32];
-    ng_pdl_trigger();
     const int row = blockIdx.x, entry = row_entry[row];                  // the batch description: older than the step's kernels
     const int ctx = entry >= 0 ? ctx_before[entry] : 0;
     float* st = state + (size_t)(entry >= 0 ? slots[entry] : 0) * (L - 1) * H;
@@ -129,6 +132,7 @@ norm_conv_token_kernel(float* __restrict__ h, const TD* __restrict__ delta, cons
             old[u][k] = in && entry >= 0 && ctx - (L - 1) + k >= 0 ? ic_ld4(st + (size_t)k * H + j) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     ng_pdl_wait();
+    ng_pdl_trigger();                                                    // not earlier: see above
     delta = ng_after_wait(delta);
     float ss = 0.f;
 #pragma unroll
