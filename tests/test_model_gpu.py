@@ -159,6 +159,34 @@ def test_mixed_steps_replay_graphs_of_padded_shapes(model_dirs, name, dtype):
         assert rel_err(torch.stack([got[r][p] for p in places]), want[r][places]) < TOL[dtype], r
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("name", ["B", "D"])
+def test_mixed_steps_of_129_to_256_rows(model_dirs, name, dtype):
+    """Steps of two portions of together 129, 150, 192, 193, 200 and 256 rows pad to 192 and 256; each of the two kinds runs
+    eagerly, is captured and replays, also where a single kind of graph may be kept (the two count as one); the logits are
+    the plain implementation's."""
+    cfg, w = plain_lfm2.load_plain(model_dirs[name])
+    cuts = [(100, 50), (130, 70), (128, 1), (129, 64), (7, 185), (56, 200), (100, 50), (130, 70)]
+    reqs = scenarios.make_requests([sum(c[i] for c in cuts) for i in (0, 1)], cfg["vocab_size"], seed=19)
+    want = {r: plain_lfm2.forward(cfg, w, t, round_bf16=(dtype == torch.bfloat16)) for r, t in reqs.items()}
+    ps = PAGE_SIZE[name]
+    runner = make_runner(model_dirs[name], dtype=dtype, device="cuda", page_size=ps, num_pages=2048 // ps, max_requests=4,
+                         max_seq_len=1024, max_tokens_per_step=256)
+    runner.MAX_MIXED_GRAPHS = 1
+    fed, got = {"r0": 0, "r1": 0}, {"r0": {}, "r1": {}}
+    for cut in cuts:
+        lg = runner.step([StepEntry(r, reqs[r][fed[r]:fed[r] + n], [n - 1]) for r, n in zip(fed, cut)]).clone()
+        for j, (r, n) in enumerate(zip(list(fed), cut)):
+            fed[r] += n
+            got[r][fed[r] - 1] = lg[j]
+    runner.check_status()
+    runner.cache.check()
+    assert runner.stats()["graph_replays"] == len(cuts) - 2          # the first meeting of each of the two shapes runs eagerly
+    for r in reqs:
+        places = sorted(got[r])
+        assert rel_err(torch.stack([got[r][p] for p in places]), want[r][places]) < TOL[dtype], r
+
+
 def test_long_portions_cut_the_keys_into_runs(model_dirs, monkeypatch):
     """A long prompt in portions, with the threshold from which the portion kernel cuts every
     block's keys into runs lowered so that a tiny model meets it: the later portions take that
