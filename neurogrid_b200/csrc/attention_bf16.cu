@@ -341,7 +341,8 @@ __device__ __forceinline__ uint32_t ld_b32(const bf16* p) {
 //
 // TI not void: the rows come as the q|k|v projection left them (one tensor of TI, or n_part float32 partial sums), and the
 // block forms its group's query rows itself: norm per head, rotation, the one rounding to bfloat16, in the arithmetic and
-// order of rope_cache.cu (the same bits).  The block whose run ends with the step's own token forms that key and value
+// order of rope_cache.cu's general kernel (the same bits; its kernel for 64 rows and more of one bfloat16 tensor with heads of
+// 64 and pairs (i, i + 32) adds a norm's squares in another order).  The block whose run ends with the step's own token forms that key and value
 // too, writes them to their page and puts them into its last tile by hand, so no block reads from memory what this
 // launch writes, and every key that is read is old: all first tiles are on their way before the wait.  A launch less a layer
 // (the figures stand at the rule, parts/attention.py).
@@ -402,7 +403,7 @@ attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages,
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(16) bf16 own[PREP ? 2 : 1][HD];
     DecodeSmem* sm = reinterpret_cast<DecodeSmem*>(smem_raw);
-    // PREP: the group's query rows lie where no tile is on its way yet (in 2.5 KB of their own they cost an SM its third block)
+    // PREP: the group's query rows lie where no tile is on its way yet (an array of their own and one barrier less take as long)
     bf16 (*prep_q)[PF_LD] = sm->k[DC_STAGES - 1];
     ng_pdl_trigger();
     // What the previous kernel of the step writes is this step's query rows and, in the cache, the key and value at

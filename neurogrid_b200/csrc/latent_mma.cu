@@ -141,8 +141,8 @@ latent_core_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ page
     constexpr int CPK = LM_R / 8;                              // 16-byte pieces of a key
     // A tile is copied asynchronously while the one before it is used; keys past the tile's last visible one are zero.
     // Lane k looks up where key k of a tile lies, a tile ahead of the tile's copies, and hands it to the lanes that copy the
-    // key's pieces: a division by the page size and a read of the table in front of every piece cost a third of the kernel
-    // (a prompt of 2,048 tokens, 8 heads, window 1,024, four such layers of 16: 3,842 us against 4,178).
+    // key's pieces.  With a division by the page size and a read of the table in front of every piece, in the chain between two
+    // tiles, a prompt of 2,048 tokens (8 heads, window 1,024, four such layers of 16) took 4,178 us instead of 3,842.
     static_assert(LM_TILE == 32, "a lane a key");
     auto lookup = [&](int k0) {                                // rows of the cache in front of the key's, -1: there is none
         const int kp = k0 + lane;

@@ -417,8 +417,9 @@ NG_EXPORT int ng_shortconv(const void* p, const float* w, const float* bias, flo
     // steps of few rows, whose input is a stack of partial sums) are cut into tiles of 4 tokens, so that their
     // tokens are spread over blocks instead; a tile re-reads the L-1 inputs before it, which is then cheap.
     // (A tile is at least L-1 tokens: only the first tile of a portion reaches back into the state slot.)  So are longer
-    // portions whose whole tiles are fewer than two blocks an SM (two of 96 tokens, 1,024 channels, 32 bits: 48 blocks; ten
-    // such launches of a pass of 10,615 us took 158 us less).
+    // portions whose whole tiles are fewer than two blocks an SM: a launch that lasts as long as one thread's walk (32 bits, us,
+    // whole tiles / small ones: L = 3, 1,024 channels, two portions of 96 tokens, 48 blocks 13.8 / 2.9; one of 600, 152 blocks
+    // 14.0 / 3.5; one of 1,100, 280 blocks 14.5 / 6.0; L = 2, 280 blocks 10.0 / 4.2; L = 8, 280 blocks 15.8 / 10.9).
     const bool few = (long long)grid.x * grid.y * grid.z < 2 * 148;
     const int tile = max_q <= 64 || few ? (NG_CONV_L - 1 > 4 ? NG_CONV_L - 1 : 4) : CONV_TILE;
     grid.y = (max_q + tile - 1) / tile;

@@ -163,10 +163,12 @@ class Attention:
 
     def _one_launch(self, ctx):
         """Whether the step is single tokens alone, in bfloat16, with heads that the decode kernel takes: then one launch may
-        prepare the rows and attend.  It is the faster where no SM has two of its blocks (every block prepares its group's
-        rows anew): a decode step of 1 row behind 19 tokens, 16 / 8 heads, 8 blocks a launch, 394 -> 381 us; behind 300 tokens,
-        32 / 8 heads, 32 blocks, 634 both; 32 rows, 256 blocks, 627 -> 628; 64 rows, 512 blocks, 851 -> 862; 8 rows behind
-        2,048, 448 blocks, 724 -> 732."""
+        prepare the rows and attend.  It is the faster, or as fast, where no SM has two of its blocks (every block prepares its
+        group's rows anew).  Decode steps, two launches / one, us, blocks a launch in brackets: 16 / 8 heads, 16 layers of which 6
+        attend, behind 19 tokens 1 row [8] 392 / 377, 4 rows [32] 401 / 387, 8 rows [64] 414 / 401, 16 rows [128] 422 / 409, behind 1,000
+        tokens 1 row [32] 413 / 402, 4 rows [128] 440 / 430, behind 4,000 1 row [120] 434 / 422; 32 / 8 heads behind 19 tokens 1 row [8]
+        616 / 611, 16 rows [128] 657 / 652, behind 300 4 rows [32] 650 / 650, 16 rows [128] 684 / 684, behind 1,000 4 rows [128] 672 / 660.
+        Beyond: 18 rows [256] 711 / 711, 64 rows [512] 851 / 862, 8 rows behind 2,048 [448] 724 / 732."""
         s = self.spec
         return (torch.device(self.device).type == "cuda" and self.dtype == torch.bfloat16 and ctx.max_q == 1 and not ctx.fixed_launches and s.n_heads // s.n_kv_heads <= 16
                 and s.head_dim % 2 == 0 and 1 in ctx.q_lens)

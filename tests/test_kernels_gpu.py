@@ -183,6 +183,33 @@ def test_shortconv(dtype, L, H, bias):
     assert torch.equal(st1[4], st2[4]) and torch.equal(st1[7], st2[7])    # untouched slots stay
 
 
+@pytest.mark.parametrize("parts", [1, 3])
+@pytest.mark.parametrize("L", [2, 3, 8])
+def test_shortconv_small_and_whole_tiles_give_the_same_bits(L, parts):
+    """Portions of more than 64 tokens on both sides of the number of blocks up to which they are cut into small tiles (16
+    blocks a tile of 32 tokens and entry at 2,048 channels): 97 tokens, four entries (256 blocks) and five (320), 129 tokens, three
+    (240) and four (320); outputs and slots."""
+    H = 2048
+    for T, few, many in ((97, 4, 5), (129, 3, 4)):
+        lens, ctx = [T, 70, 2, T - 1, 33][:many - 1] + [T], [0, 5, 1, 40, 2][:many]
+        cu, cb, N = _ragged(lens, ctx)
+        stack = rnd(parts, N, 3 * H, seed=4, std=0.5)
+        p = stack[0] if parts == 1 else stack
+        dtype = torch.float32 if parts == 1 else torch.bfloat16
+        w, b, slots = rnd(H, L, seed=5, std=0.3), rnd(H, seed=6, std=0.1), torch.randperm(7, generator=torch.Generator().manual_seed(1))[:many].to(torch.int32).to(DEV)
+        st1 = rnd(8, L - 1, H, seed=7)
+        st2, st3 = st1.clone(), st1.clone()
+        o1, o2, o3 = (torch.zeros(N, H, dtype=dtype, device=DEV) for _ in range(3))
+        ops().shortconv(p, w, b, st1, o1, cu, cb, slots, many, T)                     # whole tiles
+        first = int(cu[few])
+        ops().shortconv(p, w, b, st2, o2, cu, cb, slots, few, T)                      # small ones: the first entries alone
+        assert torch.equal(o1[:first], o2[:first]) and torch.equal(st1[slots[:few].long()], st2[slots[:few].long()])
+        whole = p if parts == 1 else functools.reduce(torch.add, stack).to(dtype)
+        ref.shortconv(whole, w, b, st3, o3, cu, cb, slots, many, T)
+        close(o1, o3, dtype)
+        close(st1, st3, torch.float32)
+
+
 @pytest.mark.parametrize("L,H,bias", [(3, 2048, False), (2, 200, True), (4, 96, True), (5, 264, False)])
 def test_shortconv_long_portions(L, H, bias):
     """Long bfloat16 portions take the kernel with 16-byte accesses: tiles of 8 tokens, portions
@@ -578,6 +605,43 @@ def test_attn_decode_prep_bf16(nH, nKV, hd, half, norm, parts, window, n_splits)
     assert torch.equal(k1, k2) and torch.equal(v1, v2) and int(s1) == int(s2) != 0
     keep = [i for i in range(n) if i != 6]                       # (a key without a page counts with a score of 0 in both)
     assert torch.equal(o1[keep], o2[keep]) and torch.equal(o1[6], o2[6])
+
+
+@pytest.mark.parametrize("n,nH,nKV", [(64, 8, 1), (72, 4, 2)])
+def test_attn_decode_prep_bf16_of_many_rows_and_few_heads(n, nH, nKV):
+    """64 rows and more of one bfloat16 tensor, heads of 64, pairs (i, i + 32): bit for bit the launch that prepares fewer rows (the
+    rows given in parts).  The launch of all rows adds a norm's squares in another order: 64 terms, so the norms agree to 64
+    * 2^-24, and k, rounded once, to one step of bfloat16 of the larger of its pair."""
+    hd, ps, per = 64, 16, 8
+    i32 = dict(dtype=torch.int32, device=DEV)
+    table = torch.randperm(n * per, device=DEV).to(torch.int32).view(n, per)
+    cb = torch.tensor([(7 * i) % 120 for i in range(n)], **i32)
+    cu, re = torch.arange(n + 1, **i32), torch.arange(n, **i32)
+    qkv = rnd(n, (nH + 2 * nKV) * hd, dtype=torch.bfloat16, seed=1)
+    qw, kw = 1 + 0.1 * rnd(hd, seed=2), 1 + 0.1 * rnd(hd, seed=3)
+    inv = (1e4 ** (-torch.arange(hd // 2, device=DEV) * 2.0 / hd)).float()
+    k0, v0 = (rnd(n * per, nKV, ps, hd, dtype=torch.bfloat16, seed=s) for s in (4, 5))
+    scale, got = 1 / math.sqrt(hd), []
+    for how in ("one", "parts", "all"):
+        k, v, st = k0.clone(), v0.clone(), torch.zeros(1, **i32)
+        out = torch.empty(n, nH * hd, dtype=torch.bfloat16, device=DEV)
+        if how == "one":
+            ops().attn_decode_prep_bf16(qkv, qw, kw, inv, True, 1.0, 1e-5, st, k, v, table, cu, cb, out, None, n, nH, None, scale, 1, 128)
+        else:
+            q = torch.empty(n, nH * hd, dtype=torch.bfloat16, device=DEV)
+            step = 32 if how == "parts" else n
+            for a in range(0, n, step):
+                z = slice(a, min(n, a + step))
+                ops().rope_cache(qkv[z], q[z], qw, kw, inv, True, 1.0, k, v, table, cb[z], re[z], nH, nKV, hd, 1e-5, st)
+            ops().attn_decode_bf16(q, k, v, table, cu, cb, out, None, n, nH, None, scale, 1, 128)
+        got.append((k, v, out))
+    (k1, v1, o1), (k2, v2, o2), (k3, v3, o3) = got
+    assert torch.equal(k1, k2) and torch.equal(v1, v2) and torch.equal(o1, o2)
+    assert torch.equal(v1, v3)
+    size = k1.float().abs()
+    size = torch.maximum(size, size.roll(hd // 2, -1))
+    assert bool(((k1.float() - k3.float()).abs() <= 2.0 ** -7 * size).all())
+    close(o1, o3, torch.bfloat16)
 
 
 # ----------------------------------------------------------------------------- tcgen05 products
