@@ -28,14 +28,14 @@ static inline bool gf_rows_cluster(int M, int N, int K) {
     if (mr == 1) return groups > 2 && ((groups > 3 && blocks <= 192) || blocks > 2 * 148);
     if (groups > 2) return true;
     if (blocks <= 96) return true;
-    // two rows: a short second group is not worth a block; of the others, where the blocks' last round would be nearly empty (296
-    // a round: 4,800 columns) or the rounds are many
+    // two rows: a short second group is not worth a block; of the others, where the blocks' last wave would be nearly empty (296
+    // a wave: 4,800 columns) or the waves are many
     if (mr == 2) return K - GF_GROUP > GF_GROUP / 2 && ((blocks > 512 && blocks <= 640) || blocks > 1024);
     return blocks > (mr == 4 ? 2 : 1) * 148;                             // more than are resident at once
 }
 
 // More rows: whether a tile's groups are the blocks of a cluster.  They are where one block a tile leaves SMs idle, or (296 tiles
-// of 64 x 64 are resident at once) where a second round would be nearly empty; a group that is half empty is worth less.
+// of 64 x 64 are resident at once) where a second wave would be nearly empty; a group that is half empty is worth less.
 // us, mean over four surroundings of the product, a cluster / one block, 64 x 64 tiles of as many blocks as stand in brackets:
 //   K = 1,280  [32] 51 / 51, [128] 83 / 68, [512] 259 / 182          K = 1,536  [48] 53 / 69, [72] 62 / 63, [96] 76 / 68 (96 rows of 3,072: 59 / 73), [576] 282 / 203
 //   K = 2,048  [144] 77 / 120, [192] 115 / 139, [256] 152 / 145, [288] 146 / 139, [320] 184 / 209, [768] 383 / 394, [1,024] 496 / 471
